@@ -459,6 +459,8 @@ void release(fe_ctx* c) {
 }
 
 dim3 chunk_grid(const fe_ctx* c) { return dim3(c->B.n_chunks); }
+// One block over the scene table: a warp for a single scene.
+dim3 scene_block(const fe_ctx* c) { return dim3(c->B.n_scenes > 32 ? kBlock : 32); }
 
 // The instantiation of a neighbour kernel for a block size (128, 256, 512)
 // and persistence.
@@ -650,7 +652,7 @@ fe_status rec_stats(fe_ctx* c, Recorder& R) {
 fe_status rec_solve(fe_ctx* c, Recorder& R, int which) {
     Bufs B = c->B;
     if (!R.graph) {
-        REC(R.k(k_solve_begin, dim3(1), dim3(32), B, which, (cudaGraphConditionalHandle)0, 0));
+        REC(R.k(k_solve_begin, dim3(1), scene_block(c), B, which, (cudaGraphConditionalHandle)0, 0));
         for (uint32_t guard = 0; guard < 200001; ++guard) {
             uint32_t cond = 0;
             REC(cudaMemcpyAsync(&cond, &B.G->cond[which], sizeof cond, cudaMemcpyDeviceToHost,
@@ -664,12 +666,12 @@ fe_status rec_solve(fe_ctx* c, Recorder& R, int which) {
                 REC(R.k(k_solve_finish, dim3(B.n_scenes), dim3(kBlock), B, which,
                         (cudaGraphConditionalHandle)0, 0));
         }
-        REC(R.k(k_solve_end, dim3(1), dim3(32), B, which));
+        REC(R.k(k_solve_end, dim3(1), scene_block(c), B, which));
         return FE_OK;
     }
     cudaGraphConditionalHandle h;
     REC(cudaGraphConditionalHandleCreate(&h, R.root, 0, 0));
-    REC(R.k(k_solve_begin, dim3(1), dim3(32), B, which, h, 1));
+    REC(R.k(k_solve_begin, dim3(1), scene_block(c), B, which, h, 1));
     // cudaGraphNodeParams has no default constructor (it holds a union);
     // zeroed storage gives the required all-zero reserved fields.
     alignas(cudaGraphNodeParams) unsigned char cp_storage[sizeof(cudaGraphNodeParams)] = {};
@@ -691,7 +693,7 @@ fe_status rec_solve(fe_ctx* c, Recorder& R, int which) {
         REC(body.k(k_solve_finish, dim3(B.n_scenes), dim3(kBlock), B, which, h, 1));
     REC(body.k(k_loop_guard, dim3(1), dim3(32), B, which, h));
     R.last = node;
-    REC(R.k(k_solve_end, dim3(1), dim3(32), B, which));
+    REC(R.k(k_solve_end, dim3(1), scene_block(c), B, which));
     return FE_OK;
 }
 

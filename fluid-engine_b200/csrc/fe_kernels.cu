@@ -759,15 +759,17 @@ __device__ void solve_finish_scene(Bufs& B, int which, uint32_t s, uint32_t c0, 
     __syncthreads();
 }
 
-// Sets the loop condition from every scene's done flag (thread 0).
+// Sets the loop condition from every scene's done flag (whole block).
 __device__ __forceinline__ void solve_set_condition(Bufs& B, int which,
                                                     cudaGraphConditionalHandle handle,
                                                     int use_handle) {
-    uint32_t any_open = 0;
-    for (uint32_t s = 0; s < B.n_scenes; ++s)
+    int any_open = 0;
+    for (uint32_t s = threadIdx.x; s < B.n_scenes; s += blockDim.x)
         if (!__ldcg(&B.S[s].solve[which].done)) any_open = 1;
-    B.G->cond[which] = any_open;
-    if (use_handle) cudaGraphSetConditional(handle, any_open);
+    any_open = __syncthreads_or(any_open);
+    if (threadIdx.x != 0) return;
+    B.G->cond[which] = (uint32_t)any_open;
+    if (use_handle) cudaGraphSetConditional(handle, (unsigned)any_open);
 }
 
 // Multi-scene contexts: the per-scene finish in parallel, one block per
@@ -781,9 +783,9 @@ __global__ void __launch_bounds__(kBlock) k_solve_finish(Bufs B, int which,
     const uint32_t s = blockIdx.x;
     const uint32_t c0 = scene_chunk_base(B, s, tmp);
     solve_finish_scene(B, which, s, c0, smem);
-    if (last_block_done(&B.G->tickets[kTicketSolve], gridDim.x) && threadIdx.x == 0) {
+    if (last_block_done(&B.G->tickets[kTicketSolve], gridDim.x)) {
         solve_set_condition(B, which, handle, use_handle);
-        B.G->tickets[kTicketSolve] = 0;
+        if (threadIdx.x == 0) B.G->tickets[kTicketSolve] = 0;
     }
 }
 
@@ -848,20 +850,24 @@ __global__ void __launch_bounds__(kBlock) k_pressure_update(Bufs B, int which,
     // k_solve_finish does, one block per scene.
     if (B.n_scenes == 1 && last_block_done(&B.G->tickets[kTicketSolve], gridDim.x)) {
         solve_finish_scene(B, which, 0, 0, smem);
-        if (threadIdx.x == 0) {
-            solve_set_condition(B, which, handle, use_handle);
-            B.G->tickets[kTicketSolve] = 0;
-        }
+        solve_set_condition(B, which, handle, use_handle);
+        if (threadIdx.x == 0) B.G->tickets[kTicketSolve] = 0;
     }
 }
 
 // Starts a solve: resets the per-scene control and sets the loop condition.
-__global__ void k_solve_begin(Bufs B, int which, cudaGraphConditionalHandle handle,
-                              int use_handle) {
-    if (threadIdx.x != 0) return;
-    uint32_t any_open = 0;
+// One block, scenes spread over its threads: a scene's control is a chain of
+// dependent loads from its parameter block, and one thread walking 256 scenes
+// took 248 us of a batch frame (about 4 us this way).
+__global__ void __launch_bounds__(kBlock) k_solve_begin(Bufs B, int which,
+                                                        cudaGraphConditionalHandle handle,
+                                                        int use_handle) {
+    __shared__ uint32_t s_cap;
+    if (threadIdx.x == 0) s_cap = 0;
+    __syncthreads();
+    int any_open = 0;
     uint32_t cap = 0;
-    for (uint32_t s = 0; s < B.n_scenes; ++s) {
+    for (uint32_t s = threadIdx.x; s < B.n_scenes; s += blockDim.x) {
         const DevParams& P = B.P[s];
         SolveCtl& ctl = B.S[s].solve[which];
         uint32_t want = (P.solver == 1u) ? P.max_it
@@ -875,10 +881,13 @@ __global__ void k_solve_begin(Bufs B, int which, cudaGraphConditionalHandle hand
         ctl.done = (P.solver == 1u) ? (P.max_it == 0u) : (ctl.K == 0u);
         if (!ctl.done) any_open = 1;
     }
-    B.G->cond[which] = any_open;
+    if (cap) atomicMax(&s_cap, cap);
+    any_open = __syncthreads_or(any_open);
+    if (threadIdx.x != 0) return;
+    B.G->cond[which] = (uint32_t)any_open;
     B.G->body_runs[which] = 0;
-    B.G->body_cap[which] = cap + 2;
-    if (use_handle) cudaGraphSetConditional(handle, any_open);
+    B.G->body_cap[which] = s_cap + 2;
+    if (use_handle) cudaGraphSetConditional(handle, (unsigned)any_open);
 }
 
 // Last node of a WHILE body: counts executions and ends the loop after a
@@ -894,10 +903,10 @@ __global__ void k_loop_guard(Bufs B, int which, cudaGraphConditionalHandle handl
     }
 }
 
-// Ends a solve: records iterations used, residual and cap hits.
-__global__ void k_solve_end(Bufs B, int which) {
-    if (threadIdx.x != 0) return;
-    for (uint32_t s = 0; s < B.n_scenes; ++s) {
+// Ends a solve: records iterations used, residual and cap hits (scenes over
+// the threads of one block, as k_solve_begin: 214 us before at 256 scenes).
+__global__ void __launch_bounds__(kBlock) k_solve_end(Bufs B, int which) {
+    for (uint32_t s = threadIdx.x; s < B.n_scenes; s += blockDim.x) {
         SceneState& S = B.S[s];
         SolveCtl& ctl = S.solve[which];
         S.last_iters[which] = ctl.iter;
