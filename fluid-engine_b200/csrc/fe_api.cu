@@ -646,32 +646,47 @@ fe_status rec_stats(fe_ctx* c, Recorder& R) {
     return FE_OK;
 }
 
-// One Jacobi solve.  Graph: begin kernel, WHILE node {force, update, the
-// per-scene finish when the context holds several scenes, guard}, end
-// kernel.  Eager: the same kernels with a host loop on the device flag.
+// Starts a Jacobi solve.  The density solve without the network's start
+// begins at pressure 0, so its first iteration needs no neighbour pass
+// (k_pressure_first).
+fe_status rec_solve_begin(fe_ctx* c, Recorder& R, int which, cudaGraphConditionalHandle h,
+                          int use_handle) {
+    const bool first = which == 0 && !c->learned();
+    if (!first || c->B.n_scenes > 1)
+        REC(R.k(k_solve_begin, dim3(1), scene_block(c), c->B, which, h, use_handle));
+    if (!first) return FE_OK;
+    REC(R.k(k_pressure_first, chunk_grid(c), dim3(kBlock), c->B, h, use_handle));
+    if (c->B.n_scenes > 1)
+        REC(R.k(k_solve_finish, dim3(c->B.n_scenes), dim3(kBlock), c->B, which, h, use_handle, 1));
+    return FE_OK;
+}
+
+// One Jacobi solve.  Graph: begin, WHILE node {force, update, the per-scene
+// finish when the context holds several scenes, guard}, end kernel.  Eager:
+// the same kernels with a host loop on the device flag.
 fe_status rec_solve(fe_ctx* c, Recorder& R, int which) {
     Bufs B = c->B;
+    fe_status st;
     if (!R.graph) {
-        REC(R.k(k_solve_begin, dim3(1), scene_block(c), B, which, (cudaGraphConditionalHandle)0, 0));
+        if ((st = rec_solve_begin(c, R, which, (cudaGraphConditionalHandle)0, 0))) return st;
         for (uint32_t guard = 0; guard < 200001; ++guard) {
             uint32_t cond = 0;
             REC(cudaMemcpyAsync(&cond, &B.G->cond[which], sizeof cond, cudaMemcpyDeviceToHost,
                                 R.stream));
             REC(cudaStreamSynchronize(R.stream));
             if (!cond) break;
-            fe_status st;
             if ((st = rec_force(c, R, which))) return st;
             if ((st = rec_update(c, R, which, (cudaGraphConditionalHandle)0, 0))) return st;
             if (B.n_scenes > 1)
                 REC(R.k(k_solve_finish, dim3(B.n_scenes), dim3(kBlock), B, which,
-                        (cudaGraphConditionalHandle)0, 0));
+                        (cudaGraphConditionalHandle)0, 0, 0));
         }
         REC(R.k(k_solve_end, dim3(1), scene_block(c), B, which));
         return FE_OK;
     }
     cudaGraphConditionalHandle h;
     REC(cudaGraphConditionalHandleCreate(&h, R.root, 0, 0));
-    REC(R.k(k_solve_begin, dim3(1), scene_block(c), B, which, h, 1));
+    if ((st = rec_solve_begin(c, R, which, h, 1))) return st;
     // cudaGraphNodeParams has no default constructor (it holds a union);
     // zeroed storage gives the required all-zero reserved fields.
     alignas(cudaGraphNodeParams) unsigned char cp_storage[sizeof(cudaGraphNodeParams)] = {};
@@ -686,11 +701,10 @@ fe_status rec_solve(fe_ctx* c, Recorder& R, int which) {
     body.stream = R.stream;
     body.graph = cp.conditional.phGraph_out[0];
     body.root = R.root;
-    fe_status st;
     if ((st = rec_force(c, body, which))) return st;
     if ((st = rec_update(c, body, which, h, 1))) return st;
     if (B.n_scenes > 1)  // the per-scene finish, one block per scene
-        REC(body.k(k_solve_finish, dim3(B.n_scenes), dim3(kBlock), B, which, h, 1));
+        REC(body.k(k_solve_finish, dim3(B.n_scenes), dim3(kBlock), B, which, h, 1, 0));
     REC(body.k(k_loop_guard, dim3(1), dim3(32), B, which, h));
     R.last = node;
     REC(R.k(k_solve_end, dim3(1), scene_block(c), B, which));

@@ -65,7 +65,7 @@ struct SceneState {
 struct GlobalState {
     uint32_t flags;        // FE_STATS_* bits raised by device code
     uint32_t cond[2];      // last loop condition of each solve (eager mode)
-    uint32_t pad;
+    uint32_t src_nonfinite;  // a density source was Inf or NaN (see k_pressure_first)
     uint32_t tickets[8];   // last-block counters, reset by the last block
     uint32_t body_runs[2]; // loop-body executions of the current solve
     uint32_t body_cap[2];  // hard bound on body_runs (guard of the WHILE node)

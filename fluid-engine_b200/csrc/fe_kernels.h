@@ -32,7 +32,7 @@ template <int kThreads, bool kPersist>
 __global__ void k_viscosity(Bufs B);
 // Per-scene finishes of a multi-scene context, one block per scene.
 __global__ void k_solve_finish(Bufs B, int which, cudaGraphConditionalHandle handle,
-                               int use_handle);
+                               int use_handle, int first);
 __global__ void k_stats_finish(Bufs B, uint4* upart);
 template <int kThreads, bool kPersist>
 __global__ void k_density_source(Bufs B);
@@ -44,6 +44,8 @@ __global__ void k_pressure_update(Bufs B, int which, cudaGraphConditionalHandle 
                                   int use_handle);
 __global__ void k_solve_begin(Bufs B, int which, cudaGraphConditionalHandle handle,
                               int use_handle);
+// The density solve's first iteration from the plain (zero) start.
+__global__ void k_pressure_first(Bufs B, cudaGraphConditionalHandle handle, int use_handle);
 __global__ void k_solve_end(Bufs B, int which);
 __global__ void k_loop_guard(Bufs B, int which, cudaGraphConditionalHandle handle);
 __global__ void k_pressure_integration(Bufs B);

@@ -4,7 +4,8 @@ import numpy as np
 import pytest
 
 from fluid_step import _abi, scene
-from fluid_step.pipelines import BatchSimulation, Simulation
+from fluid_step.pipelines import (BatchSimulation, CommandBufferBuilder, ComputePipelines,
+                                  GpuPhysicsData, Simulation)
 
 pytestmark = pytest.mark.gpu
 
@@ -34,3 +35,43 @@ def test_each_scene_keeps_its_own_iteration_counts(n_scenes):
             assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (s, f)
         one.close()
     batch.close()
+
+
+FIELDS = [_abi.FE_FIELD_POSITION_A, _abi.FE_FIELD_POSITION_B, _abi.FE_FIELD_VELOCITY_A,
+          _abi.FE_FIELD_VELOCITY_B, _abi.FE_FIELD_DENSITY, _abi.FE_FIELD_FACTOR,
+          _abi.FE_FIELD_SOURCE_TERM, _abi.FE_FIELD_PRESSURE, _abi.FE_FIELD_PRESSURE_ACCEL]
+
+
+@pytest.mark.parametrize("non_finite", [False, True])
+@pytest.mark.parametrize("n,iters", [(1, 2), (255, 0), (256, 1), (257, 2), (3001, 1), (3001, 5)])
+@pytest.mark.parametrize("mode", [_abi.FE_MODE_REFERENCE, _abi.FE_MODE_FIXED])
+def test_frame_solve_is_the_solve_pass_by_pass(mode, n, iters, non_finite):
+    """The frame's solves (the density solve's first iteration has no
+    neighbour loop there) against the general passes called one by one, bit
+    for bit: no iteration, the first one alone, several; with an infinite
+    velocity, whose source terms are not finite, the gradients' zeros do not
+    stay zeros and the frame has to run the loops as well."""
+    w = scene.workload("dam_break_16k")
+    p = _abi.copy_params(w.params)
+    p.mode = mode
+    p.density_solver_iterations = p.divergence_solver_iterations = iters
+    pos = w.positions()[:n]
+    sim = Simulation(pos, p)
+    data = GpuPhysicsData(pos, p)
+    steps = ComputePipelines()
+    steps.prepare_all(data)
+    builder = CommandBufferBuilder(data)
+    for k in range(2):
+        if non_finite and k == 1:
+            v = np.zeros((n, 4), np.float32)
+            v[n // 2, 1] = np.inf
+            for d in (sim.data, data):
+                d.upload(_abi.FE_FIELD_VELOCITY_B, v)
+        sim.step(1, want_stats=False)
+        steps.submit_substeps(builder, iters, 1, k == 0)
+        for f in FIELDS:
+            a, b = sim.data.download(f), data.download(f)
+            bad = np.nonzero(a.view(np.uint32).reshape(-1) != b.view(np.uint32).reshape(-1))[0]
+            assert bad.size == 0, (k, f, bad.size, a.reshape(-1)[bad[0]], b.reshape(-1)[bad[0]])
+    sim.close()
+    data.close()
