@@ -472,7 +472,21 @@ auto pick(void (*k128)(KArgs...), void (*k256)(KArgs...), void (*k512)(KArgs...)
 #define NBR_KERNEL_P(name, threads, persist)                                           \
     ((persist) ? pick(name<128, true>, name<256, true>, name<512, true>, (threads))   \
                : pick(name<128, false>, name<256, false>, name<512, false>, (threads)))
-#define NBR_KERNEL(name, g) NBR_KERNEL_P(name, c->nbr_threads[g], c->nbr_persistent[g])
+// Few particles: the shape with 64 threads and deep batches, whatever the tuned
+// one is.  The line is two such blocks per SM.  Times in a graph of launches
+// (us; 256 threads and batches of 4 / this shape) of viscosity, pressure_force
+// and pressure_update: 4.8k particles 9.8/7.1, 7.5/5.7, 8.2/6.9; 16k 10.5/8.8,
+// 7.9/7.0, 8.6/8.3; 25k 10.6/9.7, 8.1/7.4, 8.9/9.0; 50k 13.4/12.2, 9.3/8.8,
+// 11.4/11.2 with whole frames slower (347/390); 80k 15.4/19.1, 10.3/12.6,
+// 14.5/17.0.
+#ifndef FE_FEW_PARTICLES
+#define FE_FEW_PARTICLES (148 * 128)
+#endif
+constexpr uint32_t kFewParticles = FE_FEW_PARTICLES;
+bool few(const fe_ctx* c) { return c->n <= kFewParticles; }
+#define NBR_KERNEL(name, g)               \
+    (few(c) ? name<kFewThreads, false>    \
+            : NBR_KERNEL_P(name, c->nbr_threads[g], c->nbr_persistent[g]))
 
 // Grid of a neighbour kernel of group g: one block per chunk step (a chunk,
 // two chunks for 512 threads), or, persistent, as many blocks as fit on the
@@ -511,19 +525,29 @@ fe_status rec_check(cudaError_t e, const char* what) {
         if (s_ != FE_OK) return s_;                            \
     } while (0)
 
-// A neighbour kernel of group g with its tuned shape.
+// A kernel of group g with its tuned shape.
 template <class... KArgs, class... Args>
-fe_status rec_nbr(fe_ctx* c, Recorder& R, int g, void (*func)(KArgs...), Args... args) {
+fe_status rec_shaped(fe_ctx* c, Recorder& R, int g, void (*func)(KArgs...), Args... args) {
     const NbrGrid G = nbr_grid(c, g, (const void*)func);
     REC(R.k(func, G.grid, G.block, args...));
     return FE_OK;
+}
+
+// A neighbour kernel of group g (NBR_KERNEL) with its shape.
+template <class... KArgs, class... Args>
+fe_status rec_nbr(fe_ctx* c, Recorder& R, int g, void (*func)(KArgs...), Args... args) {
+    if (few(c)) {
+        REC(R.k(func, dim3(c->B.n_chunks * (kBlock / kFewThreads)), dim3(kFewThreads), args...));
+        return FE_OK;
+    }
+    return rec_shaped(c, R, g, func, args...);
 }
 
 // (128 or 256 threads: the shapes fe_set_tuning accepts for this group)
 fe_status rec_density_alpha(fe_ctx* c, Recorder& R) {
     const int g = FE_NBR_DENSITY_ALPHA;
     const uint32_t t = c->nbr_threads[g];
-    return rec_nbr(c, R, g,
+    return rec_shaped(c, R, g,
                    c->nbr_persistent[g]
                        ? pick(k_density_alpha<128, true>, k_density_alpha<256, true>,
                               k_density_alpha<256, true>, t)
@@ -539,7 +563,7 @@ fe_status rec_density_alpha_div(fe_ctx* c, Recorder& R) {
     const int g = FE_NBR_DENSITY_ALPHA;
     const uint32_t t = c->nbr_threads[g];
     if (c->carries())
-        return rec_nbr(c, R, g,
+        return rec_shaped(c, R, g,
                        c->nbr_persistent[g]
                            ? pick(k_density_alpha_div_learn<128, true>,
                                   k_density_alpha_div_learn<256, true>,
@@ -548,7 +572,7 @@ fe_status rec_density_alpha_div(fe_ctx* c, Recorder& R) {
                                   k_density_alpha_div_learn<256, false>,
                                   k_density_alpha_div_learn<256, false>, t),
                        c->B, c->fixed_mode() ? 1 : 0, c->L);
-    return rec_nbr(c, R, g,
+    return rec_shaped(c, R, g,
                    c->nbr_persistent[g]
                        ? pick(k_density_alpha_div<128, true>, k_density_alpha_div<256, true>,
                               k_density_alpha_div<256, true>, t)
@@ -572,7 +596,12 @@ fe_status rec_force(fe_ctx* c, Recorder& R, int which) {
 
 fe_status rec_update(fe_ctx* c, Recorder& R, int which, cudaGraphConditionalHandle h,
                      int use_handle) {
-    return rec_nbr(c, R, FE_NBR_PRESSURE_UPDATE, k_pressure_update, c->B, which, h, use_handle);
+    const int g = FE_NBR_PRESSURE_UPDATE;
+    if (!few(c)) return rec_shaped(c, R, g, k_pressure_update<kBlock>, c->B, which, h, use_handle);
+    if (which < 0) return rec_nbr(c, R, g, k_pressure_update_few, c->B);
+    REC(R.k(k_pressure_update<kFewThreads>, chunk_grid(c), dim3(kBlock), c->B, which, h,
+            use_handle));
+    return FE_OK;
 }
 
 // viscosity and the two source passes (plain or with the learned state)

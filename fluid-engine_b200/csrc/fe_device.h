@@ -16,6 +16,7 @@ namespace fe {
 
 constexpr int kBlock = 256;          // threads per block of particle kernels
 constexpr uint32_t kNbrCap = 64;     // neighbour-list capacity per particle
+constexpr int kFewThreads = 64;      // block of the neighbour passes for few particles
 
 // Parameters of one scene: `SimulationParams` (common.glsl:11-28) plus the
 // frame-driver knobs.  Written by the host (fe_set_params) and, for dt, by

@@ -370,8 +370,9 @@ __device__ __forceinline__ void coop_candidates(const Bufs& B, const DevParams& 
 
 // Blocks per SM the launch bounds ask for: 1024 resident threads per SM
 // (at most 64 registers per thread), for every block size.
+// (the shape for few particles takes the registers for its loads in flight)
 template <int kThreads>
-constexpr int kMinBlocks = 1024 / kThreads;
+constexpr int kMinBlocks = kThreads == kFewThreads ? 5 : 1024 / kThreads;
 
 // kDiv: 0 density and alpha only; 1 also the FIXED-mode divergence source
 // (velocity_b), 2 also the REFERENCE-mode one (velocity_a) -- see
@@ -532,6 +533,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>)
 // ---------------------------------------------------------------------------
 // viscosity.comp:17-66: velocity_b in, velocity_a out.
 // ---------------------------------------------------------------------------
+template <int kThreads>
 __device__ __forceinline__ void viscosity_particle(const Bufs& B, uint32_t i, uint32_t s) {
     const DevParams& P = B.P[s];
     const float m = P.mass, h = P.h;
@@ -542,7 +544,7 @@ __device__ __forceinline__ void viscosity_particle(const Bufs& B, uint32_t i, ui
     f3 sum = {0.0f, 0.0f, 0.0f};
     // velocity_b.w = m / rho_j (written by density_alpha): one 256-bit load of
     // the position/velocity record per neighbour
-    for_each_neighbor_pair(
+    for_each_neighbor_pair<kThreads>(
         B, P, i, pi, B.pv, [&](f3 rv, float, float4 vj) {
             float r2 = dot(rv, rv);
             float r = sqrtf(r2);
@@ -562,7 +564,7 @@ __device__ __forceinline__ void viscosity_particle(const Bufs& B, uint32_t i, ui
 template <int kThreads, bool kPersist>
 __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>) k_viscosity(Bufs B) {
     for_each_particle<kThreads, kPersist>(B, [&](uint32_t i, uint32_t s, bool live) {
-        if (live) viscosity_particle(B, i, s);
+        if (live) viscosity_particle<kThreads>(B, i, s);
     });
 }
 
@@ -570,12 +572,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>) k_viscosity(Bu
 // density_source_term.comp:16-74 (velocities = velocity_a).  The kLearn
 // variant also emits the warm-start features (same arithmetic for s and p).
 // ---------------------------------------------------------------------------
-struct VelRho {
-    float4 v;
-    float rho;
-};
-
-template <bool kLearn>
+template <int kThreads, bool kLearn>
 __device__ __forceinline__ void density_source_body(const Bufs& B, const LearnArgs& L,
                                                     uint32_t i, uint32_t s) {
     const DevParams& P = B.P[s];
@@ -585,7 +582,7 @@ __device__ __forceinline__ void density_source_body(const Bufs& B, const LearnAr
     float div = 0.0f;
     Moments mo;
     // velocity_a and (w) the density residual t of j from one load of its record
-    for_each_neighbor_pair(B, P, i, pi, B.pa, [&](f3 rv, float g, float4 vj) {
+    for_each_neighbor_pair<kThreads>(B, P, i, pi, B.pa, [&](f3 rv, float g, float4 vj) {
         f3 grad = scale(g, rv);
         f3 vd = sub(vi, xyz(vj));
         div += m * dot(vd, grad);
@@ -610,14 +607,14 @@ __device__ __forceinline__ void density_source_body(const Bufs& B, const LearnAr
 template <int kThreads, bool kPersist>
 __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>) k_density_source(Bufs B) {
     for_each_particle<kThreads, kPersist>(B, [&](uint32_t i, uint32_t s, bool live) {
-        if (live) density_source_body<false>(B, LearnArgs{}, i, s);
+        if (live) density_source_body<kThreads, false>(B, LearnArgs{}, i, s);
     });
 }
 template <int kThreads, bool kPersist>
 __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>)
     k_density_source_learn(Bufs B, LearnArgs L) {
     for_each_particle<kThreads, kPersist>(B, [&](uint32_t i, uint32_t s, bool live) {
-        if (live) density_source_body<true>(B, L, i, s);
+        if (live) density_source_body<kThreads, true>(B, L, i, s);
     });
 }
 
@@ -625,6 +622,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>)
 // divergence_source_term.comp:14-61 (velocities = velocity_a in REFERENCE
 // mode, velocity_b in FIXED mode).
 // ---------------------------------------------------------------------------
+template <int kThreads>
 __device__ __forceinline__ void divergence_source_body(const Bufs& B, int fixed, uint32_t i,
                                                        uint32_t s) {
     const DevParams& P = B.P[s];
@@ -632,19 +630,13 @@ __device__ __forceinline__ void divergence_source_body(const Bufs& B, int fixed,
     const f3 pi = xyz(__ldg(posb(B, i)));
     const f3 vi = xyz(__ldg(fixed ? velb(B, i) : vela(B, i)));
     float div = 0.0f;
-    auto term = [&](f3 rv, float g, float4 vj) {
-        f3 grad = scale(g, rv);
-        f3 vd = sub(vi, xyz(vj));
-        div += m * dot(vd, grad);
-    };
-    if (fixed) {
-        // velocity_b from the position/velocity record
-        for_each_neighbor_pair(B, P, i, pi, B.pv, [&](f3 rv, float g, float4 vj) { term(rv, g, vj); });
-    } else {
-        for_each_neighbor(
-            B, P, i, pi, [&](uint32_t j) { return __ldg(vela(B, j)); },
-            [&](uint32_t, f3 rv, float g, float4, float4 vj) { term(rv, g, vj); });
-    }
+    // both velocities sit in records that start with the position
+    for_each_neighbor_pair<kThreads>(B, P, i, pi, fixed ? B.pv : B.pa,
+                                     [&](f3 rv, float g, float4 vj) {
+                                         f3 grad = scale(g, rv);
+                                         f3 vd = sub(vi, xyz(vj));
+                                         div += m * dot(vd, grad);
+                                     });
     B.src[i] = -div;
 }
 
@@ -654,7 +646,7 @@ template <int kThreads, bool kPersist>
 __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>) k_divergence_source(Bufs B,
                                                                                       int fixed) {
     for_each_particle<kThreads, kPersist>(B, [&](uint32_t i, uint32_t s, bool live) {
-        if (live) divergence_source_body(B, fixed, i, s);
+        if (live) divergence_source_body<kThreads>(B, fixed, i, s);
     });
 }
 
@@ -662,6 +654,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>) k_divergence_s
 // pressure_force.comp:15-78.  pr[j] = p_j / rho_j^2 (NaN when rho_j <= 1e-6)
 // is maintained by every pass that writes p or rho.
 // ---------------------------------------------------------------------------
+template <int kThreads>
 __device__ __forceinline__ void pressure_force_particle(const Bufs& B, uint32_t i, uint32_t s) {
     const DevParams& P = B.P[s];
     const float m = P.mass;
@@ -671,16 +664,14 @@ __device__ __forceinline__ void pressure_force_particle(const Bufs& B, uint32_t 
     float p_rho_i = 0.0f;
     if (rho_i > kEpsR) p_rho_i = p_i / (rho_i * rho_i);
     f3 acc = {0.0f, 0.0f, 0.0f};
-    for_each_neighbor(
-        B, P, i, pi, [&](uint32_t) { return NoData{}; },
-        [&](uint32_t, f3 rv, float g, float4 qj, NoData) {
-            float p_rho_j = qj.w;  // p_j / rho_j^2, NaN when rho_j <= 1e-6
-            if (p_rho_j == p_rho_j) {
-                f3 grad = scale(g, rv);
-                float term = p_rho_i + p_rho_j;
-                acc = add(acc, scale(m * term, grad));
-            }
-        });
+    for_each_neighbor<kThreads>(B, P, i, pi, [&](f3 rv, float g, float4 qj) {
+        float p_rho_j = qj.w;  // p_j / rho_j^2, NaN when rho_j <= 1e-6
+        if (p_rho_j == p_rho_j) {
+            f3 grad = scale(g, rv);
+            float term = p_rho_i + p_rho_j;
+            acc = add(acc, scale(m * term, grad));
+        }
+    });
     // the whole record: this particle's position for pressure_update's
     // gathers and its acceleration
     st_record(B, i, p4, make_float4(-acc.x, -acc.y, -acc.z, 0.0f));
@@ -690,7 +681,8 @@ template <int kThreads, bool kPersist>
 __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>) k_pressure_force(Bufs B,
                                                                                    int which) {
     for_each_particle<kThreads, kPersist>(B, [&](uint32_t i, uint32_t s, bool live) {
-        if (live && !(which >= 0 && B.S[s].solve[which].done)) pressure_force_particle(B, i, s);
+        if (live && !(which >= 0 && B.S[s].solve[which].done))
+            pressure_force_particle<kThreads>(B, i, s);
     });
 }
 
@@ -819,6 +811,32 @@ __device__ __forceinline__ double pressure_update_particle(const Bufs& B, const 
     return e > 0.0f ? (double)e : 0.0;  // NaN -> 0
 }
 
+// The sum of particle i's pairs in the update.
+template <int kThreads>
+__device__ __forceinline__ float pressure_update_sum(const Bufs& B, const DevParams& P,
+                                                     uint32_t i) {
+    const float m = P.mass;
+    const f3 pi = xyz(__ldg(posb(B, i)));
+    const f3 ai = xyz(*accp(B, i));
+    float sum_ap = 0.0f;
+    for_each_neighbor_pair<kThreads>(B, P, i, pi, B.rec, [&](f3 rv, float g, float4 aj) {
+        f3 grad = scale(g, rv);
+        f3 ad = sub(ai, xyz(aj));
+        sum_ap += m * dot(ad, grad);
+    });
+    return sum_ap;
+}
+
+// The stage call for few particles: no control, so no chunk partials.
+__global__ void __launch_bounds__(kFewThreads, kMinBlocks<kFewThreads>)
+    k_pressure_update_few(Bufs B) {
+    for_each_particle<kFewThreads, false>(B, [&](uint32_t i, uint32_t s, bool live) {
+        if (!live) return;
+        const DevParams& P = B.P[s];
+        pressure_update_particle(B, P, i, -1, pressure_update_sum<kFewThreads>(B, P, i));
+    });
+}
+
 // Chunk c's partial of the fixed-order sum and its largest error (whole
 // block).
 __device__ __forceinline__ void solve_chunk_partials(const Bufs& B, uint32_t c, double e,
@@ -833,6 +851,9 @@ __device__ __forceinline__ void solve_chunk_partials(const Bufs& B, uint32_t c, 
 
 // One block per chunk, or a persistent grid whose blocks stride over the
 // chunks (the per-chunk partials, and so the sums, are the same).
+// kShape: the shape whose batches of list entries are used (the block has 256
+// threads either way: its partials are per chunk).
+template <int kShape>
 __global__ void __launch_bounds__(kBlock) k_pressure_update(Bufs B, int which,
                                                             cudaGraphConditionalHandle handle,
                                                             int use_handle) {
@@ -846,16 +867,8 @@ __global__ void __launch_bounds__(kBlock) k_pressure_update(Bufs B, int which,
         const bool skip = control && B.S[s].solve[which].done;
         double e_sum_in = 0.0;
         if (valid && !skip) {
-            const float m = P.mass;
-            const f3 pi = xyz(__ldg(posb(B, i)));
-            const f3 ai = xyz(*accp(B, i));
-            float sum_ap = 0.0f;
-            for_each_neighbor_record(B, P, i, pi, [&](f3 rv, float g, float4 aj) {
-                f3 grad = scale(g, rv);
-                f3 ad = sub(ai, xyz(aj));
-                sum_ap += m * dot(ad, grad);
-            });
-            e_sum_in = pressure_update_particle(B, P, i, which, sum_ap);
+            e_sum_in = pressure_update_particle(B, P, i, which,
+                                                pressure_update_sum<kShape>(B, P, i));
         }
         if (control && !skip && P.solver == 1u) solve_chunk_partials(B, c, e_sum_in, smem);
     }
@@ -1269,12 +1282,15 @@ __global__ void k_count_substep(Bufs B) {
     template __global__ void k_density_source_learn<T, P>(Bufs, LearnArgs);           \
     template __global__ void k_divergence_source<T, P>(Bufs, int);                    \
     template __global__ void k_pressure_force<T, P>(Bufs, int);
+FE_NBR_INSTANTIATE(kFewThreads, false)
 FE_NBR_INSTANTIATE(128, false)
 FE_NBR_INSTANTIATE(256, false)
 FE_NBR_INSTANTIATE(512, false)
 FE_NBR_INSTANTIATE(128, true)
 FE_NBR_INSTANTIATE(256, true)
 FE_NBR_INSTANTIATE(512, true)
+template __global__ void k_pressure_update<kBlock>(Bufs, int, cudaGraphConditionalHandle, int);
+template __global__ void k_pressure_update<kFewThreads>(Bufs, int, cudaGraphConditionalHandle, int);
 template __global__ void k_density_alpha<128, false>(Bufs);
 template __global__ void k_density_alpha<256, false>(Bufs);
 template __global__ void k_density_alpha<128, true>(Bufs);

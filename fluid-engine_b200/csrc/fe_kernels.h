@@ -40,8 +40,10 @@ template <int kThreads, bool kPersist>
 __global__ void k_divergence_source(Bufs B, int fixed);
 template <int kThreads, bool kPersist>
 __global__ void k_pressure_force(Bufs B, int which);
+template <int kShape>
 __global__ void k_pressure_update(Bufs B, int which, cudaGraphConditionalHandle handle,
                                   int use_handle);
+__global__ void k_pressure_update_few(Bufs B);
 __global__ void k_solve_begin(Bufs B, int which, cudaGraphConditionalHandle handle,
                               int use_handle);
 // The density solve's first iteration from the plain (zero) start.

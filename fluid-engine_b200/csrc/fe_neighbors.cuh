@@ -16,6 +16,14 @@ __device__ __forceinline__ bool chunk_of(const Bufs& B, uint32_t& i, uint32_t& s
     return threadIdx.x < c.y;
 }
 
+// The shape of the neighbour passes for few particles: blocks of 64 threads, a
+// quarter of a chunk each, so that the particles spread over all SMs, and
+// deep batches of list entries (for_each_entry).
+template <int kThreads>
+constexpr int kEntryBatch = kThreads == kFewThreads ? 12 : 4;
+template <int kThreads>
+constexpr bool kEntryAhead = kThreads == kFewThreads;
+
 // Block-size-agnostic particle loop of the neighbour kernels over the chunk
 // table (the scene-offset table: every chunk is <= 256 consecutive particles
 // of one scene).  A block of kThreads threads takes kThreads / 256 chunks at a
@@ -27,7 +35,9 @@ __device__ __forceinline__ bool chunk_of(const Bufs& B, uint32_t& i, uint32_t& s
 // warp together (live: i is a particle of the chunk).
 template <int kThreads>
 struct ParticleLoop {
-    static_assert(kThreads == 128 || kThreads == 256 || kThreads == 512, "block size");
+    static_assert(kThreads == kFewThreads || kThreads == 128 || kThreads == 256 ||
+                      kThreads == 512,
+                  "block size");
     static constexpr uint32_t kChunksPerStep = kThreads >= kBlock ? kThreads / kBlock : 1;
     static constexpr uint32_t kPasses = kThreads >= kBlock ? 1 : kBlock / kThreads;
 };
@@ -37,6 +47,19 @@ struct ParticleLoop {
 template <int kThreads, bool kPersist, class F>
 __device__ __forceinline__ void for_each_particle(const Bufs& B, F&& f) {
     using L = ParticleLoop<kThreads>;
+    if constexpr (kThreads == kFewThreads) {
+        static_assert(!kPersist, "one block per quarter chunk");
+        constexpr uint32_t per = kBlock / kFewThreads;
+        if (B.n_scenes == 1) {   // chunk c starts at 256 c: no table read
+            const uint32_t i = blockIdx.x * kFewThreads + threadIdx.x;
+            f(i, 0u, i < B.n_total);
+        } else {
+            const uint4 cc = B.chunks[blockIdx.x / per];
+            const uint32_t off = (blockIdx.x % per) * kFewThreads + threadIdx.x;
+            f(cc.x + off, cc.z, off < cc.y);
+        }
+        return;
+    }
     const uint32_t sub = kThreads >= kBlock ? threadIdx.x / kBlock : 0u;
     const uint32_t t = kThreads >= kBlock ? threadIdx.x % kBlock : threadIdx.x;
     auto step = [&](uint32_t c0) {
@@ -101,87 +124,101 @@ __device__ __forceinline__ uint2 ld_list(const uint2* p, uint64_t pol) {
     return v;
 }
 
-// Neighbours with r > 1e-6 in walk order: f(j, r_vec, grad_scale, pos_j, d_j)
-// where pos_j = pos_b[j] (w = p_j / rho_j^2) and d_j = gather(j).  List
-// entries are consumed four at a time with all their loads issued before the
-// arithmetic, which then runs strictly in list order.
-template <class G, class F>
-__device__ __forceinline__ void for_each_neighbor(const Bufs& B, const DevParams& P, uint32_t i,
-                                                  f3 pi, G&& gather, F&& f) {
-    const uint32_t cnt = B.nbr_count[i];
-    if (cnt <= kNbrCap) {
-        const uint2* e = B.nbr + i;
-        const size_t stride = B.n_total;
-        const uint64_t pol = evict_first_policy();
+// The list entries of particle i in order: f(entry, load(entry.x)).  kBatch
+// entries at a time, all their loads issued before the arithmetic, which runs
+// strictly in list order.
+// kAhead: also the next batch's list words are loaded before this batch's
+// gathers are used.  The shape for few particles (see kFewParticles), where a
+// pass is one chain of load latencies per thread and nothing else hides them;
+// with many particles the passes are bound by the gathers' throughput and the
+// registers cost more than the order gains.
+template <int kBatch, bool kAhead, class Load, class F>
+__device__ __forceinline__ void for_each_entry(const Bufs& B, uint32_t i, uint32_t cnt,
+                                               Load&& load, F&& f) {
+    const uint2* e = B.nbr + i;
+    const size_t stride = B.n_total;
+    const uint64_t pol = evict_first_policy();
+    uint2 v[kBatch];
+    decltype(load(0u)) d[kBatch];
+    if constexpr (kAhead) {
+        uint2 next[kBatch];
+#pragma unroll
+        for (int q = 0; q < kBatch; ++q)
+            if (q < cnt) next[q] = ld_list(e + q * stride, pol);
+        for (uint32_t k = 0; k < cnt; k += kBatch) {
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) {
+                v[q] = next[q];
+                if (k + q < cnt) d[q] = load(v[q].x);
+            }
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q)
+                if (k + kBatch + q < cnt) next[q] = ld_list(e + (k + kBatch + q) * stride, pol);
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q)
+                if (k + q < cnt) f(v[q], d[q]);
+        }
+    } else {
         uint32_t k = 0;
-        for (; k + 4 <= cnt; k += 4) {
-            uint2 v0 = ld_list(e + (k + 0) * stride, pol);
-            uint2 v1 = ld_list(e + (k + 1) * stride, pol);
-            uint2 v2 = ld_list(e + (k + 2) * stride, pol);
-            uint2 v3 = ld_list(e + (k + 3) * stride, pol);
-            float4 q0 = __ldg(posb(B, v0.x)), q1 = __ldg(posb(B, v1.x));
-            float4 q2 = __ldg(posb(B, v2.x)), q3 = __ldg(posb(B, v3.x));
-            auto d0 = gather(v0.x);
-            auto d1 = gather(v1.x);
-            auto d2 = gather(v2.x);
-            auto d3 = gather(v3.x);
-            f(v0.x, sub(pi, xyz(q0)), __uint_as_float(v0.y), q0, d0);
-            f(v1.x, sub(pi, xyz(q1)), __uint_as_float(v1.y), q1, d1);
-            f(v2.x, sub(pi, xyz(q2)), __uint_as_float(v2.y), q2, d2);
-            f(v3.x, sub(pi, xyz(q3)), __uint_as_float(v3.y), q3, d3);
+        for (; k + kBatch <= cnt; k += kBatch) {
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) v[q] = ld_list(e + (k + q) * stride, pol);
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) d[q] = load(v[q].x);
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) f(v[q], d[q]);
         }
         for (; k < cnt; ++k) {
-            uint2 v = ld_list(e + k * stride, pol);
-            float4 q = __ldg(posb(B, v.x));
-            f(v.x, sub(pi, xyz(q)), __uint_as_float(v.y), q, gather(v.x));
+            v[0] = ld_list(e + k * stride, pol);
+            f(v[0], load(v[0].x));
         }
+    }
+}
+
+// Neighbours with r > 1e-6 in walk order: f(r_vec, grad_scale, pos_j), where
+// pos_j = pos_b[j] (w = p_j / rho_j^2).
+template <int kThreads, class F>
+__device__ __forceinline__ void for_each_neighbor(const Bufs& B, const DevParams& P, uint32_t i,
+                                                  f3 pi, F&& f) {
+    const uint32_t cnt = B.nbr_count[i];
+    if (cnt <= kNbrCap) {
+        for_each_entry<kEntryBatch<kThreads>, kEntryAhead<kThreads>>(
+            B, i, cnt, [&](uint32_t j) { return __ldg(posb(B, j)); },
+            [&](uint2 v, float4 q) { f(sub(pi, xyz(q)), __uint_as_float(v.y), q); });
     } else {
         const float h = P.h;
         walk(B, P, pi, [&](uint32_t j, f3 rv, float r2) {
             float r = sqrtf(r2);
-            if (r > kEpsR) f(j, rv, kernel_grad_scale(r, h), __ldg(posb(B, j)), gather(j));
+            if (r > kEpsR) f(rv, kernel_grad_scale(r, h), __ldg(posb(B, j)));
         });
     }
 }
-
-struct NoData {};
 
 // As for_each_neighbor, over a 32-byte record array whose first half of
 // record j is a copy of position_b: f(r_vec, grad_scale, second_half_j), with
 // both halves of j fetched by one 256-bit load.  B.rec (position,
 // acceleration) for pressure_update, B.pv (position, velocity_b) for
-// viscosity and the FIXED-mode divergence source.
-template <class F>
+// viscosity and the FIXED-mode divergence source, B.pa (position,
+// velocity_a) for the density source and the REFERENCE-mode divergence source.
+struct Pair {
+    float4 pos, data;
+};
+template <int kThreads, class F>
 __device__ __forceinline__ void for_each_neighbor_pair(const Bufs& B, const DevParams& P,
                                                        uint32_t i, f3 pi, const float4* recs,
                                                        F&& f) {
     const uint32_t cnt = B.nbr_count[i];
     if (cnt <= kNbrCap) {
-        const uint2* e = B.nbr + i;
-        const size_t stride = B.n_total;
-        const uint64_t pol = evict_first_policy();
-        uint32_t k = 0;
-        for (; k + 4 <= cnt; k += 4) {
-            uint2 v0 = ld_list(e + (k + 0) * stride, pol);
-            uint2 v1 = ld_list(e + (k + 1) * stride, pol);
-            uint2 v2 = ld_list(e + (k + 2) * stride, pol);
-            uint2 v3 = ld_list(e + (k + 3) * stride, pol);
-            float4 q0, a0, q1, a1, q2, a2, q3, a3;
-            ld_pair(recs, v0.x, q0, a0);
-            ld_pair(recs, v1.x, q1, a1);
-            ld_pair(recs, v2.x, q2, a2);
-            ld_pair(recs, v3.x, q3, a3);
-            f(sub(pi, xyz(q0)), __uint_as_float(v0.y), a0);
-            f(sub(pi, xyz(q1)), __uint_as_float(v1.y), a1);
-            f(sub(pi, xyz(q2)), __uint_as_float(v2.y), a2);
-            f(sub(pi, xyz(q3)), __uint_as_float(v3.y), a3);
-        }
-        for (; k < cnt; ++k) {
-            uint2 v = ld_list(e + k * stride, pol);
-            float4 q, a;
-            ld_pair(recs, v.x, q, a);
-            f(sub(pi, xyz(q)), __uint_as_float(v.y), a);
-        }
+        for_each_entry<kEntryBatch<kThreads>, kEntryAhead<kThreads>>(
+            B, i, cnt,
+            [&](uint32_t j) {
+                Pair p;
+                ld_pair(recs, j, p.pos, p.data);
+                return p;
+            },
+            [&](uint2 v, const Pair& p) {
+                f(sub(pi, xyz(p.pos)), __uint_as_float(v.y), p.data);
+            });
     } else {
         const float h = P.h;
         walk(B, P, pi, [&](uint32_t j, f3 rv, float r2) {
@@ -189,12 +226,6 @@ __device__ __forceinline__ void for_each_neighbor_pair(const Bufs& B, const DevP
             if (r > kEpsR) f(rv, kernel_grad_scale(r, h), __ldg(recs + 2 * (size_t)j + 1));
         });
     }
-}
-
-template <class F>
-__device__ __forceinline__ void for_each_neighbor_record(const Bufs& B, const DevParams& P,
-                                                         uint32_t i, f3 pi, F&& f) {
-    for_each_neighbor_pair(B, P, i, pi, B.rec, f);
 }
 
 }  // namespace fe
