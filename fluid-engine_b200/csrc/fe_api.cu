@@ -332,9 +332,7 @@ struct fe_ctx {
     std::vector<fe_params> params;  // host copy per scene
     std::vector<DevParams> dparams;
     Bufs B;
-    uint32_t* tmp_keys = nullptr;
-    uint32_t* tmp_vals = nullptr;
-    uint32_t* sort_scratch = nullptr;
+    CellSort cell_sort{};
     uint4* upart = nullptr;
     uint32_t key_bits = 32;
     bool prepared = false;
@@ -624,41 +622,36 @@ fe_status rec_list_pass(fe_ctx* c, Recorder& R, int pass) {
 // current; the substep's search leaves it to density_alpha_div, which runs
 // next and does it per particle.
 fe_status rec_neighbor_search(fe_ctx* c, Recorder& R, bool take = true) {
-    Bufs B = c->B;
-    const bool radix = c->sort_algorithm() == FE_SORT_RADIX;
-    uint32_t passes = radix_passes(c->key_bits, c->radix_cfg.digit_bits);
-    // Radix ping-pongs through tmp; hashing into tmp when the pass count is
-    // odd leaves the sorted entries in keys/vals.
-    Bufs H = B;
-    if (radix && (passes % 2 == 1)) {
-        H.keys = c->tmp_keys;
-        H.vals = c->tmp_vals;
-    }
-    REC(R.k(k_hash, chunk_grid(c), dim3(kBlock), H));
-    SortLaunch L = R.sort_launch();
-    if (radix) {
-        bool in_tmp = false;
-        REC(radix_sort(L, H.keys, H.vals, H.keys == B.keys ? c->tmp_keys : B.keys,
-                       H.vals == B.vals ? c->tmp_vals : B.vals, c->n, c->key_bits,
-                       c->sort_scratch, &B.G->flags, &in_tmp, c->radix_cfg));
-    } else {
-        REC(bitonic_sort(L, B.keys, B.vals, c->T));
-    }
-    REC(R.k(k_fill_cells, dim3(std::min<uint32_t>((c->T + 255) / 256, 148 * 8)), dim3(256),
-            B.cells, (size_t)c->T));
-    REC(R.k(k_offsets, flat_grid(c->n), dim3(kBlock), B));
+    const Bufs B = c->B;
     const int fixed = c->fixed_mode() ? 1 : 0;
-    if (c->carries()) {
-        // the learned state rides along with the gather and the copy-back
-        REC(R.k(k_reorder_carry, flat_grid(c->n), dim3(kBlock), B, fixed, c->L));
-        if (!take) return FE_OK;
+    if (c->sort_algorithm() == FE_SORT_RADIX) {
+        const CellSort C = c->cell_sort;
+        REC(R.k(k_cell_count, chunk_grid(c), dim3(kBlock), B, C));
+        REC(R.k(k_cell_scan, dim3((c->T + kScanTile - 1) / kScanTile), dim3(kScanThreads), B, C));
+        REC(R.k(k_cell_scatter, flat_grid(c->n), dim3(kBlock), B, C));
+        if (c->carries())  // the learned state rides along with the gather
+            REC(R.k(k_cell_reorder_carry, flat_grid(c->n), dim3(kBlock), B, C, fixed, c->L));
+        else
+            REC(R.k(k_cell_reorder, flat_grid(c->n), dim3(kBlock), B, C, fixed));
+    } else {
+        REC(R.k(k_hash, chunk_grid(c), dim3(kBlock), B));
+        REC(bitonic_sort(R.sort_launch(), B.keys, B.vals, c->T));
+        REC(R.k(k_fill_cells, dim3(std::min<uint32_t>((c->T + 255) / 256, 148 * 8)), dim3(256),
+                B.cells, (size_t)c->T));
+        REC(R.k(k_offsets, flat_grid(c->n), dim3(kBlock), B));
+        if (c->carries())
+            REC(R.k(k_reorder_carry, flat_grid(c->n), dim3(kBlock), B, fixed, c->L));
+        else
+            REC(R.k(k_reorder, flat_grid(c->n), dim3(kBlock), B, fixed));
+    }
+    if (!take) return FE_OK;
+    if (c->carries()) {   // and with the copy-back
         if (fixed)
             REC(R.k(k_take_pressure_carry, flat_grid(c->n), dim3(kBlock), B, c->L));
         else
             REC(R.k(k_carry_take, flat_grid(c->n), dim3(kBlock), B, c->L));
-    } else {
-        REC(R.k(k_reorder, flat_grid(c->n), dim3(kBlock), B, fixed));
-        if (fixed && take) REC(R.k(k_take_pressure, flat_grid(c->n), dim3(kBlock), B));
+    } else if (fixed) {
+        REC(R.k(k_take_pressure, flat_grid(c->n), dim3(kBlock), B));
     }
     return FE_OK;
 }
@@ -1176,7 +1169,8 @@ fe_status create_ctx(const fe_params* params, const uint32_t* counts, uint32_t n
     B.n_chunks = nchunks;
     B.n_scenes = n_scenes;
     uint4* chunks_d = nullptr;
-    const size_t scratch_words = radix_scratch_words_any(n, c->key_bits);
+    CellSort& cs = c->cell_sort;
+    const uint32_t scan_tiles = (c->T + kScanTile - 1) / kScanTile;
     if ((s = dev_alloc(c, &B.pos_a, n)) || (s = dev_alloc(c, &B.pos_b, n)) ||
         (s = dev_alloc(c, &B.rec, 2 * (size_t)n)) ||
         (s = dev_alloc(c, &B.pa, 2 * (size_t)n)) || (s = dev_alloc(c, &B.pv, 2 * (size_t)n)) ||
@@ -1189,9 +1183,10 @@ fe_status create_ctx(const fe_params* params, const uint32_t* counts, uint32_t n
         (s = dev_alloc(c, &chunks_d, nchunks)) || (s = dev_alloc(c, &B.P, n_scenes)) ||
         (s = dev_alloc(c, &B.S, n_scenes)) || (s = dev_alloc(c, &B.G, 1)) ||
         (s = dev_alloc(c, &B.partials, 2 * (size_t)nchunks)) ||
-        (s = dev_alloc(c, &c->upart, nchunks)) || (s = dev_alloc(c, &c->tmp_keys, n)) ||
-        (s = dev_alloc(c, &c->tmp_vals, n)) ||
-        (s = dev_alloc(c, &c->sort_scratch, scratch_words)))
+        (s = dev_alloc(c, &c->upart, nchunks)) || (s = dev_alloc(c, &cs.count, c->T)) ||
+        (s = dev_alloc(c, &cs.key, n)) || (s = dev_alloc(c, &cs.place, n)) ||
+        (s = dev_alloc(c, &cs.slot, n)) ||
+        (s = dev_alloc(c, &cs.status, (size_t)scan_tiles + 1)))
         return fail(s);
     B.chunks = chunks_d;
     if (cudaMallocHost(&c->h_state, sizeof(SceneState) * n_scenes) != cudaSuccess ||
@@ -1224,6 +1219,9 @@ fe_status create_ctx(const fe_params* params, const uint32_t* counts, uint32_t n
             FE_CUDA(cudaMemset(B.vals + n, 0xFF, (size_t)(c->T - n) * 4));
         }
         FE_CUDA(cudaMemset(B.cells, 0xFF, (size_t)c->T * 8));
+        cs.ticket = cs.status + scan_tiles;
+        FE_CUDA(cudaMemset(cs.count, 0, (size_t)c->T * 4));
+        FE_CUDA(cudaMemset(cs.status, 0, ((size_t)scan_tiles + 1) * 8));
         FE_CUDA(cudaMemset(B.S, 0, sizeof(SceneState) * n_scenes));
         FE_CUDA(cudaMemset(B.G, 0, sizeof(GlobalState)));
         FE_CUDA(cudaMemcpy(B.P, c->dparams.data(), sizeof(DevParams) * n_scenes,

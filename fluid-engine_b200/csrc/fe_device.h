@@ -119,6 +119,17 @@ struct Bufs {
     uint32_t n_total, T_total, n_chunks, n_scenes;
 };
 
+// Scratch of the search by cell counts (k_cell_*).
+constexpr uint32_t kScanTile = 4096;   // table slots per block of k_cell_scan
+constexpr int kScanThreads = 512;
+constexpr int kScanSpins = 1 << 22;    // bound of its look-back wait
+struct CellSort {
+    uint32_t* count;              // per table slot; zero between searches
+    uint32_t *key, *place, *slot; // per particle
+    unsigned long long* status;   // per tile of the scan
+    unsigned long long* ticket;
+};
+
 // Learned warm start and training-data capture (fe_learned.cu).
 // carry[i] travels with particle i through every re-sort:
 //   x = final pressure of the last density solve, y = of the last

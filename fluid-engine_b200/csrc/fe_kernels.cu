@@ -70,12 +70,8 @@ __global__ void k_offsets(Bufs B) {
 // read-modify-write of pos_b, no half-written record): partial sectors
 // made this pass about twice as slow.
 template <bool kCarry>
-__device__ __forceinline__ void reorder_body(const Bufs& B, int carry_pressure,
-                                             const LearnArgs& L) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B.n_total) return;
-    uint32_t src = B.vals[i];
-    if (src >= B.n_total) src = i;  // unreachable for a valid permutation
+__device__ __forceinline__ void reorder_slot(const Bufs& B, int carry_pressure,
+                                             const LearnArgs& L, uint32_t i, uint32_t src) {
     B.nbr_count[i] = kNbrCap + 1;
     // pos_b.w holds p / rho^2 of slot i (pressures and densities are not
     // permuted here): the value every pass that writes p or rho maintains,
@@ -96,12 +92,227 @@ __device__ __forceinline__ void reorder_body(const Bufs& B, int carry_pressure,
     }
 }
 
+template <bool kCarry>
+__device__ __forceinline__ void reorder_body(const Bufs& B, int carry_pressure,
+                                             const LearnArgs& L) {
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= B.n_total) return;
+    uint32_t src = B.vals[i];
+    if (src >= B.n_total) src = i;  // unreachable for a valid permutation
+    reorder_slot<kCarry>(B, carry_pressure, L, i, src);
+}
+
 __global__ void __launch_bounds__(kBlock) k_reorder(Bufs B, int carry_pressure) {
     reorder_body<false>(B, carry_pressure, LearnArgs{});
 }
 __global__ void __launch_bounds__(kBlock) k_reorder_carry(Bufs B, int carry_pressure,
                                                           LearnArgs L) {
     reorder_body<true>(B, carry_pressure, L);
+}
+
+// ---------------------------------------------------------------------------
+// The search by cell counts (radix selected): the stable sort of the cell
+// hashes as a counting sort over the table itself, which also yields the
+// bucket bounds.
+//   k_cell_count    hash of every particle; its cell's counter gives it a
+//                   place among the cell's particles, in no particular order
+//   k_cell_scan     exclusive sum over the table: {start, end} per slot
+//   k_cell_scatter  particle indices to start + place
+//   k_cell_reorder  each entry finds its rank among its cell's indices (so
+//                   the order is the stable sort's) and takes the particle's
+//                   state to that slot
+// Four launches instead of hash, scratch fill, histogram, 2-4 radix passes,
+// table fill, offsets and reorder, and 4 bytes moved per particle and pass
+// instead of 16.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t particle_key(const DevParams& P, f3 p) {
+    const float h = P.h;
+    return P.table_base + cell_hash_pow2(cell_coord(p.x, h), cell_coord(p.y, h),
+                                         cell_coord(p.z, h), P.T - 1u);
+}
+
+// The warp's particles come in the last search's order, so neighbours in the
+// warp mostly share a cell: one atomic per run of equal keys.  All 32 lanes.
+__device__ __forceinline__ void cell_count(const CellSort& C, uint32_t i, uint32_t key,
+                                           bool live) {
+    const uint32_t lane = threadIdx.x & 31u;
+    if (!live) key = kEmpty;
+    const uint32_t prev = __shfl_up_sync(kFull, key, 1);
+    const bool head = lane == 0 || prev != key;
+    const uint32_t heads = __ballot_sync(kFull, head);
+    const uint32_t mine = 31u - __clz(heads & (kFull >> (31u - lane)));  // head of my run
+    const uint32_t after = heads & ~(kFull >> (31u - lane));
+    const uint32_t next = after ? __ffs(after) - 1u : 32u;
+    uint32_t place = 0;
+    if (head && live) place = atomicAdd(C.count + key, next - lane);
+    place = __shfl_sync(kFull, place, mine) + (lane - mine);
+    if (!live) return;
+    C.key[i] = key;
+    C.place[i] = place;
+}
+
+__global__ void __launch_bounds__(kBlock) k_cell_count(Bufs B, CellSort C) {
+    uint32_t i, s, c;
+    const bool live = chunk_of(B, i, s, c);
+    const DevParams& P = B.P[s];
+    const float4 p = live ? __ldg(B.pos_a + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    cell_count(C, i, particle_key(P, xyz(p)), live);
+}
+
+// Single-pass scan with decoupled look-back: a tile of kScanTile slots per
+// block, taken in ticket order.  A status word holds the launch's number next
+// to its state, so nothing has to be cleared between searches; the counters
+// are left at zero for the next one.
+constexpr unsigned long long kScanSum = 1ull << 32, kScanPrefix = 2ull << 32;
+// A thread owns 8 slots, 32 bytes of counters and 64 of bounds, so every access
+// is to whole sectors (16 slots a thread: 15.7 us at 2^20 slots; 8: 9 us).
+__global__ void __launch_bounds__(kScanThreads) k_cell_scan(Bufs B, CellSort C) {
+    constexpr int kWarps = kScanThreads / 32;
+    __shared__ uint32_t s_warp[kWarps], s_base;
+    __shared__ unsigned long long s_ticket;
+    if (threadIdx.x == 0) s_ticket = atomicAdd(C.ticket, 1ull);
+    __syncthreads();
+    const uint32_t tile = (uint32_t)(s_ticket % gridDim.x);
+    const unsigned long long epoch = ((s_ticket / gridDim.x) + 1ull) << 34;
+    constexpr int kPer = kScanTile / kScanThreads;
+    static_assert(kPer == 8, "two 16-byte loads and two 32-byte stores per thread");
+    const uint32_t k0 = tile * kScanTile + threadIdx.x * kPer;
+    uint32_t cnt[kPer], sum = 0;
+    if (k0 + kPer <= B.T_total) {
+#pragma unroll
+        for (int q = 0; q < kPer; q += 4) {
+            uint4* p = reinterpret_cast<uint4*>(C.count + k0 + q);
+            const uint4 v = *p;
+            *p = make_uint4(0u, 0u, 0u, 0u);
+            cnt[q] = v.x; cnt[q + 1] = v.y; cnt[q + 2] = v.z; cnt[q + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+            cnt[q] = 0;
+            if (k0 + q < B.T_total) {
+                cnt[q] = C.count[k0 + q];
+                C.count[k0 + q] = 0;
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) sum += cnt[q];
+    // exclusive sum over the block
+    const int lane = lane_id(), warp = threadIdx.x >> 5;
+    uint32_t x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s_warp[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t w = lane < kWarps ? s_warp[lane] : 0u, total = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, total, o);
+            if (lane >= o) total += y;
+        }
+        if (lane < kWarps) s_warp[lane] = total - w;
+        total = __shfl_sync(kFull, total, 31);
+        // this tile's sum, then the sums of the tiles before it: 32 status
+        // words at a time, nearest last, until one holds a whole prefix
+        volatile unsigned long long* st = C.status;
+        if (lane == 0) {
+            st[tile] = epoch | (tile == 0 ? kScanPrefix : kScanSum) | total;
+        }
+        uint32_t base = 0;
+        int pred = (int)tile - 1 - lane;
+        int spins = 0;
+        bool ok = true;
+        for (int last = (int)tile - 1; ok && last >= 0;) {
+            pred = last - lane;
+            unsigned long long v = epoch | kScanPrefix;   // before tile 0: 0
+            if (pred >= 0) v = st[pred];
+            const bool ready = (v >> 34) == (epoch >> 34);
+            const uint32_t not_ready = __ballot_sync(kFull, !ready);
+            const uint32_t whole = __ballot_sync(kFull, ready && (v & kScanPrefix));
+            // usable: the words up to the nearest whole prefix, or up to the
+            // first one that is not there yet
+            const uint32_t stop = whole ? __ffs(whole) : 33u;           // count to take
+            const uint32_t gap = not_ready ? __ffs(not_ready) - 1u : 32u;
+            const uint32_t take = min(stop, gap);
+            uint32_t part = (uint32_t)lane < take ? (uint32_t)v : 0u;
+#pragma unroll
+            for (int m = 16; m >= 1; m >>= 1) part += __shfl_xor_sync(kFull, part, m);
+            base += part;
+            if (stop <= gap) break;
+            last -= (int)take;
+            if (take == 0) {
+                if (++spins > kScanSpins) ok = false;
+                __nanosleep(32);
+            }
+        }
+        if (lane == 0) {
+            if (!ok) atomicOr(&B.G->flags, 0x4u);
+            if (tile) st[tile] = epoch | kScanPrefix | (unsigned long long)(base + total);
+            s_base = base;
+        }
+    }
+    __syncthreads();
+    uint32_t start = s_base + s_warp[warp] + (x - sum);
+    uint2 cell[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        cell[q] = cnt[q] ? make_uint2(start, start + cnt[q]) : make_uint2(kEmpty, kEmpty);
+        start += cnt[q];
+    }
+    if (k0 + kPer <= B.T_total) {
+#pragma unroll
+        for (int q = 0; q < kPer; q += 4)
+            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(
+                             B.cells + k0 + q),
+                         "r"(cell[q].x), "r"(cell[q].y), "r"(cell[q + 1].x), "r"(cell[q + 1].y),
+                         "r"(cell[q + 2].x), "r"(cell[q + 2].y), "r"(cell[q + 3].x),
+                         "r"(cell[q + 3].y)
+                         : "memory");
+    } else {
+#pragma unroll
+        for (int q = 0; q < kPer; ++q)
+            if (k0 + q < B.T_total) B.cells[k0 + q] = cell[q];
+    }
+}
+
+__global__ void __launch_bounds__(kBlock) k_cell_scatter(Bufs B, CellSort C) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= B.n_total) return;
+    const uint32_t at = B.cells[C.key[i]].x + C.place[i];
+    if (at < B.n_total) C.slot[at] = i;  // always, unless a scan's wait gave up
+}
+
+template <bool kCarry>
+__device__ __forceinline__ void cell_reorder(const Bufs& B, const CellSort& C, int carry_pressure,
+                                             const LearnArgs& L, uint32_t t) {
+    uint32_t src = __ldcg(C.slot + t);
+    if (src >= B.n_total) src = t;  // unreachable, unless a scan's wait gave up
+    const uint32_t key = C.key[src];
+    const uint2 cell = B.cells[key];
+    uint32_t i = t;
+    if (cell.x <= t && t < cell.y && cell.y <= B.n_total) {
+        uint32_t rank = 0;
+        for (uint32_t q = cell.x; q < cell.y; ++q) rank += C.slot[q] < src;
+        i = cell.x + rank;
+    }
+    if (i >= B.n_total) return;
+    B.keys[i] = key;
+    B.vals[i] = src;
+    reorder_slot<kCarry>(B, carry_pressure, L, i, src);
+}
+__global__ void __launch_bounds__(kBlock) k_cell_reorder(Bufs B, CellSort C, int carry_pressure) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < B.n_total) cell_reorder<false>(B, C, carry_pressure, LearnArgs{}, t);
+}
+__global__ void __launch_bounds__(kBlock) k_cell_reorder_carry(Bufs B, CellSort C,
+                                                               int carry_pressure, LearnArgs L) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < B.n_total) cell_reorder<true>(B, C, carry_pressure, L, t);
 }
 
 // FIXED mode: the gathered pressures become current; pr = p / rho^2 keeps

@@ -19,6 +19,11 @@ __global__ void k_hash(Bufs B);
 __global__ void k_offsets(Bufs B);
 __global__ void k_reorder(Bufs B, int carry_pressure);
 __global__ void k_reorder_carry(Bufs B, int carry_pressure, LearnArgs L);
+__global__ void k_cell_count(Bufs B, CellSort C);
+__global__ void k_cell_scan(Bufs B, CellSort C);
+__global__ void k_cell_scatter(Bufs B, CellSort C);
+__global__ void k_cell_reorder(Bufs B, CellSort C, int carry_pressure);
+__global__ void k_cell_reorder_carry(Bufs B, CellSort C, int carry_pressure, LearnArgs L);
 __global__ void k_take_pressure(Bufs B);
 __global__ void k_take_pressure_carry(Bufs B, LearnArgs L);
 __global__ void k_refresh_pr(Bufs B);
