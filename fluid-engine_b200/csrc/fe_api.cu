@@ -523,6 +523,10 @@ fe_status rec_check(cudaError_t e, const char* what) {
         if (s_ != FE_OK) return s_;                            \
     } while (0)
 
+// The blocks of 64 threads, four per chunk, of density_alpha and of the passes
+// for few particles.
+dim3 quarter_grid(const fe_ctx* c) { return dim3(c->B.n_chunks * (kBlock / kFewThreads)); }
+
 // A kernel of group g with its tuned shape.
 template <class... KArgs, class... Args>
 fe_status rec_shaped(fe_ctx* c, Recorder& R, int g, void (*func)(KArgs...), Args... args) {
@@ -535,48 +539,29 @@ fe_status rec_shaped(fe_ctx* c, Recorder& R, int g, void (*func)(KArgs...), Args
 template <class... KArgs, class... Args>
 fe_status rec_nbr(fe_ctx* c, Recorder& R, int g, void (*func)(KArgs...), Args... args) {
     if (few(c)) {
-        REC(R.k(func, dim3(c->B.n_chunks * (kBlock / kFewThreads)), dim3(kFewThreads), args...));
+        REC(R.k(func, quarter_grid(c), dim3(kFewThreads), args...));
         return FE_OK;
     }
     return rec_shaped(c, R, g, func, args...);
 }
 
-// (128 or 256 threads: the shapes fe_set_tuning accepts for this group)
+// (its one shape: the shapes fe_set_tuning takes for this group are accepted
+// and make no difference)
 fe_status rec_density_alpha(fe_ctx* c, Recorder& R) {
-    const int g = FE_NBR_DENSITY_ALPHA;
-    const uint32_t t = c->nbr_threads[g];
-    return rec_shaped(c, R, g,
-                   c->nbr_persistent[g]
-                       ? pick(k_density_alpha<128, true>, k_density_alpha<256, true>,
-                              k_density_alpha<256, true>, t)
-                       : pick(k_density_alpha<128, false>, k_density_alpha<256, false>,
-                              k_density_alpha<256, false>, t),
-                   c->B);
+    REC(R.k(k_density_alpha, quarter_grid(c), dim3(kFewThreads), c->B));
+    return FE_OK;
 }
 
 // density_alpha that also sums the divergence source (the mid-substep
 // neighbour search's pass); with the learned state it also emits the
 // divergence solve's features.
 fe_status rec_density_alpha_div(fe_ctx* c, Recorder& R) {
-    const int g = FE_NBR_DENSITY_ALPHA;
-    const uint32_t t = c->nbr_threads[g];
+    const int fixed = c->fixed_mode() ? 1 : 0;
     if (c->carries())
-        return rec_shaped(c, R, g,
-                       c->nbr_persistent[g]
-                           ? pick(k_density_alpha_div_learn<128, true>,
-                                  k_density_alpha_div_learn<256, true>,
-                                  k_density_alpha_div_learn<256, true>, t)
-                           : pick(k_density_alpha_div_learn<128, false>,
-                                  k_density_alpha_div_learn<256, false>,
-                                  k_density_alpha_div_learn<256, false>, t),
-                       c->B, c->fixed_mode() ? 1 : 0, c->L);
-    return rec_shaped(c, R, g,
-                   c->nbr_persistent[g]
-                       ? pick(k_density_alpha_div<128, true>, k_density_alpha_div<256, true>,
-                              k_density_alpha_div<256, true>, t)
-                       : pick(k_density_alpha_div<128, false>, k_density_alpha_div<256, false>,
-                              k_density_alpha_div<256, false>, t),
-                   c->B, c->fixed_mode() ? 1 : 0);
+        REC(R.k(k_density_alpha_div_learn, quarter_grid(c), dim3(kFewThreads), c->B, fixed, c->L));
+    else
+        REC(R.k(k_density_alpha_div, quarter_grid(c), dim3(kFewThreads), c->B, fixed));
+    return FE_OK;
 }
 
 // Whether a shape may run group g.

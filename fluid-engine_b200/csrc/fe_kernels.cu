@@ -15,6 +15,8 @@
 // ~216 candidates; they visit the same pairs in the same order and therefore
 // produce identical sums.  A particle with more than kNbrCap neighbours keeps
 // walking the buckets in every pass.
+#include <cuda_fp16.h>
+
 #include "fe_common.cuh"
 #include "fe_features.cuh"
 #include "fe_kernels.h"
@@ -372,40 +374,60 @@ __global__ void __launch_bounds__(kBlock) k_refresh_pr(Bufs B) {
 // Phase 1 takes one of two forms, chosen per warp.  The lanes of a warp hold
 // consecutive particles of the sorted order, and a run of lanes whose
 // particles share a cell also shares that cell's 27 buckets.
-//  * Few runs (bulk fluid, several particles per cell): cell-cooperative.
-//    For each run the warp lays the 27 buckets end to end in walk order (z,
-//    y, x offsets, each bucket's entries in sorted order) and visits the
-//    candidates 32 at a time, one per lane: every lane tests its candidate
-//    against each particle of the run, and the ballot of the lanes that pass
-//    is that particle's in-range mask for the slab.  No lane idles on
-//    another's longer bucket, and a candidate's position is loaded once per
-//    run.  In phase 2 the set bits of a particle's masks, slab by slab and bit
-//    by bit, are its candidates in walk order; the run's table of non-empty
-//    buckets turns a bit back into a particle index.
+//  * Few runs (bulk fluid, several particles per cell): cell-cooperative.  A
+//    run's buckets laid end to end in walk order (z, y, x offsets, each
+//    bucket's entries in sorted order) are its row of candidates.  The warp
+//    takes all its runs' rows a slab of 32 candidates at a time: it stages the
+//    slab's positions (each loaded once per run) in shared memory, and every
+//    lane then tests its own particle against the 32 candidates of its run
+//    and keeps the mask.  The test is a superset of the exact one, in packed
+//    half precision relative to the run's first particle (see kNearHalf);
+//    phase 2 applies the exact test.  In phase 2 the set bits of a particle's
+//    masks, slab by slab and bit by bit, are its candidates in walk order; a
+//    bit mask of where buckets start in the slab turns a bit back into a
+//    particle index.
 //  * Many runs (spray, sparse cells): each lane walks its own 27 buckets and
-//    records its in-range candidates.
-// A particle with more than kStage in-range candidates, or a run with more
-// than kMaxSlabs * 32 candidates, redoes everything in a single-phase walk.
+//    records its in-range candidates, kStage of them at a time.
+// A run whose row is longer than kMaxSlabs * 32 does everything in a
+// single-phase walk.
 // ---------------------------------------------------------------------------
+// In-range candidates a lane can keep in the per-lane form; row length and runs
+// of the cooperative form: what fits 5.6 KB per warp, 32 warps an SM.  A
+// moving dam break has 5 to 8 runs in the mean warp and more than 10 in 5 to
+// 15 % of them; its rows are 70 to 320 candidates long.
 constexpr int kStage = 44;
-constexpr int kMaxSlabs = 16;
-constexpr int kCoopRuns = 8;   // most runs per warp for the cooperative form
+constexpr int kMaxSlabs = 12;
+constexpr int kCoopRuns = 10;
 
-struct RunTable {
-    uint32_t start[27];   // non-empty buckets in walk order: first entry
-    uint16_t excl[28];    // place of the bucket's first entry in the run's row; [K] = row length
-};
+// The near test in half precision, in units of h, relative to the first
+// particle of the run.  A particle of the run lies within 1 of it on each axis
+// and a candidate within 2, so rounding moves a coordinate difference by at
+// most 2^-12 + 2^-11 + 2^-11, the sum of squares by at most 4.3e-3 where it
+// is 1, and its three roundings add 1.5e-3: no pair with r <= h exceeds
+// 1.0058.  Coordinates beyond half's range become Inf (rejected, as such a
+// pair is far apart) or, Inf - Inf and NaN, pass on to the exact test.
+constexpr float kNearHalf = 1.0078125f;
+// h for which the scaled coordinates and h^2 stay far from FP32's limits.
+constexpr float kCoopMinH = 1e-15f, kCoopMaxH = 1e15f;
 
 // Per-warp scratch: one form or the other.
 union DensityScratch {
     struct {
-        alignas(8) float rx[32];        // the run being tested: its particles' positions
-        alignas(8) float ry[32];
-        alignas(8) float rz[32];
         uint32_t mask[kMaxSlabs][32];
-        RunTable table[kCoopRuns];
-        uint32_t row[kMaxSlabs * 32];   // the run being tested: its candidates' indices
-    } coop;
+        // the row of each run: where non-empty buckets start (bit c of word w:
+        // at candidate 32 w + c), how many start before a word, each bucket's
+        // first entry minus its place in the row, and the row's length (0: too
+        // long)
+        uint32_t starts[kCoopRuns][kMaxSlabs];
+        uint8_t before[kCoopRuns][kMaxSlabs];
+        uint32_t first[kCoopRuns][27];
+        uint32_t total[kCoopRuns];
+        alignas(16) float4 head[kCoopRuns];   // position of the run's first particle
+        // a slab of each run: x, y, z as 16 pairs (candidate k, candidate
+        // k + 16).  208 bytes apart, so that eight runs' 16-byte reads fall
+        // into different banks
+        alignas(16) __half near[kCoopRuns][104];
+    };
     uint32_t cand[kStage][32];
 };
 
@@ -466,124 +488,188 @@ __device__ __forceinline__ f3 neighbour_pos(const Bufs& B, uint32_t j, float4& v
     return xyz(q);
 }
 
-// Cooperative phase 1 over the runs of one warp (see above).  Returns, for
-// the calling lane, the table of its run (-1: single-phase walk) and its
-// number of in-range candidates.
-__device__ __forceinline__ void coop_candidates(const Bufs& B, const DevParams& P,
-                                                DensityScratch& S, uint32_t heads, int n_live,
-                                                int cx, int cy, int cz, float4 p4, int& my_table,
-                                                uint32_t& n_in) {
-    const int lane = lane_id();
-    const float h = P.h;
-    const float h2_wide = (h * h) * (1.0f + 0x1p-18f);
+// A row's candidate c in slab `sl` (c = 32 sl + bit) as a particle index.
+__device__ __forceinline__ uint32_t row_entry(const uint32_t* first, uint32_t starts,
+                                              uint32_t before, uint32_t sl, uint32_t bit) {
+    const uint32_t slot = before + __popc(starts & ((2u << bit) - 1u)) - 1u;
+    return first[slot] + (sl << 5) + bit;
+}
+
+// Cooperative phase 1 over the runs of one warp (see above), given by their
+// first lanes.  Returns the calling lane's run, or -1 if its row is too long,
+// and the number of candidates that passed the near test.  All 32 lanes.
+__device__ __forceinline__ int coop_candidates(const Bufs& B, const DevParams& P,
+                                               DensityScratch& S, uint32_t heads, bool live,
+                                               int cx, int cy, int cz, float4 p4,
+                                               uint32_t& n_in) {
+    constexpr int kGroup = 4;   // runs whose loads are in flight together
+    constexpr uint32_t kLong = 2047u;   // stands for any longer bucket: 27 fit 16 bits
+    const uint32_t lane = (uint32_t)lane_id();
     const uint32_t lt_mask = (1u << lane) - 1u;
-    int n_tables = 0;
-    while (heads) {
-        const int r0 = __ffs(heads) - 1;
-        heads &= heads - 1;
-        const int r1 = heads ? __ffs(heads) - 1 : n_live;
-        const int rx = __shfl_sync(kFull, cx, r0), ry = __shfl_sync(kFull, cy, r0),
-                  rz = __shfl_sync(kFull, cz, r0);
-        // lane t < 27: bucket t of the walk
-        uint32_t start = 0, len = 0;
-        if (lane < 27) {
-            const int x = lane % 3 - 1, y = (lane / 3) % 3 - 1, z = lane / 9 - 1;
-            const uint32_t k = P.table_base +
-                               cell_hash_pow2((int)((uint32_t)rx + (uint32_t)x),
-                                              (int)((uint32_t)ry + (uint32_t)y),
-                                              (int)((uint32_t)rz + (uint32_t)z), P.T - 1u);
-            const uint2 cell = B.cells[k];
-            if (cell.x != kEmpty) {
-                start = cell.x;
-                len = cell.y - cell.x;
+    const int runs = __popc(heads);
+    const int run = __popc(heads & (lt_mask | (1u << lane))) - 1;
+    for (uint32_t t = lane; t < kCoopRuns * kMaxSlabs; t += 32) (&S.starts[0][0])[t] = 0u;
+    if ((heads >> lane) & 1u) S.head[run] = p4;
+    __syncwarp();
+    uint32_t left = heads;
+#pragma unroll 1
+    for (int r0 = 0; r0 < runs; r0 += kGroup) {
+        uint32_t start[kGroup], len[kGroup];
+#pragma unroll
+        for (int q = 0; q < kGroup; ++q) {
+            start[q] = len[q] = 0;
+            if (r0 + q >= runs) continue;
+            const int h0 = __ffs(left) - 1;
+            left &= left - 1;
+            const int rx = __shfl_sync(kFull, cx, h0), ry = __shfl_sync(kFull, cy, h0),
+                      rz = __shfl_sync(kFull, cz, h0);
+            if (lane < 27u) {   // lane t: bucket t of the walk
+                const int t = (int)lane;
+                const int x = t % 3 - 1, y = (t / 3) % 3 - 1, z = t / 9 - 1;
+                const uint2 cell = B.cells[P.table_base +
+                                           cell_hash_pow2((int)((uint32_t)rx + (uint32_t)x),
+                                                          (int)((uint32_t)ry + (uint32_t)y),
+                                                          (int)((uint32_t)rz + (uint32_t)z),
+                                                          P.T - 1u)];
+                start[q] = cell.x;
+                len[q] = cell.x != kEmpty ? min(cell.y - cell.x, kLong) : 0u;
             }
         }
-        uint32_t incl = len;
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t v = __shfl_up_sync(kFull, incl, d);
-            if (lane >= d) incl += v;
-        }
-        const uint32_t excl = incl - len;
-        const uint32_t total = __shfl_sync(kFull, incl, 31);
-        const uint32_t nslab = (total + 31u) >> 5;
-        const bool mine = lane >= r0 && lane < r1;
-        if (nslab > (uint32_t)kMaxSlabs) continue;   // this run walks in phase 2
-        if (mine) my_table = n_tables;
-        RunTable& T = S.coop.table[n_tables++];
-        const uint32_t nonempty = __ballot_sync(kFull, len != 0);
-        if (len != 0) {
-            const int slot = __popc(nonempty & lt_mask);
-            T.start[slot] = start;
-            T.excl[slot] = (uint16_t)excl;
-        }
-        if (lane == 0) T.excl[__popc(nonempty)] = (uint16_t)total;
-        // the run's row: candidate c of the walk is particle row[c] (each
-        // bucket's lane writes its entries)
-        for (uint32_t u = 0; u < len; ++u) S.coop.row[excl + u] = start + u;
-        if (mine) {
-            S.coop.rx[lane - r0] = p4.x;
-            S.coop.ry[lane - r0] = p4.y;
-            S.coop.rz[lane - r0] = p4.z;
-        }
-        __syncwarp();
-        for (uint32_t sl = 0; sl < nslab; ++sl) {
-            const uint32_t cidx = (sl << 5) + (uint32_t)lane;
-            const bool valid = cidx < total;
-            const float4 q =
-                valid ? __ldg(posb(B, S.coop.row[cidx])) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            // particle p's mask for this slab is the ballot; lane 0 stores it.
-            // The test is a superset of the exact r^2 <= h^2 (contracted r^2
-            // against h^2 (1 + 2^-18)); phase 2 applies the exact test.
-            // two particles of the run per step in packed FP32 (the test
-            // above; the contraction that packing allows is covered by the
-            // widened bound), their coordinates read as pairs from the run's
-            // position arrays
-            uint64_t qx2, qy2, qz2;
-            asm("mov.b64 %0, {%1, %1};" : "=l"(qx2) : "f"(q.x));
-            asm("mov.b64 %0, {%1, %1};" : "=l"(qy2) : "f"(q.y));
-            asm("mov.b64 %0, {%1, %1};" : "=l"(qz2) : "f"(q.z));
-            const int cnt = r1 - r0;
-            int p = 0;
-#pragma unroll 1
-            for (; p + 1 < cnt; p += 2) {
-                const uint64_t ax = *reinterpret_cast<const uint64_t*>(&S.coop.rx[p]);
-                const uint64_t ay = *reinterpret_cast<const uint64_t*>(&S.coop.ry[p]);
-                const uint64_t az = *reinterpret_cast<const uint64_t*>(&S.coop.rz[p]);
-                uint64_t dx, dy, dz, r2;
-                asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(dx) : "l"(ax), "l"(qx2));
-                asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(dy) : "l"(ay), "l"(qy2));
-                asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(dz) : "l"(az), "l"(qz2));
-                asm("mul.rn.f32x2 %0, %1, %1;" : "=l"(r2) : "l"(dz));
-                asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(r2) : "l"(dy), "l"(r2));
-                asm("fma.rn.f32x2 %0, %1, %1, %2;" : "=l"(r2) : "l"(dx), "l"(r2));
-                float r2a, r2b;
-                asm("mov.b64 {%0, %1}, %2;" : "=f"(r2a), "=f"(r2b) : "l"(r2));
-                const uint32_t b0 = __ballot_sync(kFull, valid && !(r2a > h2_wide));
-                const uint32_t b1 = __ballot_sync(kFull, valid && !(r2b > h2_wide));
+        for (int q = 0; q < kGroup; q += 2) {
+            if (r0 + q >= runs) continue;
+            uint32_t both = len[q] | len[q + 1] << 16;   // two runs' sums in one
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t v = __shfl_up_sync(kFull, both, d);
+                if (lane >= (uint32_t)d) both += v;
+            }
+            const uint32_t totals = __shfl_sync(kFull, both, 31);
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+                const int r = r0 + q + w;
+                if (r >= runs) continue;
+                const uint32_t l = len[q + w];
+                const uint32_t total = w ? totals >> 16 : totals & 0xFFFFu;
+                const uint32_t nonempty = __ballot_sync(kFull, l != 0);
+                const bool fits = total <= (uint32_t)kMaxSlabs * 32u;
+                if (l != 0 && fits) {
+                    const uint32_t incl = w ? both >> 16 : both & 0xFFFFu, excl = incl - l;
+                    const uint32_t slot = __popc(nonempty & lt_mask);
+                    S.first[r][slot] = start[q + w] - excl;
+                    atomicOr(&S.starts[r][excl >> 5], 1u << (excl & 31u));
+                    // words that begin after this bucket's first entry and not
+                    // after its last have slot + 1 starts before them
+                    for (uint32_t k = (excl >> 5) + 1; k <= incl >> 5 && k < kMaxSlabs; ++k)
+                        S.before[r][k] = (uint8_t)(slot + 1);
+                }
                 if (lane == 0) {
-                    S.coop.mask[sl][r0 + p] = b0;
-                    S.coop.mask[sl][r0 + p + 1] = b1;
+                    S.total[r] = fits ? total : 0u;   // (a row is never empty)
+                    S.before[r][0] = 0;
                 }
             }
-            if (p < cnt) {
-                const float dx = S.coop.rx[p] - q.x, dy = S.coop.ry[p] - q.y,
-                            dz = S.coop.rz[p] - q.z;
-                const float r2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
-                const uint32_t bits = __ballot_sync(kFull, valid && !(r2 > h2_wide));
-                if (lane == 0) S.coop.mask[sl][r0 + p] = bits;
-            }
-            __syncwarp();
-            if (mine) n_in += __popc(S.coop.mask[sl][lane]);
         }
     }
+    __syncwarp();
+    const uint32_t my_total = live ? S.total[run] : 0u;
+    const int my_run = my_total ? run : -1;
+    const uint32_t my_slabs = (my_total + 31u) >> 5;
+    const uint32_t slabs = __reduce_max_sync(kFull, my_slabs);
+    const float inv_h = P.inv_h;
+    const float4 o = live ? S.head[run] : p4;
+    const __half2 ax = __float2half2_rn((p4.x - o.x) * inv_h),
+                  ay = __float2half2_rn((p4.y - o.y) * inv_h),
+                  az = __float2half2_rn((p4.z - o.z) * inv_h);
+    const __half2 bound = __float2half2_rn(kNearHalf);
+    const uint32_t at = 2u * (lane & 15u) + (lane >> 4);   // my candidate's place in `near`
+#pragma unroll 1
+    for (uint32_t sl = 0; sl < slabs; ++sl) {
+        const uint32_t c = (sl << 5) + lane;
+        {
+#pragma unroll 1
+            for (int r0 = 0; r0 < runs; r0 += kGroup) {
+                float4 q[kGroup];
+#pragma unroll
+                for (int k = 0; k < kGroup; ++k) {
+                    const int r = r0 + k;
+                    q[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    // (a lane past the row's end stages anything: its bit is masked)
+                    if (r < runs && c < S.total[r])
+                        q[k] = __ldg(posb(B, row_entry(S.first[r], S.starts[r][sl],
+                                                       S.before[r][sl], sl, lane)));
+                }
+#pragma unroll
+                for (int k = 0; k < kGroup; ++k) {
+                    if (r0 + k >= runs) continue;
+                    __half* near = S.near[r0 + k];
+                    const float4 o = S.head[r0 + k];
+                    near[at] = __float2half_rn((q[k].x - o.x) * inv_h);
+                    near[32 + at] = __float2half_rn((q[k].y - o.y) * inv_h);
+                    near[64 + at] = __float2half_rn((q[k].z - o.z) * inv_h);
+                }
+            }
+            __syncwarp();
+            if (sl < my_slabs) {
+                const uint4* near = reinterpret_cast<const uint4*>(S.near[run]);
+                uint32_t far = 0;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    const uint4 x4 = near[g], y4 = near[4 + g], z4 = near[8 + g];
+                    const uint32_t xs[4] = {x4.x, x4.y, x4.z, x4.w},
+                                   ys[4] = {y4.x, y4.y, y4.z, y4.w},
+                                   zs[4] = {z4.x, z4.y, z4.z, z4.w};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const __half2 dx = __hsub2(ax, *reinterpret_cast<const __half2*>(&xs[k]));
+                        const __half2 dy = __hsub2(ay, *reinterpret_cast<const __half2*>(&ys[k]));
+                        const __half2 dz = __hsub2(az, *reinterpret_cast<const __half2*>(&zs[k]));
+                        const __half2 r2 = __hfma2(dx, dx, __hfma2(dy, dy, __hmul2(dz, dz)));
+                        far |= __hgt2_mask(r2, bound) & (0x00010001u << (4 * g + k));
+                    }
+                }
+                const uint32_t rest = my_total - (sl << 5);
+                const uint32_t bits = ~far & (rest < 32u ? (1u << rest) - 1u : kFull);
+                S.mask[sl][lane] = bits;
+                n_in += __popc(bits);
+            }
+            __syncwarp();
+        }
+    }
+    return my_run;
 }
+
+// The candidates of a lane that passed the near test, in walk order.
+struct RowWalk {
+    uint32_t sl = 0, bits = 0, starts = 0, before = 0;
+    __device__ __forceinline__ RowWalk(const DensityScratch& S, int run, int lane) {
+        bits = S.mask[0][lane];
+        starts = S.starts[run][0];
+    }
+    // the next one (there is one)
+    __device__ __forceinline__ uint32_t next(const DensityScratch& S, int run, int lane) {
+        while (bits == 0) {
+            bits = S.mask[++sl][lane];
+            starts = S.starts[run][sl];
+            before = S.before[run][sl];
+        }
+        const uint32_t bit = __ffs(bits) - 1;
+        bits &= bits - 1;
+        return row_entry(S.first[run], starts, before, sl, bit);
+    }
+};
 
 // Blocks per SM the launch bounds ask for: 1024 resident threads per SM
 // (at most 64 registers per thread), for every block size.
 // (the shape for few particles takes the registers for its loads in flight)
 template <int kThreads>
 constexpr int kMinBlocks = kThreads == kFewThreads ? 5 : 1024 / kThreads;
+
+// Two warps a block, whatever the tuned shape: warps differ by a factor of two
+// and more in their runs and candidates, and a block keeps its shared memory
+// until its last warp is done.  On 1M particles 40 frames into a fall, 256
+// threads take 0.50 ms, 64 threads 0.46.
+constexpr int kDensityThreads = kFewThreads;
+constexpr int kDensityBlocks = 16;   // 64 registers a thread
 
 // kDiv: 0 density and alpha only; 1 also the FIXED-mode divergence source
 // (velocity_b), 2 also the REFERENCE-mode one (velocity_a) -- see
@@ -608,12 +694,11 @@ __device__ __forceinline__ void density_alpha_particle(const Bufs& B, DensityScr
               pz = __shfl_up_sync(kFull, cz, 1);
     const bool head = live && (lane == 0 || cx != px || cy != py || cz != pz);
     const uint32_t heads = __ballot_sync(kFull, head);
-    const int n_live = 32 - __clz(__ballot_sync(kFull, live));
-    const bool coop = __popc(heads) <= kCoopRuns;
-    int my_table = -1;
+    const bool coop = __popc(heads) <= kCoopRuns && h > kCoopMinH && h < kCoopMaxH;
+    int my_run = -1;
     uint32_t n1 = 0;
     if (coop) {
-        coop_candidates(B, P, S, heads, n_live, cx, cy, cz, p4, my_table, n1);
+        my_run = coop_candidates(B, P, S, heads, live, cx, cy, cz, p4, n1);
     } else if (live) {
         walk(B, P, pi, [&](uint32_t j, f3, float) {
             if (n1 < (uint32_t)kStage) S.cand[n1][lane] = j;
@@ -623,37 +708,52 @@ __device__ __forceinline__ void density_alpha_particle(const Bufs& B, DensityScr
     __syncwarp();
     if (!live) return;
 
-    uint2* out = B.nbr + i;
     const uint32_t stride = B.n_total;
     DensityAcc a;
-    a.op = out;
+    a.op = B.nbr + i;
     const f3 vi = kDiv ? xyz(__ldg(kDiv == 1 ? velb(B, i) : vela(B, i))) : f3{0.0f, 0.0f, 0.0f};
     float4 vj = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (coop && my_table >= 0) {
-        const RunTable& T = S.coop.table[my_table];
-        uint32_t sl = 0, bits = S.coop.mask[0][lane];
-        uint32_t t = 0, cur_start = T.start[0], cur_excl = 0, next_excl = T.excl[1];
-        for (uint32_t k = 0; k < n1; ++k) {
-            while (bits == 0) bits = S.coop.mask[++sl][lane];
-            const uint32_t cidx = (sl << 5) + (uint32_t)(__ffs(bits) - 1);
-            bits &= bits - 1;
-            while (cidx >= next_excl) {
-                ++t;
-                cur_start = T.start[t];
-                cur_excl = next_excl;
-                next_excl = T.excl[t + 1];
+    // n candidates in order, the next one's position on its way while this one's
+    // terms are computed
+    auto sums = [&](uint32_t n, auto&& next) {
+        if (n == 0) return;
+        uint32_t j = next();
+        f3 pj = neighbour_pos<kDiv>(B, j, vj);
+        for (uint32_t k = 1; k <= n; ++k) {
+            const uint32_t j0 = j;
+            const f3 p0 = pj;
+            const float4 v0 = vj;
+            if (k < n) {
+                j = next();
+                pj = neighbour_pos<kDiv>(B, j, vj);
             }
-            const uint32_t j = cur_start + (cidx - cur_excl);
-            f3 rv = sub(pi, neighbour_pos<kDiv>(B, j, vj));
+            const f3 rv = sub(pi, p0);
             const float r2 = dot(rv, rv);
-            if (r2 > h * h) continue;   // the shader's test (phase 1 passed a superset)
-            density_term<kDiv>(a, m, P, kn, j, rv, r2, stride, vi, vj);
+            if (r2 > h * h) continue;   // the shader's test (phase 1 may pass a superset)
+            density_term<kDiv>(a, m, P, kn, j0, rv, r2, stride, vi, v0);
         }
+    };
+    if (my_run >= 0) {
+        RowWalk w(S, my_run, lane);
+        sums(n1, [&] { return w.next(S, my_run, lane); });
     } else if (!coop && n1 <= (uint32_t)kStage) {
-        for (uint32_t k = 0; k < n1; ++k) {
-            uint32_t j = S.cand[k][lane];
-            f3 rv = sub(pi, neighbour_pos<kDiv>(B, j, vj));
-            density_term<kDiv>(a, m, P, kn, j, rv, dot(rv, rv), stride, vi, vj);
+        uint32_t k = 0;
+        sums(n1, [&] { return S.cand[k++][lane]; });
+    } else if (!coop) {
+        // more candidates than the scratch holds: kStage of them at a time
+        for (uint32_t from = 0; from < n1; from += kStage) {
+            uint32_t seen = 0;
+            walk(B, P, pi, [&](uint32_t j, f3, float) {
+                const uint32_t at = seen++ - from;
+                if (at < (uint32_t)kStage) S.cand[at][lane] = j;
+            });
+            const uint32_t n = min(n1 - from, (uint32_t)kStage);
+#pragma unroll 1
+            for (uint32_t k = 0; k < n; ++k) {
+                const uint32_t j = S.cand[k][lane];
+                const f3 rv = sub(pi, neighbour_pos<kDiv>(B, j, vj));
+                density_term<kDiv>(a, m, P, kn, j, rv, dot(rv, rv), stride, vi, vj);
+            }
         }
     } else {
         walk(B, P, pi, [&](uint32_t j, f3 rv, float r2) {
@@ -691,11 +791,10 @@ __device__ __forceinline__ void density_alpha_particle(const Bufs& B, DensityScr
     }
 }
 
-template <int kThreads, bool kPersist>
-__global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>) k_density_alpha(Bufs B) {
-    __shared__ DensityScratch scratch[kThreads / 32];
+__global__ void __launch_bounds__(kDensityThreads, kDensityBlocks) k_density_alpha(Bufs B) {
+    __shared__ DensityScratch scratch[kDensityThreads / 32];
     DensityScratch& S = scratch[threadIdx.x >> 5];
-    for_each_particle<kThreads, kPersist>(B, [&](uint32_t i, uint32_t s, bool live) {
+    for_each_particle<kDensityThreads, false>(B, [&](uint32_t i, uint32_t s, bool live) {
         density_alpha_particle<0, false>(B, S, i, s, live, LearnArgs{});
     });
 }
@@ -707,17 +806,16 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>) k_density_alph
 // else REFERENCE mode (velocity_a).  It runs right after the substep's
 // re-sort and takes over that search's last copy: FIXED mode's gathered
 // pressures (prs_tmp) become current here.
-template <int kThreads, bool kPersist>
-__global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>)
+__global__ void __launch_bounds__(kDensityThreads, kDensityBlocks)
     k_density_alpha_div(Bufs B, int fixed) {
-    __shared__ DensityScratch scratch[kThreads / 32];
+    __shared__ DensityScratch scratch[kDensityThreads / 32];
     DensityScratch& S = scratch[threadIdx.x >> 5];
     if (fixed) {
-        for_each_particle<kThreads, kPersist>(B, [&](uint32_t i, uint32_t s, bool live) {
+        for_each_particle<kDensityThreads, false>(B, [&](uint32_t i, uint32_t s, bool live) {
             density_alpha_particle<1, false>(B, S, i, s, live, LearnArgs{});
         });
     } else {
-        for_each_particle<kThreads, kPersist>(B, [&](uint32_t i, uint32_t s, bool live) {
+        for_each_particle<kDensityThreads, false>(B, [&](uint32_t i, uint32_t s, bool live) {
             density_alpha_particle<2, false>(B, S, i, s, live, LearnArgs{});
         });
     }
@@ -725,17 +823,16 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>)
 
 // The same with the learned state: also the divergence solve's features,
 // and the gathered carry (carry_tmp) becomes current here in both modes.
-template <int kThreads, bool kPersist>
-__global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>)
+__global__ void __launch_bounds__(kDensityThreads, kDensityBlocks)
     k_density_alpha_div_learn(Bufs B, int fixed, LearnArgs L) {
-    __shared__ DensityScratch scratch[kThreads / 32];
+    __shared__ DensityScratch scratch[kDensityThreads / 32];
     DensityScratch& S = scratch[threadIdx.x >> 5];
     if (fixed) {
-        for_each_particle<kThreads, kPersist>(B, [&](uint32_t i, uint32_t s, bool live) {
+        for_each_particle<kDensityThreads, false>(B, [&](uint32_t i, uint32_t s, bool live) {
             density_alpha_particle<1, true>(B, S, i, s, live, L);
         });
     } else {
-        for_each_particle<kThreads, kPersist>(B, [&](uint32_t i, uint32_t s, bool live) {
+        for_each_particle<kDensityThreads, false>(B, [&](uint32_t i, uint32_t s, bool live) {
             density_alpha_particle<2, true>(B, S, i, s, live, L);
         });
     }
@@ -747,7 +844,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>)
 template <int kThreads>
 __device__ __forceinline__ void viscosity_particle(const Bufs& B, uint32_t i, uint32_t s) {
     const DevParams& P = B.P[s];
-    const float m = P.mass, h = P.h;
+    const float h = P.h;
     const float kn = kernel_norm(h), inv_h = P.inv_h;
     const uint32_t exact = P.h_recip_exact;
     const f3 pi = xyz(__ldg(posb(B, i)));
@@ -1502,17 +1599,5 @@ FE_NBR_INSTANTIATE(256, true)
 FE_NBR_INSTANTIATE(512, true)
 template __global__ void k_pressure_update<kBlock>(Bufs, int, cudaGraphConditionalHandle, int);
 template __global__ void k_pressure_update<kFewThreads>(Bufs, int, cudaGraphConditionalHandle, int);
-template __global__ void k_density_alpha<128, false>(Bufs);
-template __global__ void k_density_alpha<256, false>(Bufs);
-template __global__ void k_density_alpha<128, true>(Bufs);
-template __global__ void k_density_alpha<256, true>(Bufs);
-template __global__ void k_density_alpha_div<128, false>(Bufs, int);
-template __global__ void k_density_alpha_div<256, false>(Bufs, int);
-template __global__ void k_density_alpha_div<128, true>(Bufs, int);
-template __global__ void k_density_alpha_div<256, true>(Bufs, int);
-template __global__ void k_density_alpha_div_learn<128, false>(Bufs, int, LearnArgs);
-template __global__ void k_density_alpha_div_learn<256, false>(Bufs, int, LearnArgs);
-template __global__ void k_density_alpha_div_learn<128, true>(Bufs, int, LearnArgs);
-template __global__ void k_density_alpha_div_learn<256, true>(Bufs, int, LearnArgs);
 
 }  // namespace fe

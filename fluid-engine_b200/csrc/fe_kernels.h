@@ -27,11 +27,8 @@ __global__ void k_cell_reorder_carry(Bufs B, CellSort C, int carry_pressure, Lea
 __global__ void k_take_pressure(Bufs B);
 __global__ void k_take_pressure_carry(Bufs B, LearnArgs L);
 __global__ void k_refresh_pr(Bufs B);
-template <int kThreads, bool kPersist>
 __global__ void k_density_alpha(Bufs B);
-template <int kThreads, bool kPersist>
 __global__ void k_density_alpha_div(Bufs B, int fixed);
-template <int kThreads, bool kPersist>
 __global__ void k_density_alpha_div_learn(Bufs B, int fixed, LearnArgs L);
 template <int kThreads, bool kPersist>
 __global__ void k_viscosity(Bufs B);

@@ -96,7 +96,7 @@ __device__ __forceinline__ void walk(const Bufs& B, const DevParams& P, f3 pi, F
                              cell_hash_pow2((int)((uint32_t)cx + (uint32_t)x),
                                             (int)((uint32_t)cy + (uint32_t)y),
                                             (int)((uint32_t)cz + (uint32_t)z), P.T - 1u);
-                uint2 cell = B.cells[k];
+                const uint2 cell = __ldg(B.cells + k);
                 if (cell.x == kEmpty) continue;
                 for (uint32_t j = cell.x; j < cell.y; ++j) {
                     f3 rv = sub(pi, xyz(__ldg(posb(B, j))));
