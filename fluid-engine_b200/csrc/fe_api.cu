@@ -545,23 +545,40 @@ fe_status rec_nbr(fe_ctx* c, Recorder& R, int g, void (*func)(KArgs...), Args...
     return rec_shaped(c, R, g, func, args...);
 }
 
-// (its one shape: the shapes fe_set_tuning takes for this group are accepted
-// and make no difference)
-fe_status rec_density_alpha(fe_ctx* c, Recorder& R) {
-    REC(R.k(k_density_alpha, quarter_grid(c), dim3(kFewThreads), c->B));
+// density_alpha: blocks of 64 threads (the shapes fe_set_tuning takes for this
+// group are accepted and make no difference).  Particles per warp: 8 while all
+// those warps are resident at once (32 an SM), 16 up to half as many particles
+// again, else 32.  Times in a graph of launches (us, 8 / 16 / 32 per warp, a
+// fall after 40 frames): 4.8k particles 28/43/58, 25k 43/60/65, 50k 72/63/68,
+// 80k 99/78/70, 131k 152/112/80.
+#ifndef FE_LANES8
+#define FE_LANES8 (148 * 32 * 8)
+#define FE_LANES16 (148 * 32 * 12)
+#endif
+template <class... KArgs, class... Args>
+fe_status rec_density(fe_ctx* c, Recorder& R, void (*k8)(KArgs...), void (*k16)(KArgs...),
+                      void (*k32)(KArgs...), Args... args) {
+    const uint32_t lanes = c->n <= FE_LANES8 ? 8u : c->n <= FE_LANES16 ? 16u : 32u;
+    const uint32_t blocks = c->B.n_chunks * (kBlock / lanes) / (kFewThreads / 32);
+    REC(R.k(lanes == 8 ? k8 : lanes == 16 ? k16 : k32, dim3(blocks), dim3(kFewThreads), args...));
     return FE_OK;
+}
+#define DENSITY_DIV(name, div) name<8, div>, name<16, div>, name<32, div>
+
+fe_status rec_density_alpha(fe_ctx* c, Recorder& R) {
+    return rec_density(c, R, k_density_alpha<8>, k_density_alpha<16>, k_density_alpha<32>, c->B);
 }
 
 // density_alpha that also sums the divergence source (the mid-substep
 // neighbour search's pass); with the learned state it also emits the
 // divergence solve's features.
 fe_status rec_density_alpha_div(fe_ctx* c, Recorder& R) {
-    const int fixed = c->fixed_mode() ? 1 : 0;
     if (c->carries())
-        REC(R.k(k_density_alpha_div_learn, quarter_grid(c), dim3(kFewThreads), c->B, fixed, c->L));
-    else
-        REC(R.k(k_density_alpha_div, quarter_grid(c), dim3(kFewThreads), c->B, fixed));
-    return FE_OK;
+        return c->fixed_mode()
+                   ? rec_density(c, R, DENSITY_DIV(k_density_alpha_div_learn, 1), c->B, c->L)
+                   : rec_density(c, R, DENSITY_DIV(k_density_alpha_div_learn, 2), c->B, c->L);
+    return c->fixed_mode() ? rec_density(c, R, DENSITY_DIV(k_density_alpha_div, 1), c->B)
+                           : rec_density(c, R, DENSITY_DIV(k_density_alpha_div, 2), c->B);
 }
 
 // Whether a shape may run group g.

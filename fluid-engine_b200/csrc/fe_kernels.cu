@@ -791,10 +791,30 @@ __device__ __forceinline__ void density_alpha_particle(const Bufs& B, DensityScr
     }
 }
 
+// kLanes: particles per warp, in its first lanes.  A warp's time is a chain of
+// some 8000 instructions and their latencies whatever its number of
+// particles, so with few particles 8 or 16 of them per warp make more, and
+// shorter, chains (fewer cells each) where the SMs would otherwise idle.
+template <int kLanes, class F>
+__device__ __forceinline__ void density_particle(const Bufs& B, F&& f) {
+    constexpr uint32_t per = kBlock / kLanes;   // warps per chunk
+    const uint32_t unit = blockIdx.x * (kDensityThreads / 32) + (threadIdx.x >> 5);
+    const uint32_t lane = threadIdx.x & 31u;
+    if (B.n_scenes == 1) {   // chunk c starts at 256 c: no table read
+        const uint32_t i = unit * kLanes + lane;
+        f(i, 0u, lane < kLanes && i < B.n_total);
+    } else {
+        const uint4 cc = B.chunks[unit / per];
+        const uint32_t off = (unit % per) * kLanes + lane;
+        f(cc.x + off, cc.z, lane < kLanes && off < cc.y);
+    }
+}
+
+template <int kLanes>
 __global__ void __launch_bounds__(kDensityThreads, kDensityBlocks) k_density_alpha(Bufs B) {
     __shared__ DensityScratch scratch[kDensityThreads / 32];
     DensityScratch& S = scratch[threadIdx.x >> 5];
-    for_each_particle<kDensityThreads, false>(B, [&](uint32_t i, uint32_t s, bool live) {
+    density_particle<kLanes>(B, [&](uint32_t i, uint32_t s, bool live) {
         density_alpha_particle<0, false>(B, S, i, s, live, LearnArgs{});
     });
 }
@@ -802,40 +822,30 @@ __global__ void __launch_bounds__(kDensityThreads, kDensityBlocks) k_density_alp
 // density_alpha with the (plain) divergence source of the same substep
 // summed in its pair loop: the divergence source needs exactly these pairs,
 // gradients and order, and the neighbour's velocity shares a 32-byte record
-// with the position copy the loop loads.  fixed: FIXED mode (velocity_b),
-// else REFERENCE mode (velocity_a).  It runs right after the substep's
+// with the position copy the loop loads.  kDiv: 1 FIXED mode (velocity_b),
+// 2 REFERENCE mode (velocity_a); a kernel each, since with both in one the
+// compiler no longer inlines them (2079 -> 2437 us a 1M frame).  It runs right after the substep's
 // re-sort and takes over that search's last copy: FIXED mode's gathered
 // pressures (prs_tmp) become current here.
-__global__ void __launch_bounds__(kDensityThreads, kDensityBlocks)
-    k_density_alpha_div(Bufs B, int fixed) {
+template <int kLanes, int kDiv>
+__global__ void __launch_bounds__(kDensityThreads, kDensityBlocks) k_density_alpha_div(Bufs B) {
     __shared__ DensityScratch scratch[kDensityThreads / 32];
     DensityScratch& S = scratch[threadIdx.x >> 5];
-    if (fixed) {
-        for_each_particle<kDensityThreads, false>(B, [&](uint32_t i, uint32_t s, bool live) {
-            density_alpha_particle<1, false>(B, S, i, s, live, LearnArgs{});
-        });
-    } else {
-        for_each_particle<kDensityThreads, false>(B, [&](uint32_t i, uint32_t s, bool live) {
-            density_alpha_particle<2, false>(B, S, i, s, live, LearnArgs{});
-        });
-    }
+    density_particle<kLanes>(B, [&](uint32_t i, uint32_t s, bool live) {
+        density_alpha_particle<kDiv, false>(B, S, i, s, live, LearnArgs{});
+    });
 }
 
 // The same with the learned state: also the divergence solve's features,
 // and the gathered carry (carry_tmp) becomes current here in both modes.
+template <int kLanes, int kDiv>
 __global__ void __launch_bounds__(kDensityThreads, kDensityBlocks)
-    k_density_alpha_div_learn(Bufs B, int fixed, LearnArgs L) {
+    k_density_alpha_div_learn(Bufs B, LearnArgs L) {
     __shared__ DensityScratch scratch[kDensityThreads / 32];
     DensityScratch& S = scratch[threadIdx.x >> 5];
-    if (fixed) {
-        for_each_particle<kDensityThreads, false>(B, [&](uint32_t i, uint32_t s, bool live) {
-            density_alpha_particle<1, true>(B, S, i, s, live, L);
-        });
-    } else {
-        for_each_particle<kDensityThreads, false>(B, [&](uint32_t i, uint32_t s, bool live) {
-            density_alpha_particle<2, true>(B, S, i, s, live, L);
-        });
-    }
+    density_particle<kLanes>(B, [&](uint32_t i, uint32_t s, bool live) {
+        density_alpha_particle<kDiv, true>(B, S, i, s, live, L);
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -1582,8 +1592,6 @@ __global__ void k_count_substep(Bufs B) {
 }
 
 // The block sizes the autotuner chooses from.
-// (density_alpha: 128 and 256 only; its per-warp scratch would exceed the
-// 48 KB of static shared memory of a block at 512 threads)
 #define FE_NBR_INSTANTIATE(T, P)                                                      \
     template __global__ void k_viscosity<T, P>(Bufs);                                 \
     template __global__ void k_density_source<T, P>(Bufs);                            \
@@ -1597,6 +1605,15 @@ FE_NBR_INSTANTIATE(512, false)
 FE_NBR_INSTANTIATE(128, true)
 FE_NBR_INSTANTIATE(256, true)
 FE_NBR_INSTANTIATE(512, true)
+#define FE_DENSITY_INSTANTIATE(L)                                              \
+    template __global__ void k_density_alpha<L>(Bufs);                         \
+    template __global__ void k_density_alpha_div<L, 1>(Bufs);                  \
+    template __global__ void k_density_alpha_div<L, 2>(Bufs);                  \
+    template __global__ void k_density_alpha_div_learn<L, 1>(Bufs, LearnArgs); \
+    template __global__ void k_density_alpha_div_learn<L, 2>(Bufs, LearnArgs);
+FE_DENSITY_INSTANTIATE(8)
+FE_DENSITY_INSTANTIATE(16)
+FE_DENSITY_INSTANTIATE(32)
 template __global__ void k_pressure_update<kBlock>(Bufs, int, cudaGraphConditionalHandle, int);
 template __global__ void k_pressure_update<kFewThreads>(Bufs, int, cudaGraphConditionalHandle, int);
 

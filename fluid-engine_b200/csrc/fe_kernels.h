@@ -27,9 +27,12 @@ __global__ void k_cell_reorder_carry(Bufs B, CellSort C, int carry_pressure, Lea
 __global__ void k_take_pressure(Bufs B);
 __global__ void k_take_pressure_carry(Bufs B, LearnArgs L);
 __global__ void k_refresh_pr(Bufs B);
+template <int kLanes>
 __global__ void k_density_alpha(Bufs B);
-__global__ void k_density_alpha_div(Bufs B, int fixed);
-__global__ void k_density_alpha_div_learn(Bufs B, int fixed, LearnArgs L);
+template <int kLanes, int kDiv>
+__global__ void k_density_alpha_div(Bufs B);
+template <int kLanes, int kDiv>
+__global__ void k_density_alpha_div_learn(Bufs B, LearnArgs L);
 template <int kThreads, bool kPersist>
 __global__ void k_viscosity(Bufs B);
 // Per-scene finishes of a multi-scene context, one block per scene.

@@ -86,3 +86,18 @@ def test_half_precision_near_test_is_a_superset():
     s = (f[:, 1] ** 2 + s).astype(np.float16).astype(np.float64)
     s = (f[:, 0] ** 2 + s).astype(np.float16).astype(np.float64)
     assert s.max() <= 1.0058
+
+
+@pytest.mark.parametrize("n", [7, 8, 9, 37888, 37889, 56832, 56833])
+def test_particles_per_warp(oracle_mod, n):
+    """Both sides of 8, 16 and 32 particles per warp, and ragged last warps."""
+    p = scene.dam_break_params((0, 0, 0), (4.0, 4.0, 4.0), mode=_abi.FE_MODE_FIXED)
+    pos, _ = scene.lattice((0, 0, 0), (39, 39, 39), 0.025, 1000.0, 0.05, 0.04, 5)
+    pos = pos[:n]
+    sim, orc = Simulation(pos, p), oracle_mod.Oracle(p, pos)
+    sim.step(1)
+    orc.step(1)
+    for f in FIELDS:
+        a, b = sim.data.download(f).view(np.uint32), orc.field(f).view(np.uint32)
+        assert np.array_equal(a, b), f
+    sim.close()
