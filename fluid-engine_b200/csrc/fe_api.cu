@@ -351,12 +351,12 @@ struct fe_ctx {
     unsigned char* trace = nullptr;
     uint32_t trace_slots = 0, trace_cap = 0;
 
-    // density splat: headless grid and the non-zero taps of the splat kernel
+    // density splat: headless grid and the splat kernel's weights
     uint32_t* splat_grid = nullptr;
     size_t splat_cap = 0;          // voxels allocated
     int splat_res[3] = {0, 0, 0};  // resolution of the last splat
-    int4* splat_taps = nullptr;
-    uint32_t splat_ntaps = 0;
+    SplatWeights splat_weights{};
+    bool splat_ready = false;
     uint32_t* splat_hist = nullptr;    // particles per centre voxel
     size_t splat_hist_cap = 0;
 
@@ -1601,9 +1601,9 @@ fe_status fe_density_splat(fe_ctx* c) {
         c->splat_grid = g;
         c->splat_cap = voxels;
     }
-    if (!c->splat_taps) {
+    if (!c->splat_ready) {
         // The splat's weights per voxel offset, evaluated once on the device;
-        // the non-zero ones become the tap table (x fastest).
+        // they depend on the squared distance alone.
         constexpr int kAll = kSplatSide * kSplatSide * kSplatSide;
         uint32_t* w = nullptr;
         fe_status s = dev_alloc(c, &w, kAll);
@@ -1612,22 +1612,25 @@ fe_status fe_density_splat(fe_ctx* c) {
         std::vector<uint32_t> hw(kAll);
         FE_CUDA(cudaMemcpyAsync(hw.data(), w, kAll * 4, cudaMemcpyDeviceToHost, c->stream));
         FE_CUDA(cudaStreamSynchronize(c->stream));
-        std::vector<int4> taps;
-        for (int t = 0; t < kAll; ++t)
-            if (hw[t])
-                taps.push_back(make_int4(t % kSplatSide - kSplatRadius,
-                                         (t / kSplatSide) % kSplatSide - kSplatRadius,
-                                         t / (kSplatSide * kSplatSide) - kSplatRadius, (int)hw[t]));
-        int4* d = nullptr;
-        if ((s = dev_alloc(c, &d, taps.size()))) return s;
-        FE_CUDA(cudaMemcpy(d, taps.data(), taps.size() * sizeof(int4), cudaMemcpyHostToDevice));
-        c->splat_taps = d;
-        c->splat_ntaps = (uint32_t)taps.size();
+        std::memset(&c->splat_weights, 0, sizeof c->splat_weights);
+        for (int pass = 0; pass < 2; ++pass)
+            for (int t = 0; t < kAll; ++t) {
+                const int x = t % kSplatSide - kSplatRadius,
+                          y = (t / kSplatSide) % kSplatSide - kSplatRadius,
+                          z = t / (kSplatSide * kSplatSide) - kSplatRadius;
+                const int d2 = x * x + y * y + z * z;
+                if (pass == 0 && d2 <= kSplatMaxD2) c->splat_weights.w[d2] = hw[t];
+                if (pass == 1 && hw[t] != (d2 <= kSplatMaxD2 ? c->splat_weights.w[d2] : 0u)) {
+                    set_error("fe_density_splat: weight of offset (%d, %d, %d)", x, y, z);
+                    return FE_ERR_CUDA;
+                }
+            }
+        c->splat_ready = true;
     }
     c->splat_res[0] = rx;
     c->splat_res[1] = ry;
     c->splat_res[2] = rz;
-    // Counts per centre voxel, then the convolution with the tap table
+    // Counts per centre voxel, then the convolution with the weights
     // (fe_splat.cu).
     const int3 res = make_int3(rx, ry, rz);
     const size_t hist_n = (size_t)(rx + 1) * (ry + 1) * (rz + 1);
@@ -1641,8 +1644,7 @@ fe_status fe_density_splat(fe_ctx* c) {
     FE_CUDA(cudaMemsetAsync(c->splat_grid, 0, voxels * 4, c->stream));
     FE_CUDA(cudaMemsetAsync(c->splat_hist, 0, hist_n * 4, c->stream));
     FE_CUDA(splat_histogram(c->B.pos_a, c->n, b0, b1, res, c->splat_hist, c->stream));
-    FE_CUDA(splat_convolve(c->splat_hist, res, c->splat_taps, c->splat_ntaps, c->splat_grid,
-                           c->stream));
+    FE_CUDA(splat_convolve(c->splat_hist, res, c->splat_weights, c->splat_grid, c->stream));
     return FE_OK;
 }
 

@@ -3,16 +3,22 @@
 // Each particle inside the box adds uint(200 (1 - (d/8)^2)^3) to every voxel
 // at integer offset (x, y, z), d = |(x, y, z)| < 8, from its centre voxel
 // ivec3(uvw * grid_res), uvw = (p - box_min) / (box_max - box_min).  The
-// weight depends only on the offset, so it is evaluated once per offset (in
-// the shader's FP32 operation order) into a table of the 1,647 non-zero taps,
-// and the grid is the convolution of the per-centre-voxel particle counts with
-// that table: grid[v] = sum_t w_t * count[v - d_t].  Integer sums do not
-// depend on order, so the grid is bit-identical to the shader's scatter of
-// atomic adds.  One block per 8^3 output tile holds a 24^3 window of the
-// counts in shared memory; windows with no particle are skipped.  (Scattering
-// per particle with global reductions, or accumulating per tile with
-// shared-memory atomics, did the same sums 2.4x and 2.7x slower at 1M
-// particles on 128^3.)
+// weight depends on d^2 alone, so it is evaluated once per d^2 (in the shader's
+// FP32 operation order; 1,647 offsets, d^2 <= 53, have one that is not 0), and
+// the grid is the convolution of the per-centre-voxel particle counts with it:
+// grid[v] = sum_t w_t * count[v - d_t].  Integer sums do not depend on order,
+// so the grid is bit-identical to the shader's scatter of atomic adds.
+// (Scattering per particle with global reductions, or accumulating per tile
+// with shared-memory atomics, did the same sums 2.4x and 2.7x slower at 1M
+// particles on 128^3 than a plain convolution.)
+//
+// The weight depends on (y, z) through s = y^2 + z^2 alone, so the rows of
+// counts along x with the same s (up to 12 of the 169) are added up first and
+// then convolved along x once, with the weights of +x and -x together, eight
+// voxels a thread: per voxel some 340 additions and 400 multiply-adds on
+// registers and 100 16-byte shared loads, where the plain convolution's one
+// shared load and multiply-add per tap (1,647 of each) made it wait for shared
+// memory.
 #include "fe_splat.h"
 
 #include "fe_common.cuh"
@@ -59,8 +65,83 @@ __device__ __forceinline__ bool centre_voxel(float4 p, float3 bmin, float3 bmax,
     return true;
 }
 
-constexpr int kWin = kSplatTile + 2 * kSplatRadius;  // 24 voxels per axis
-constexpr int kWinVox = kWin * kWin * kWin;          // 13824
+// A block's output tile, and the window of counts it needs: 7 voxels around
+// it (the weights are 0 beyond), x rounded out to whole 16-byte groups and
+// padded so that the 16-byte loads of a quarter warp fall into different banks.
+constexpr int kTileX = 32, kTileY = 8, kTileZ = 8;
+constexpr int kReach = 7;
+constexpr int kPer = 8;                           // voxels along x per thread
+constexpr int kThreads = kTileX / kPer * kTileY * kTileZ;
+constexpr int kWinX = kTileX + 16, kWinY = kTileY + 2 * kReach, kWinZ = kTileZ + 2 * kReach;
+constexpr int kRow = kWinX + 4;                   // words from row to row
+constexpr size_t kWinBytes = (size_t)kRow * kWinY * kWinZ * 4;
+
+// The rows (y, z) with y^2 + z^2 <= kSplatMaxD2 sorted by that sum: one class
+// per sum, its rows as offsets in words into the window.
+struct RowClasses {
+    int n, rows;
+    int s[54], first[55], offset[192];
+};
+constexpr RowClasses make_classes() {
+    RowClasses c{};
+    for (int s = 0; s <= kSplatMaxD2; ++s) {
+        const int before = c.rows;
+        for (int z = -kReach; z <= kReach; ++z)
+            for (int y = -kReach; y <= kReach; ++y)
+                if (y * y + z * z == s) c.offset[c.rows++] = (z * kWinY + y) * kRow;
+        if (c.rows == before) continue;
+        c.s[c.n] = s;
+        c.first[c.n++] = before;
+    }
+    c.first[c.n] = c.rows;
+    return c;
+}
+constexpr RowClasses kClassTable = make_classes();
+__constant__ RowClasses kClasses = kClassTable;
+// Classes from here on reach at most 4 voxels along x.
+constexpr int first_narrow() {
+    int k = 0;
+    while (kClassTable.s[k] + 25 <= kSplatMaxD2) ++k;
+    return k;
+}
+constexpr int kNarrow = first_narrow();
+
+// Classes [c0, c1): adds up their rows from kReachX voxels left of the thread's
+// first one to kReachX right of its last (whole 16-byte groups) and convolves
+// along x.  `at`: the thread's first voxel in the window.
+template <int kReachX>
+__device__ __forceinline__ void add_classes(uint32_t (&acc)[kPer], const uint32_t* at, int c0,
+                                            int c1, const SplatWeights& W) {
+    constexpr int kSide = (kReachX + 3) / 4 * 4, kWords = kPer + 2 * kSide;
+    static_assert(kSide <= 8, "inside the window");
+#pragma unroll 1
+    for (int c = c0; c < c1; ++c) {
+        uint32_t row[kWords];
+#pragma unroll
+        for (int i = 0; i < kWords; ++i) row[i] = 0u;
+        const int end = kClasses.first[c + 1];
+#pragma unroll 2
+        for (int r = kClasses.first[c]; r < end; ++r) {
+            const uint4* p = reinterpret_cast<const uint4*>(at + kClasses.offset[r] - kSide);
+#pragma unroll
+            for (int i = 0; i < kWords; i += 4) {
+                const uint4 v = p[i / 4];
+                row[i] += v.x;
+                row[i + 1] += v.y;
+                row[i + 2] += v.z;
+                row[i + 3] += v.w;
+            }
+        }
+        const int s = kClasses.s[c];
+#pragma unroll
+        for (int k = 0; k <= kReachX; ++k) {
+            const uint32_t w = W.w[s + k * k];
+#pragma unroll
+            for (int i = 0; i < kPer; ++i)
+                acc[i] += w * (k ? row[kSide + i - k] + row[kSide + i + k] : row[kSide + i]);
+        }
+    }
+}
 
 __global__ void __launch_bounds__(256) k_splat_hist(const float4* __restrict__ pos, uint32_t n,
                                                     float3 bmin, float3 bmax, int3 res,
@@ -75,45 +156,39 @@ __global__ void __launch_bounds__(256) k_splat_hist(const float4* __restrict__ p
     atomicAdd(hist + ((size_t)cz * (res.y + 1) + cy) * (res.x + 1) + cx, 1u);
 }
 
-// grid[v] = sum_t w_t * hist[v - d_t] over the taps (offset d_t from a centre
-// to a voxel).  Block: 8^3 output voxels, 256 threads, two voxels each (z and
-// z + 4); the window holds hist for centres v - d, d in [-8, 8]^3.
-__global__ void __launch_bounds__(256) k_splat_conv(const uint32_t* __restrict__ hist, int3 res,
-                                                    const int4* __restrict__ taps,
-                                                    uint32_t n_taps,
-                                                    uint32_t* __restrict__ grid) {
-    extern __shared__ uint32_t win[];  // [kWin][kWin][kWin], origin = tile origin - radius
-    const int tdx = (res.x + kSplatTile - 1) / kSplatTile, tdy = (res.y + kSplatTile - 1) / kSplatTile;
+// One block per output tile; a window without particles leaves the grid at 0.
+__global__ void __launch_bounds__(kThreads, 2) k_splat_conv(const uint32_t* __restrict__ hist,
+                                                            int3 res, SplatWeights W,
+                                                            uint32_t* __restrict__ grid) {
+    extern __shared__ __align__(16) uint32_t win[];  // [kWinZ][kWinY][kRow]
+    const int tdx = (res.x + kTileX - 1) / kTileX, tdy = (res.y + kTileY - 1) / kTileY;
     const int tx = blockIdx.x % tdx, ty = (blockIdx.x / tdx) % tdy, tz = blockIdx.x / (tdx * tdy);
-    const int ox = tx * kSplatTile - kSplatRadius, oy = ty * kSplatTile - kSplatRadius,
-              oz = tz * kSplatTile - kSplatRadius;
+    const int ox = tx * kTileX - 8, oy = ty * kTileY - kReach, oz = tz * kTileZ - kReach;
     const int hx = res.x + 1, hy = res.y + 1, hz = res.z + 1;   // hist extent
     int any = 0;
-    for (int v = threadIdx.x; v < kWinVox; v += blockDim.x) {
-        const int x = ox + v % kWin, y = oy + (v / kWin) % kWin, z = oz + v / (kWin * kWin);
+#pragma unroll 4
+    for (int v = threadIdx.x; v < kWinX * kWinY * kWinZ; v += kThreads) {
+        const int wx = v % kWinX, wr = v / kWinX;
+        const int x = ox + wx, y = oy + wr % kWinY, z = oz + wr / kWinY;
         uint32_t c = 0u;
         if (x >= 0 && y >= 0 && z >= 0 && x < hx && y < hy && z < hz)
             c = __ldg(hist + ((size_t)z * hy + y) * hx + x);
-        win[v] = c;
+        win[wr * kRow + wx] = c;
         any |= c != 0u;
     }
-    if (!__syncthreads_or(any)) return;  // no particle within reach: the grid stays 0
-    const int lx = threadIdx.x & 7, ly = (threadIdx.x >> 3) & 7, lz = threadIdx.x >> 6;  // lz 0..3
-    uint32_t a0 = 0u, a1 = 0u;
-    for (uint32_t t = 0; t < n_taps; ++t) {
-        const int4 k = __ldg(taps + t);
-        // centre = voxel - offset, in window coordinates (+ radius)
-        const int wx = lx + kSplatRadius - k.x, wy = ly + kSplatRadius - k.y,
-                  wz = lz + kSplatRadius - k.z;
-        const uint32_t w = (uint32_t)k.w;
-        a0 += w * win[(wz * kWin + wy) * kWin + wx];
-        a1 += w * win[((wz + 4) * kWin + wy) * kWin + wx];
-    }
-    const int x = tx * kSplatTile + lx, y = ty * kSplatTile + ly, z0 = tz * kSplatTile + lz;
-    if (x < res.x && y < res.y) {
-        if (z0 < res.z) grid[((size_t)z0 * res.y + y) * res.x + x] = a0;
-        if (z0 + 4 < res.z) grid[((size_t)(z0 + 4) * res.y + y) * res.x + x] = a1;
-    }
+    if (!__syncthreads_or(any)) return;
+    const int lx = threadIdx.x % (kTileX / kPer) * kPer, ly = threadIdx.x / (kTileX / kPer) % kTileY,
+              lz = threadIdx.x / (kTileX / kPer * kTileY);
+    const uint32_t* at = win + ((lz + kReach) * kWinY + ly + kReach) * kRow + lx + 8;
+    uint32_t acc[kPer] = {};
+    add_classes<kReach>(acc, at, 0, kNarrow, W);
+    add_classes<4>(acc, at, kNarrow, kClassTable.n, W);
+    const int x = tx * kTileX + lx, y = ty * kTileY + ly, z = tz * kTileZ + lz;
+    if (y >= res.y || z >= res.z) return;
+    uint32_t* out = grid + ((size_t)z * res.y + y) * res.x + x;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i)
+        if (x + i < res.x) out[i] = acc[i];
 }
 
 }  // namespace
@@ -125,15 +200,14 @@ cudaError_t splat_histogram(const float4* pos, uint32_t n, float3 box_min, float
     return cudaGetLastError();
 }
 
-cudaError_t splat_convolve(const uint32_t* hist, int3 res, const int4* taps, uint32_t n_taps,
-                           uint32_t* grid, cudaStream_t stream) {
-    const int tdx = (res.x + kSplatTile - 1) / kSplatTile, tdy = (res.y + kSplatTile - 1) / kSplatTile,
-              tdz = (res.z + kSplatTile - 1) / kSplatTile;
-    const size_t smem = (size_t)kWinVox * 4;
+cudaError_t splat_convolve(const uint32_t* hist, int3 res, const SplatWeights& w, uint32_t* grid,
+                           cudaStream_t stream) {
+    const int tdx = (res.x + kTileX - 1) / kTileX, tdy = (res.y + kTileY - 1) / kTileY,
+              tdz = (res.z + kTileZ - 1) / kTileZ;
     cudaError_t e = cudaFuncSetAttribute(k_splat_conv, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+                                         (int)kWinBytes);
     if (e != cudaSuccess) return e;
-    k_splat_conv<<<tdx * tdy * tdz, 256, smem, stream>>>(hist, res, taps, n_taps, grid);
+    k_splat_conv<<<tdx * tdy * tdz, kThreads, kWinBytes, stream>>>(hist, res, w, grid);
     return cudaGetLastError();
 }
 
