@@ -367,6 +367,9 @@ struct fe_ctx {
     float4* image = nullptr;
     size_t image_cap = 0;
     int image_w = 0, image_h = 0;
+    uint32_t* ray_bits = nullptr;   // raymarch scratch, by grid size
+    uint8_t* ray_coarse = nullptr;
+    size_t ray_bits_cap = 0, ray_coarse_cap = 0;
 
     // fe_download_async: two device snapshots, the copy stream, and which
     // ticket each snapshot slot serves (0: none)
@@ -1708,6 +1711,18 @@ fe_status fe_raymarch(fe_ctx* c, const fe_camera* cam) {
     RaymarchArgs a;
     a.grid = c->splat_grid;
     a.res = make_int3(c->splat_res[0], c->splat_res[1], c->splat_res[2]);
+    const size_t bit_words = raymarch_bit_words(a.res), coarse_bytes = raymarch_coarse_bytes(a.res);
+    fe_status st;
+    if (bit_words > c->ray_bits_cap) {
+        if ((st = dev_alloc(c, &c->ray_bits, bit_words)) != FE_OK) return st;
+        c->ray_bits_cap = bit_words;
+    }
+    if (coarse_bytes > c->ray_coarse_cap) {
+        if ((st = dev_alloc(c, &c->ray_coarse, coarse_bytes)) != FE_OK) return st;
+        c->ray_coarse_cap = coarse_bytes;
+    }
+    a.bits = c->ray_bits;
+    a.coarse = c->ray_coarse;
     a.sky = c->sky;
     a.sky_w = c->sky_w;
     a.sky_h = c->sky_h;

@@ -9,6 +9,16 @@
 // Densities are nearest texel fetches of the splat grid with the shader's
 // manual trilinear blend; the sky is bilinear with clamp-to-edge (the
 // skybox sampler of water.rs:78-84).  discard -> alpha 0.
+//
+// The march and the thickness only ask whether the density at a point is above
+// the threshold, and for most points a coarse look answers that: a byte per
+// 4^3 voxels tells whether every texel that a point in them can blend (one
+// voxel more on each side, for the coarse index is approximate) is at most
+// 300, or every one at least 301.  A blend of texels up to 300 minus the
+// offset 300 is below the threshold 0.01 by far more than its rounding, and
+// one of texels from 301 on above it.  Only points near the surface evaluate
+// the shader's eight texels, three divisions and seven blends (about 120
+// instructions against 15).
 #include "fe_raymarch.h"
 
 namespace fe {
@@ -52,7 +62,56 @@ struct Scene {
     const uint32_t* grid;
     int3 res;
     V3 bmin, bmax;
+    const uint8_t* coarse;
+    V3 scale;   // voxels per length, rounded: for the coarse index alone
 };
+
+enum Coarse : uint8_t { kBelow = 0, kAbove = 1, kMixed = 2 };
+constexpr int kCoarse = 4;   // voxels per coarse block and axis
+__host__ __device__ constexpr int coarse_dim(int res) { return (res + kCoarse - 1) / kCoarse; }
+
+// Bit x % 32 of word [z][y][x / 32]: texel x is at least 301.
+__global__ void __launch_bounds__(256) k_coarse_bits(const uint32_t* __restrict__ grid, int3 res,
+                                                     uint32_t* __restrict__ bits) {
+    const int words = (res.x + 31) / 32;
+    const size_t w = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (w >= (size_t)words * res.y * res.z) return;
+    const int x = (int)(w % words) * 32 + (int)(threadIdx.x & 31u);
+    const bool above = x < res.x && __ldg(grid + w / words * res.x + x) > (uint32_t)kOffset;
+    const uint32_t b = __ballot_sync(0xFFFFFFFFu, above);
+    if ((threadIdx.x & 31u) == 0) bits[w] = b;
+}
+
+// Block b covers the points whose lower texel is in [4b, 4b + 3]; with the
+// upper texel and one voxel of slack on each side, texels 4b - 1 .. 4b + 5.
+// kAbove only where all of those are inside the grid: beyond the box the
+// density is 0.
+__global__ void __launch_bounds__(128) k_coarse(const uint32_t* __restrict__ bits, int3 res,
+                                                uint8_t* __restrict__ coarse) {
+    const int nx = coarse_dim(res.x), ny = coarse_dim(res.y), nz = coarse_dim(res.z);
+    const size_t t = (size_t)blockIdx.x * 128 + threadIdx.x;
+    if (t >= (size_t)nx * ny * nz) return;
+    const int x0 = (int)(t % nx) * kCoarse - 1, y0 = (int)(t / nx % ny) * kCoarse - 1,
+              z0 = (int)(t / ((size_t)nx * ny)) * kCoarse - 1;
+    constexpr int kSpan = kCoarse + 3;
+    const int words = (res.x + 31) / 32;
+    uint32_t any = 0, all = kSpan < 32 ? (1u << kSpan) - 1u : 0u;
+    const uint32_t span = all;
+    for (int z = max(z0, 0); z < min(z0 + kSpan, res.z); ++z)
+        for (int y = max(y0, 0); y < min(y0 + kSpan, res.y); ++y) {
+            const uint32_t* row = bits + ((size_t)z * res.y + y) * words;
+            // bits x0 .. x0 + kSpan - 1 (0 outside the grid)
+            const int lo = x0 >> 5;   // -1 for x0 = -1
+            const uint32_t a = lo >= 0 ? __ldg(row + lo) : 0u;
+            const uint32_t b = lo + 1 < words ? __ldg(row + lo + 1) : 0u;
+            const uint32_t m = __funnelshift_r(a, b, x0 & 31) & span;
+            any |= m;
+            all &= m;
+        }
+    const bool inside = x0 >= 0 && y0 >= 0 && z0 >= 0 && x0 + kSpan <= res.x &&
+                        y0 + kSpan <= res.y && z0 + kSpan <= res.z;
+    coarse[t] = !any ? kBelow : (inside && all == span) ? kAbove : kMixed;
+}
 
 __device__ __forceinline__ float texel(const Scene& S, int x, int y, int z) {
     x = min(max(x, 0), S.res.x - 1);
@@ -79,6 +138,22 @@ __device__ float get_density(const Scene& S, V3 p) {
     const float v0 = mixf(mixf(v000, v100, tx), mixf(v010, v110, tx), ty);
     const float v1 = mixf(mixf(v001, v101, tx), mixf(v011, v111, tx), ty);
     return fmaxf(0.0f, (mixf(v0, v1, tz) - kOffset) * kMultiplier);
+}
+
+// Coarse cell of a point along one axis.
+__device__ __forceinline__ int coarse_index(float d, float scale, int res) {
+    const int i = __float2int_rd(__fmaf_rn(d, scale, -0.5f));   // NaN -> 0, saturating
+    return min(max(i, 0), res - 1) / kCoarse;
+}
+
+// getDensity(p) > DENSITY_THRESHOLD.
+__device__ bool is_water(const Scene& S, V3 p) {
+    const int x = coarse_index(p.x - S.bmin.x, S.scale.x, S.res.x),
+              y = coarse_index(p.y - S.bmin.y, S.scale.y, S.res.y),
+              z = coarse_index(p.z - S.bmin.z, S.scale.z, S.res.z);
+    const uint8_t c = __ldg(S.coarse + ((size_t)z * coarse_dim(S.res.y) + y) *
+                                           coarse_dim(S.res.x) + x);
+    return c == kMixed ? get_density(S, p) > kThreshold : c == kAbove;
 }
 
 __device__ V3 calc_normal(const Scene& S, V3 p) {
@@ -117,7 +192,7 @@ __device__ float calc_thickness(const Scene& S, V3 p, V3 dir, float t_max) {
     const float d_step = 0.015f;
     float t = 0.0f;
     for (int i = 0; i < 64 && t < t_max; i++, t += d_step)
-        if (get_density(S, p + dir * t) > kThreshold) thickness += d_step;
+        if (is_water(S, p + dir * t)) thickness += d_step;
     return thickness;
 }
 
@@ -149,7 +224,8 @@ __global__ void __launch_bounds__(128) k_raymarch(RaymarchArgs A) {
     const V3 center = v3(A.box_min.x + size.x * 0.5f, A.box_min.y + size.y * 0.5f,
                          A.box_min.z + size.z * 0.5f);
     const V3 scale = v3(sqrtf(size.x * size.x), sqrtf(size.y * size.y), sqrtf(size.z * size.z));
-    Scene S{A.grid, A.res, center - scale * 0.5f, center + scale * 0.5f};
+    Scene S{A.grid, A.res, center - scale * 0.5f, center + scale * 0.5f, A.coarse, {}};
+    S.scale = v3((float)A.res.x, (float)A.res.y, (float)A.res.z) / (S.bmax - S.bmin);
 
     // intersectAABB (raymarch.frag:47-52)
     const V3 t1 = (S.bmin - ray_org) / ray_dir, t2 = (S.bmax - ray_org) / ray_dir;
@@ -164,7 +240,7 @@ __global__ void __launch_bounds__(128) k_raymarch(RaymarchArgs A) {
     bool hit = false;
     for (int i = 0; i < kMaxSteps; i++) {
         if (t_cur > t_far) break;
-        if (get_density(S, ray_org + ray_dir * t_cur) > kThreshold) {
+        if (is_water(S, ray_org + ray_dir * t_cur)) {
             hit = true;
             break;
         }
@@ -177,7 +253,7 @@ __global__ void __launch_bounds__(128) k_raymarch(RaymarchArgs A) {
     float ta = t_cur - step_world, tb = t_cur;
     for (int i = 0; i < 8; i++) {
         const float m = (ta + tb) * 0.5f;
-        if (get_density(S, ray_org + ray_dir * m) > kThreshold)
+        if (is_water(S, ray_org + ray_dir * m))
             tb = m;
         else
             ta = m;
@@ -232,7 +308,15 @@ __global__ void __launch_bounds__(128) k_raymarch(RaymarchArgs A) {
 
 }  // namespace
 
+size_t raymarch_bit_words(int3 res) { return (size_t)((res.x + 31) / 32) * res.y * res.z; }
+size_t raymarch_coarse_bytes(int3 res) {
+    return (size_t)coarse_dim(res.x) * coarse_dim(res.y) * coarse_dim(res.z);
+}
+
 cudaError_t raymarch(const RaymarchArgs& a, cudaStream_t stream) {
+    const size_t words = raymarch_bit_words(a.res), blocks = raymarch_coarse_bytes(a.res);
+    k_coarse_bits<<<(unsigned)((words + 7) / 8), 256, 0, stream>>>(a.grid, a.res, a.bits);
+    k_coarse<<<(unsigned)((blocks + 127) / 128), 128, 0, stream>>>(a.bits, a.res, a.coarse);
     dim3 grid((a.width + 15) / 16, (a.height + 7) / 8);
     k_raymarch<<<grid, 128, 0, stream>>>(a);
     return cudaGetLastError();
