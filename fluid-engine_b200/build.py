@@ -24,12 +24,12 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "fluid_step", "libfluidstep.so")
 CONTRACT_OUT = os.path.join(HERE, "fluid_step", "libfluidstep_contract.so")
-CONTRACT_SOURCES = ["fe_kernels.cu"]
+CONTRACT_SOURCES = ["fe_kernels.cu", "fe_resident.cu"]
 BUILD = os.path.join(HERE, "_build")
 
 SOURCES = ["fe_kernels.cu", "fe_sort.cu", "fe_api.cu", "fe_sort_noalloc.cu", "fe_mlp.cu", "fe_tune.cu",
            "fe_splat.cu", "fe_raymarch.cu",
-           "fe_model.cu", "fe_learned.cu"]
+           "fe_model.cu", "fe_learned.cu", "fe_resident.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-prec-div=true",
          "-prec-sqrt=true", "-ftz=false", "-Xcompiler", "-fPIC,-fvisibility=hidden",

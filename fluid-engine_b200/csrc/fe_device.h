@@ -130,6 +130,14 @@ struct CellSort {
     unsigned long long* ticket;
 };
 
+// Scratch of the resident solve (k_solve_resident).
+constexpr int kResidentMaxThreads = 384;
+struct ResidentScratch {
+    float* pr;               // p / rho^2 per particle
+    double *sums, *maxes;    // per warp of 32 particles, 8 per chunk
+    uint32_t* barrier;       // arrivals, leavers; zero between launches
+};
+
 // Learned warm start and training-data capture (fe_learned.cu).
 // carry[i] travels with particle i through every re-sort:
 //   x = final pressure of the last density solve, y = of the last

@@ -75,3 +75,29 @@ def test_frame_solve_is_the_solve_pass_by_pass(mode, n, iters, non_finite):
             assert bad.size == 0, (k, f, bad.size, a.reshape(-1)[bad[0]], b.reshape(-1)[bad[0]])
     sim.close()
     data.close()
+
+
+@pytest.mark.parametrize("n", [9472, 9473, 18945, 28417])
+@pytest.mark.parametrize("cap", [100, 3])
+def test_resident_solve_of_every_block_size(oracle_mod, n, cap):
+    """The solve of few particles as one kernel, around the sizes where its
+    block grows: iterations to a tolerance (the FP64 sums over warps and chunks)
+    and to a cap, against the oracle."""
+    p = scene.dam_break_params((0, 0, 0), (4.0, 4.0, 4.0), mode=_abi.FE_MODE_FIXED,
+                               solver=_abi.FE_SOLVER_TOLERANCE)
+    p.max_iterations = cap
+    pos, _ = scene.lattice((0, 0, 0), (31, 31, 31), 0.025, 1000.0, 0.05, 0.03, 5)
+    pos = pos[:n]
+    vel = np.random.default_rng(n).normal(0, 0.3, pos.shape).astype(np.float32)
+    sim, orc = Simulation(pos, p, velocities=vel), oracle_mod.Oracle(p, pos, vel)
+    for _ in range(2):
+        a, b = sim.step(1), orc.step(1)
+        for name in ("density_iterations", "divergence_iterations", "density_residual",
+                     "divergence_residual", "density_residual_max", "divergence_residual_max"):
+            assert getattr(a, name) == getattr(b, name), name
+        assert bool(a.flags & _abi.FE_STATS_ITERATION_CAP_HIT) == (
+            cap == 3 or bool(b.flags & _abi.FE_STATS_ITERATION_CAP_HIT))
+    for f in FIELDS:
+        x, y = sim.data.download(f).view(np.uint32), orc.field(f).view(np.uint32)
+        assert np.array_equal(x, y), f
+    sim.close()
