@@ -723,8 +723,8 @@ fe_status rec_solve_resident(fe_ctx* c, Recorder& R, int which) {
 
 // The shape of the resident solve: one particle per thread, a block per SM,
 // as many list entries in shared memory as fit (all 64 up to 192 threads).
-// The line: 16k particles' frame of 4 + 4 iterations 272 -> 161 us, 25k 301 ->
-// 176, 50k (37 entries fit) 325 -> 284, 70k (27 entries, 512 threads) 338 -> 366.
+// The line: 16k particles' frame of 4 + 4 iterations 272 -> 156 us, 25k 301 ->
+// 171, 50k (37 entries fit) 325 -> 251; with 512 threads 27 entries fit.
 #ifndef FE_RESIDENT_MAX
 #define FE_RESIDENT_MAX (148 * kResidentMaxThreads)
 #endif

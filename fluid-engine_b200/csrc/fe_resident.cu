@@ -4,7 +4,7 @@
 // pressure_update each take some 7 us of which 2 are the launch and most of the
 // rest the chain parameters -> count -> list words -> neighbours, and the graph's
 // WHILE node adds 7 us between iterations (16k particles: 24 us an iteration,
-// here 9.4).
+// here 8.6).
 // Here every particle keeps a thread, and every SM a block, for all the
 // iterations.  The pair gradients, which do not change during a solve, stay in
 // shared memory with the neighbours' indices, so an iteration is two gathers
@@ -29,7 +29,11 @@ namespace {
 constexpr int kBarrierSpins = 1 << 22;
 
 // Barrier number `k` (1, 2, ...) of the launch over all blocks.  False, with
-// the flag raised, if it did not come about.  Whole block.
+// the flag raised, if it did not come about.  Whole block.  Every thread's
+// stores before it come before every thread's loads after it (release and
+// acquire by one thread, bar.sync for the others), so the gathers are plain
+// loads, which the neighbours that a cell's particles share make L1 hits
+// (through L2 alone an iteration took 14.0 us instead of 11.2 at 37k particles).
 __device__ __forceinline__ bool grid_barrier(const Bufs& B, uint32_t* count, uint32_t k) {
     __syncthreads();
     int ok = 1;
@@ -50,10 +54,6 @@ __device__ __forceinline__ bool grid_barrier(const Bufs& B, uint32_t* count, uin
     }
     return __syncthreads_and(ok || threadIdx.x != 0);
 }
-
-// Loads that see other blocks' stores of this launch.
-__device__ __forceinline__ float ld_shared_l2(const float* p) { return __ldcg(p); }
-__device__ __forceinline__ float4 ld_shared_l2(const float4* p) { return __ldcg(p); }
 
 struct Particle {
     const float4* cache;   // [rows][blockDim.x]: gradient, neighbour index
@@ -138,7 +138,7 @@ __device__ __forceinline__ void sum_warps(const double* sums, const double* maxe
 // shared memory.
 // kMaxThreads: bounds the block, and with it the registers a thread may take
 // for its loads in flight.  16 entries at a time in the force and 8 in the
-// update; all 36 and 18 at once made an iteration 9.4 -> 12.2 us at 16k
+// update; all 36 and 18 at once made an iteration 2.8 us longer at 16k
 // particles (more predicated instructions than latencies saved).
 template <int kMaxThreads>
 __global__ void __launch_bounds__(kMaxThreads, 1)
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         if (live) {
             float sum_ap = 0.0f;
             for_each_cached<kUpdateBatch>(
-                B, P, q, [&](uint32_t j) { return ld_shared_l2(accp(B, j)); },
+                B, P, q, [&](uint32_t j) { return *accp(B, j); },
                 [&](f3 grad, float4 aj) {
                     const f3 ad = sub(ai, xyz(aj));
                     sum_ap += m * dot(ad, grad);
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         acc = {0.0f, 0.0f, 0.0f};
         const float pr_i = p_over_rho2();
         for_each_cached<kForceBatch>(
-            B, P, q, [&](uint32_t j) { return ld_shared_l2(R.pr + j); },
+            B, P, q, [&](uint32_t j) { return R.pr[j]; },
             [&](f3 grad, float pr_j) {
                 if (pr_j == pr_j) acc = add(acc, scale(m * (pr_i + pr_j), grad));
             });
