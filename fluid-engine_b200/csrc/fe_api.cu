@@ -2124,6 +2124,26 @@ fe_status sort_pairs_impl(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t k
     std::lock_guard<std::mutex> lock(g_sort_mutex);
     SortScratch& S = g_sort[dev];
     const uint32_t kb = key_bits ? key_bits : 32;
+    // Few pairs: one cluster sorts them in one launch, whatever shape is tuned
+    // (us, 32-bit keys, copies of the input included; onesweep at its default
+    // shape / this: 1k 48/24, 32k 60/31, 64k 62/43).  An explicit shape is taken
+    // as it is.
+    if (!forced && n <= kSmallSortMax) {
+        if (S.flags) {
+            FE_CUDA(cudaStreamWaitEvent(stream, S.done, 0));
+        } else {   // the error word alone: its scratch grows when a sort needs it
+            if (!S.done) FE_CUDA(cudaEventCreateWithFlags(&S.done, cudaEventDisableTiming));
+            FE_CUDA(cudaMalloc(&S.words, 32));
+            S.flags = S.words;
+            S.device = dev;
+        }
+        const cudaError_t e = radix_sort_small(keys, vals, n, kb, S.flags, stream);
+        if (e == cudaSuccess) {
+            FE_CUDA(cudaEventRecord(S.done, stream));
+            return FE_OK;
+        }
+        (void)cudaGetLastError();   // no room for the cluster: the general sort
+    }
     RadixConfig cfg = kRadixDefault;
     if (forced)
         cfg = *forced;
@@ -2135,7 +2155,7 @@ fe_status sort_pairs_impl(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t k
         cudaFree(S.tk);
         cudaFree(S.tv);
         cudaFree(S.words);
-        S.tk = S.tv = S.words = nullptr;
+        S.tk = S.tv = S.words = S.flags = nullptr;
         uint32_t cap = std::max(n, S.cap);
         size_t nw = std::max(words, S.nwords);
         FE_CUDA(cudaMalloc(&S.tk, (size_t)cap * 4));

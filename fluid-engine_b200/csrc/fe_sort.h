@@ -60,6 +60,14 @@ cudaError_t radix_sort(const SortLaunch& L, uint32_t* keys, uint32_t* vals, uint
                        uint32_t* error_flags, bool* result_in_tmp,
                        RadixConfig cfg = kRadixDefault);
 
+// The same sort of at most kSmallSortMax pairs, in place and in one launch (a
+// cluster of blocks), without scratch.  Clears the 8 error words (may be NULL):
+// it has no wait that could give up.  Fails where the device cannot place a
+// cluster of the size it takes.
+constexpr uint32_t kSmallSortMax = 65536;
+cudaError_t radix_sort_small(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t key_bits,
+                             uint32_t* error_flags, cudaStream_t stream);
+
 // In-place bitonic network; n must be a power of two.
 cudaError_t bitonic_sort(const SortLaunch& L, uint32_t* keys, uint32_t* vals, uint32_t n);
 
