@@ -75,18 +75,27 @@ cudaError_t infer(const Params& P, const __nv_bfloat16* X, float* out, uint32_t 
                   uint32_t* error_flags, cudaStream_t stream, int num_sms,
                   int ctas_per_sm = kInferDefaultCtasPerSm);
 
-// Writes d(loss)/d(params) of the mean squared error over the n samples to
-// grad[kParams] and the summed squared error to grad[kParams].  Blocks sum
-// their tiles into their own slice of part[min(tiles, num_sms)][kParams + 1],
-// and the slices are added in block order: the same inputs give the same
-// gradients bit for bit.
-cudaError_t train_grads(const Params& P, const __nv_bfloat16* X, const float* Y, uint32_t n,
-                        float* grad, float* part, uint32_t* error_flags, cudaStream_t stream,
-                        int num_sms);
+// Floats of a block's gradient slice: kParams, the loss, and padding to 16
+// bytes.
+constexpr uint32_t kSlice = (kParams + 1 + 3) / 4 * 4;
 
-cudaError_t adam(float* master, float* grad, float* m, float* v, __nv_bfloat16* bf16_copy,
-                 uint32_t count, uint32_t bf16_count, float lr, float beta1, float beta2, float eps,
-                 uint32_t step, float weight_decay, cudaStream_t stream);
+// Writes d(loss)/d(params) of the mean squared error over the n samples (raw
+// rows of kFeatures features and 2 targets, standardised with norm: x mean,
+// x std, y mean, y std) to grad[kParams] and the summed squared error to
+// grad[kParams].  Blocks sum their tiles into their own slice of
+// part[min(tiles, num_sms)][kSlice], and the slices are added in block order:
+// the same inputs give the same gradients bit for bit.
+cudaError_t train_grads(const Params& P, const float* X, const float* Y, const float* norm,
+                        uint32_t n, float* grad, float* part, uint32_t* error_flags,
+                        cudaStream_t stream, int num_sms);
+
+// The same followed by one Adam step on the slices' sums (P: the parameters in
+// bf16_copy and master, which are updated); the summed squared error to *loss.
+cudaError_t train_step(const Params& P, const float* X, const float* Y, const float* norm,
+                       uint32_t n, float* part, uint32_t* error_flags, float* master, float* m,
+                       float* v, __nv_bfloat16* bf16_copy, float* loss, float lr, float beta1,
+                       float beta2, float eps, uint32_t step, float weight_decay,
+                       cudaStream_t stream, int num_sms);
 
 }  // namespace mlp
 }  // namespace fe

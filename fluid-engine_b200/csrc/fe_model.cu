@@ -40,14 +40,6 @@ __global__ void k_prepare_x(const float* __restrict__ x, const float* __restrict
     dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
 }
 
-__global__ void k_standardize_y(const float* __restrict__ y, const float* __restrict__ norm,
-                                float* __restrict__ ys, uint32_t n) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 2 * n) return;
-    uint32_t c = i & 1u;
-    ys[i] = (y[i] - norm[24 + c]) / norm[26 + c];
-}
-
 __global__ void k_destandardize_y(float* __restrict__ y, const float* __restrict__ norm, uint32_t n) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= 2 * n) return;
@@ -74,12 +66,9 @@ __global__ void k_to_bf16(const float* __restrict__ src, __nv_bfloat16* __restri
 fe_status fe_model::ensure_scratch(uint32_t n) {
     if (n <= scratch_rows) return FE_OK;
     cudaFree(xb);
-    cudaFree(ys);
     xb = nullptr;
-    ys = nullptr;
     uint32_t rows = n + 1024;
     M_CUDA(cudaMalloc(&xb, (size_t)rows * 16 * sizeof(__nv_bfloat16)));
-    M_CUDA(cudaMalloc(&ys, (size_t)rows * 2 * sizeof(float)));
     scratch_rows = rows;
     return FE_OK;
 }
@@ -123,7 +112,7 @@ FE_API fe_status fe_model_create(uint32_t seed, int device, fe_model** out) {
     };
     if (cudaMalloc(&m->master, mlp::kParams * 4) != cudaSuccess ||
         cudaMalloc(&m->grad, (mlp::kParams + 1) * 4) != cudaSuccess ||
-        cudaMalloc(&m->grad_part, (size_t)m->num_sms * (mlp::kParams + 1) * 4) != cudaSuccess ||
+        cudaMalloc(&m->grad_part, (size_t)m->num_sms * mlp::kSlice * 4) != cudaSuccess ||
         cudaMalloc(&m->adam_m, mlp::kParams * 4) != cudaSuccess ||
         cudaMalloc(&m->adam_v, mlp::kParams * 4) != cudaSuccess ||
         cudaMalloc(&m->wbf16, mlp::kWeights * 2) != cudaSuccess ||
@@ -165,7 +154,7 @@ FE_API fe_status fe_model_destroy(fe_model* m) {
     cudaDeviceSynchronize();
     for (void* p : {(void*)m->master, (void*)m->grad, (void*)m->grad_part, (void*)m->adam_m,
                     (void*)m->adam_v,
-                    (void*)m->wbf16, (void*)m->norm, (void*)m->flags, (void*)m->xb, (void*)m->ys})
+                    (void*)m->wbf16, (void*)m->norm, (void*)m->flags, (void*)m->xb})
         if (p) cudaFree(p);
     delete m;
     return FE_OK;
@@ -255,17 +244,6 @@ FE_API fe_status fe_model_forward(fe_model* m, const float* d_x, float* d_y, uin
     return FE_OK;
 }
 
-static fe_status model_grads(fe_model* m, const float* d_x, const float* d_y, uint32_t n,
-                             cudaStream_t s) {
-    fe_status st = m->prepare_x(d_x, n, s);
-    if (st != FE_OK) return st;
-    k_standardize_y<<<(2 * n + 255) / 256, 256, 0, s>>>(d_y, m->norm, m->ys, n);
-    M_CUDA(cudaGetLastError());
-    M_CUDA(mlp::train_grads(m->params(), m->xb, m->ys, n, m->grad, m->grad_part, m->flags, s,
-                            m->num_sms));
-    return FE_OK;
-}
-
 FE_API fe_status fe_model_gradients(fe_model* m, const float* d_x, const float* d_y, uint32_t n,
                                     float* h_grads, float* h_loss) {
     if (!m || !d_x || !d_y || n == 0) {
@@ -274,8 +252,8 @@ FE_API fe_status fe_model_gradients(fe_model* m, const float* d_x, const float* 
     }
     M_CUDA(cudaSetDevice(m->device));
     M_CUDA(cudaMemset(m->grad, 0, (mlp::kParams + 1) * 4));
-    fe_status st = model_grads(m, d_x, d_y, n, nullptr);
-    if (st != FE_OK) return st;
+    M_CUDA(mlp::train_grads(m->params(), d_x, d_y, m->norm, n, m->grad, m->grad_part, m->flags,
+                            nullptr, m->num_sms));
     M_CUDA(cudaDeviceSynchronize());
     uint32_t flags = 0;
     M_CUDA(cudaMemcpy(&flags, m->flags, 4, cudaMemcpyDeviceToHost));
@@ -297,12 +275,10 @@ FE_API fe_status fe_model_train_step(fe_model* m, const float* d_x, const float*
     }
     cudaStream_t s = (cudaStream_t)stream;
     M_CUDA(cudaSetDevice(m->device));
-    if (h_loss) M_CUDA(cudaMemsetAsync(m->grad + mlp::kParams, 0, 4, s));
-    fe_status st = model_grads(m, d_x, d_y, n, s);
-    if (st != FE_OK) return st;
     m->step += 1;
-    M_CUDA(mlp::adam(m->master, m->grad, m->adam_m, m->adam_v, m->wbf16, mlp::kParams,
-                     mlp::kWeights, lr, 0.9f, 0.999f, 1e-8f, m->step, weight_decay, s));
+    M_CUDA(mlp::train_step(m->params(), d_x, d_y, m->norm, n, m->grad_part, m->flags, m->master,
+                           m->adam_m, m->adam_v, m->wbf16, m->grad + mlp::kParams, lr, 0.9f,
+                           0.999f, 1e-8f, m->step, weight_decay, s, m->num_sms));
     if (h_loss) {
         M_CUDA(cudaMemcpyAsync(h_loss, m->grad + mlp::kParams, 4, cudaMemcpyDeviceToHost, s));
         M_CUDA(cudaStreamSynchronize(s));

@@ -14,7 +14,7 @@ struct fe_model {
     int num_sms = 148;
     float* master = nullptr;          // FP32 parameters (fe::mlp layout)
     float* grad = nullptr;            // gradients + 1 loss accumulator
-    float* grad_part = nullptr;       // per-block gradient slices [num_sms][kParams + 1]
+    float* grad_part = nullptr;       // per-block gradient slices [num_sms][kSlice]
     float* adam_m = nullptr;
     float* adam_v = nullptr;
     __nv_bfloat16* wbf16 = nullptr;   // BF16 weights for the tensor cores
@@ -22,7 +22,6 @@ struct fe_model {
     float h_norm[32] = {0};
     uint32_t* flags = nullptr;        // device error word
     __nv_bfloat16* xb = nullptr;      // scratch: standardised BF16 rows
-    float* ys = nullptr;              // scratch: standardised targets
     uint32_t scratch_rows = 0;
     uint32_t step = 0;
 
