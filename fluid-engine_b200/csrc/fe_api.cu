@@ -345,6 +345,7 @@ struct fe_ctx {
     // resident solve: its scratch and launch shape (threads 0: not used)
     ResidentScratch resident{};
     uint32_t resident_threads = 0, resident_rows = 0;
+    uint32_t resident_many_blocks = 0;   // of k_solve_resident_many
     uint4* upart = nullptr;
     uint32_t key_bits = 32;
     bool prepared = false;
@@ -721,6 +722,29 @@ fe_status rec_solve_resident(fe_ctx* c, Recorder& R, int which) {
     return FE_OK;
 }
 
+// Whether the solves run resident over strided chunks: one scene, or several
+// that all iterate a fixed number of times.
+bool resident_many(const fe_ctx* c) {
+    if (!c->resident_many_blocks) return false;
+    if (c->B.n_scenes == 1) return true;
+    for (const fe_params& p : c->params)
+        if (p.solver != FE_SOLVER_FIXED_ITERS) return false;
+    return !c->learned();
+}
+
+fe_status rec_solve_resident_many(fe_ctx* c, Recorder& R, int which) {
+    int begun = 0;
+    if (which == 0 && !c->learned()) {
+        REC(R.k(k_pressure_first, chunk_grid(c), dim3(kBlock), c->B, (cudaGraphConditionalHandle)0,
+                0));
+        begun = 1;
+    }
+    void* args[] = {&c->B, &c->resident, &which, &begun};
+    REC(R.launch((const void*)k_solve_resident_many, dim3(c->resident_many_blocks), dim3(kBlock), 0,
+                 args, true));
+    return FE_OK;
+}
+
 // The shape of the resident solve: one particle per thread, a block per SM,
 // as many list entries in shared memory as fit (all 64 up to 192 threads).
 // The line: 16k particles' frame of 4 + 4 iterations 272 -> 156 us, 25k 301 ->
@@ -728,11 +752,20 @@ fe_status rec_solve_resident(fe_ctx* c, Recorder& R, int which) {
 #ifndef FE_RESIDENT_MAX
 #define FE_RESIDENT_MAX (148 * kResidentMaxThreads)
 #endif
+#ifndef FE_RESIDENT_MANY_MAX
+#define FE_RESIDENT_MANY_MAX (1u << 20)
+#endif
 fe_status choose_resident(fe_ctx* c) {
-    if (c->B.n_scenes != 1 || c->n > FE_RESIDENT_MAX) return FE_OK;
     int smem_max = 0, cooperative = 0, blocks = 0;
     FE_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
     FE_CUDA(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, c->device));
+    if (cooperative && c->n <= FE_RESIDENT_MANY_MAX) {
+        FE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_solve_resident_many,
+                                                              kBlock, 0));
+        c->resident_many_blocks =
+            std::min<uint32_t>(c->B.n_chunks, (uint32_t)(blocks * c->num_sms));
+    }
+    if (c->B.n_scenes != 1 || c->n > FE_RESIDENT_MAX) return FE_OK;
     uint32_t threads = 64;
     while ((c->n + threads - 1) / threads > (uint32_t)c->num_sms) threads += 64;
     if (!cooperative || threads > (uint32_t)kResidentMaxThreads) return FE_OK;
@@ -754,6 +787,7 @@ fe_status choose_resident(fe_ctx* c) {
 // the same kernels with a host loop on the device flag.
 fe_status rec_solve(fe_ctx* c, Recorder& R, int which) {
     if (c->resident_threads) return rec_solve_resident(c, R, which);
+    if (resident_many(c)) return rec_solve_resident_many(c, R, which);
     Bufs B = c->B;
     fe_status st;
     if (!R.graph) {
@@ -962,7 +996,8 @@ size_t field_bytes(const fe_ctx* c, fe_field f, void** dptr, size_t* elem, size_
 uint64_t graph_key(const fe_ctx* c, uint32_t n_substeps, bool init) {
     return (uint64_t)n_substeps | ((uint64_t)init << 32) | ((uint64_t)c->sort_algorithm() << 33) |
            ((uint64_t)c->fixed_mode() << 34) | ((uint64_t)c->learned() << 35) |
-           ((uint64_t)c->capture << 36) | ((uint64_t)c->trace_slots << 40);
+           ((uint64_t)c->capture << 36) | ((uint64_t)resident_many(c) << 37) |
+           ((uint64_t)c->trace_slots << 40);
 }
 
 fe_status get_graph(fe_ctx* c, uint32_t n_substeps, bool init, cudaGraphExec_t* out) {
@@ -1256,9 +1291,9 @@ fe_status create_ctx(const fe_params* params, const uint32_t* counts, uint32_t n
         (s = dev_alloc(c, &cs.status, (size_t)scan_tiles + 1)) || (s = choose_resident(c)))
         return fail(s);
     ResidentScratch& rs = c->resident;
+    if ((s = dev_alloc(c, &rs.barrier, 2))) return fail(s);
     if (c->resident_threads) {
-        if ((s = dev_alloc(c, &rs.pr, n)) || (s = dev_alloc(c, &rs.sums, 16 * (size_t)nchunks)) ||
-            (s = dev_alloc(c, &rs.barrier, 2)))
+        if ((s = dev_alloc(c, &rs.pr, n)) || (s = dev_alloc(c, &rs.sums, 16 * (size_t)nchunks)))
             return fail(s);
         rs.maxes = rs.sums + 8 * (size_t)nchunks;
     }
@@ -1296,7 +1331,7 @@ fe_status create_ctx(const fe_params* params, const uint32_t* counts, uint32_t n
         cs.ticket = cs.status + scan_tiles;
         FE_CUDA(cudaMemset(cs.count, 0, (size_t)c->T * 4));
         FE_CUDA(cudaMemset(cs.status, 0, ((size_t)scan_tiles + 1) * 8));
-        if (c->resident_threads) FE_CUDA(cudaMemset(rs.barrier, 0, 8));
+        FE_CUDA(cudaMemset(rs.barrier, 0, 8));
         FE_CUDA(cudaMemset(B.S, 0, sizeof(SceneState) * n_scenes));
         FE_CUDA(cudaMemset(B.G, 0, sizeof(GlobalState)));
         FE_CUDA(cudaMemcpy(B.P, c->dparams.data(), sizeof(DevParams) * n_scenes,

@@ -152,6 +152,17 @@ __device__ __forceinline__ void ld_pair(const float4* base, uint32_t j, float4& 
                  : "l"(p));
 }
 
+// The same where other blocks of the launch write the records.
+__device__ __forceinline__ void ld_pair_coherent(const float4* base, uint32_t j, float4& a,
+                                                 float4& b) {
+    const float4* p = base + 2 * (size_t)j;
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z),
+                   "=f"(b.w)
+                 : "l"(p)
+                 : "memory");
+}
+
 // Both halves of particle i's record in one 256-bit store: the 32-byte sector
 // is written whole, so L2 never merges a half-written sector with DRAM.
 __device__ __forceinline__ void st_record(const Bufs& B, uint32_t i, float4 pos, float4 acc) {

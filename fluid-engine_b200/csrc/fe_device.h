@@ -132,6 +132,7 @@ struct CellSort {
 
 // Scratch of the resident solve (k_solve_resident).
 constexpr int kResidentMaxThreads = 384;
+constexpr int kResidentBlocks = 4;   // per SM, of k_solve_resident_many
 struct ResidentScratch {
     float* pr;               // p / rho^2 per particle
     double *sums, *maxes;    // per warp of 32 particles, 8 per chunk

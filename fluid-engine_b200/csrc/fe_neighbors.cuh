@@ -176,20 +176,23 @@ __device__ __forceinline__ void for_each_entry(const Bufs& B, uint32_t i, uint32
 }
 
 // Neighbours with r > 1e-6 in walk order: f(r_vec, grad_scale, pos_j), where
-// pos_j = pos_b[j] (w = p_j / rho_j^2).
-template <int kThreads, class F>
+// pos_j = pos_b[j] (w = p_j / rho_j^2).  kCoherent: other blocks of the same
+// launch write what is gathered (between grid barriers), so the loads are not
+// read-only ones.
+template <int kThreads, bool kCoherent = false, class F>
 __device__ __forceinline__ void for_each_neighbor(const Bufs& B, const DevParams& P, uint32_t i,
                                                   f3 pi, F&& f) {
     const uint32_t cnt = B.nbr_count[i];
     if (cnt <= kNbrCap) {
         for_each_entry<kEntryBatch<kThreads>, kEntryAhead<kThreads>>(
-            B, i, cnt, [&](uint32_t j) { return __ldg(posb(B, j)); },
+            B, i, cnt, [&](uint32_t j) { return kCoherent ? *posb(B, j) : __ldg(posb(B, j)); },
             [&](uint2 v, float4 q) { f(sub(pi, xyz(q)), __uint_as_float(v.y), q); });
     } else {
         const float h = P.h;
         walk(B, P, pi, [&](uint32_t j, f3 rv, float r2) {
             float r = sqrtf(r2);
-            if (r > kEpsR) f(rv, kernel_grad_scale(r, h), __ldg(posb(B, j)));
+            if (r > kEpsR)
+                f(rv, kernel_grad_scale(r, h), kCoherent ? *posb(B, j) : __ldg(posb(B, j)));
         });
     }
 }
@@ -203,7 +206,7 @@ __device__ __forceinline__ void for_each_neighbor(const Bufs& B, const DevParams
 struct Pair {
     float4 pos, data;
 };
-template <int kThreads, class F>
+template <int kThreads, bool kCoherent = false, class F>
 __device__ __forceinline__ void for_each_neighbor_pair(const Bufs& B, const DevParams& P,
                                                        uint32_t i, f3 pi, const float4* recs,
                                                        F&& f) {
@@ -213,7 +216,10 @@ __device__ __forceinline__ void for_each_neighbor_pair(const Bufs& B, const DevP
             B, i, cnt,
             [&](uint32_t j) {
                 Pair p;
-                ld_pair(recs, j, p.pos, p.data);
+                if (kCoherent)
+                    ld_pair_coherent(recs, j, p.pos, p.data);
+                else
+                    ld_pair(recs, j, p.pos, p.data);
                 return p;
             },
             [&](uint2 v, const Pair& p) {
@@ -223,7 +229,8 @@ __device__ __forceinline__ void for_each_neighbor_pair(const Bufs& B, const DevP
         const float h = P.h;
         walk(B, P, pi, [&](uint32_t j, f3 rv, float r2) {
             float r = sqrtf(r2);
-            if (r > kEpsR) f(rv, kernel_grad_scale(r, h), __ldg(recs + 2 * (size_t)j + 1));
+            const float4* data = recs + 2 * (size_t)j + 1;
+            if (r > kEpsR) f(rv, kernel_grad_scale(r, h), kCoherent ? *data : __ldg(data));
         });
     }
 }

@@ -21,6 +21,7 @@
 #include "fe_common.cuh"
 #include "fe_kernels.h"
 #include "fe_neighbors.cuh"
+#include "fe_pressure.cuh"
 
 namespace fe {
 
@@ -130,6 +131,74 @@ __device__ __forceinline__ void sum_warps(const double* sums, const double* maxe
     __syncthreads();
 }
 
+// The metric of an iteration from its sum and largest error (solve_finish_scene).
+__device__ __forceinline__ void finish_metric(const DevParams& P, int which, double sum, double mx,
+                                              double& metric, double& metric_max) {
+    double avg = sum / (double)P.n;
+    if (which == 1) {
+        avg = avg * (double)P.dt;
+        mx = mx * (double)P.dt;
+    }
+    metric = avg / (double)P.rho0;
+    metric_max = mx / (double)P.rho0;
+}
+
+// The fixed-order sum and the largest of the chunks' partials, in every thread
+// of a block of 256.
+__device__ __forceinline__ void sum_chunks(const Bufs& B, double* smem, double& sum, double& mx) {
+    __shared__ double s_result[2];
+    const double a = block_final_sum(B.partials, B.n_chunks, smem);
+    double m = 0.0;
+    for (uint32_t k = threadIdx.x; k < B.n_chunks; k += kBlock)
+        m = fmax(m, __ldcg(B.partials + B.n_chunks + k));
+    m = block_max256(m, smem);
+    if (threadIdx.x == 0) {
+        s_result[0] = a;
+        s_result[1] = m;
+    }
+    __syncthreads();
+    sum = s_result[0];
+    mx = s_result[1];
+    __syncthreads();
+}
+
+// Scene s's control as its solve leaves it, and what k_solve_end records.
+__device__ __forceinline__ void end_scene(const Bufs& B, int which, uint32_t s, uint32_t K,
+                                          uint32_t iter, bool done, bool cap_hit, double metric,
+                                          double metric_max) {
+    SceneState& S = B.S[s];
+    SolveCtl& ctl = S.solve[which];
+    ctl.iter = iter;
+    ctl.K = K;
+    ctl.done = done;
+    ctl.cap_hit = cap_hit;
+    ctl.metric = metric;
+    ctl.metric_max = metric_max;
+    S.last_iters[which] = iter;
+    S.last_metric[which] = metric;
+    S.last_metric_max[which] = metric_max;
+    S.total_iters[which] += iter;
+    if (cap_hit) {
+        S.cap_hits += 1;
+        atomicOr(&B.G->flags, 0x1u);
+    }
+}
+__device__ __forceinline__ void end_solve(const Bufs& B, int which) {
+    B.G->cond[which] = 0;
+    if (which == 1) B.G->src_nonfinite = 0;   // for the next density source
+}
+
+// The last block to leave resets the barrier for the next launch.
+__device__ __forceinline__ void leave(uint32_t* barrier) {
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(barrier + 1, 1u) == gridDim.x - 1) {
+        barrier[0] = 0;
+        barrier[1] = 0;
+    }
+}
+
 }  // namespace
 
 // A solve of a single-scene context: iterations from the current pressures (or
@@ -143,7 +212,7 @@ __device__ __forceinline__ void sum_warps(const double* sums, const double* maxe
 template <int kMaxThreads>
 __global__ void __launch_bounds__(kMaxThreads, 1)
     k_solve_resident(Bufs B, ResidentScratch R, int which, int begun, uint32_t rows) {
-    constexpr int kForceBatch = 16, kUpdateBatch = 8;
+    constexpr int kForceBatch = kMaxThreads <= 256 ? 16 : 8, kUpdateBatch = 8;
     extern __shared__ float4 s_cache[];
     __shared__ double s_sum[16];
     const DevParams& P = B.P[0];
@@ -152,7 +221,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     const bool tolerance = P.solver == 1u;
     const uint32_t K = which == 0 ? S.iters_rho : S.iters_div;
     const uint32_t limit = tolerance ? P.max_it : K, min_it = P.min_it;
-    const double tol = (double)(which == 0 ? P.tol_d : P.tol_v), rho0 = (double)P.rho0;
+    const double tol = (double)(which == 0 ? P.tol_d : P.tol_v);
     const float m = P.mass, dt = P.dt, omega = P.omega;
     uint32_t iter = begun ? ctl.iter : 0u;
     bool done = begun ? ctl.done != 0u : limit == 0u;
@@ -257,13 +326,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         if (tolerance) {
             double sum, mx;
             sum_warps(R.sums, R.maxes, chunks, s_sum, sum, mx);
-            double avg = sum / (double)P.n;
-            if (which == 1) {
-                avg = avg * (double)dt;
-                mx = mx * (double)dt;
-            }
-            metric = avg / rho0;
-            metric_max = mx / rho0;
+            finish_metric(P, which, sum, mx, metric, metric_max);
             if (iter >= min_it && metric <= tol) {
                 done = true;
             } else if (iter >= limit) {
@@ -289,34 +352,88 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         *rec_pos(B, i) = make_float4(p4.x, p4.y, p4.z, pr_before);
         posb(B, i)->w = pressure_over_rho2(p_i, rho_i);
     }
-    // the solve's control and its end (k_solve_end)
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ctl.iter = iter;
-        ctl.K = K;
-        ctl.done = done;
-        ctl.cap_hit = cap_hit;
-        ctl.metric = metric;
-        ctl.metric_max = metric_max;
-        S.last_iters[which] = iter;
-        S.last_metric[which] = metric;
-        S.last_metric_max[which] = metric_max;
-        S.total_iters[which] += iter;
-        B.G->cond[which] = 0;
-        if (which == 1) B.G->src_nonfinite = 0;   // for the next density source
-        if (cap_hit) {
-            S.cap_hits += 1;
-            atomicOr(&B.G->flags, 0x1u);
-        }
+        end_scene(B, which, 0, K, iter, done, cap_hit, metric, metric_max);
+        end_solve(B, which);
     }
-    // the last block to leave resets the barrier for the next launch
+    leave(R.barrier);
+}
+
+// The same for any number of particles: a grid of resident blocks strides over
+// the chunks in each half iteration, with the passes' own list loops, and two
+// grid barriers take the place of two launches and the WHILE node between
+// iterations.  One scene, or several that all iterate a fixed number of times
+// (then begun: k_pressure_first has run for them, without control).
+__global__ void __launch_bounds__(kBlock, kResidentBlocks)
+    k_solve_resident_many(Bufs B, ResidentScratch R, int which, int begun) {
+    __shared__ double smem[8];
+    __shared__ uint32_t s_limit;
+    const bool one = B.n_scenes == 1;
+    const DevParams& P0 = B.P[0];
+    SolveCtl& ctl = B.S[0].solve[which];
+    const bool tolerance = one && P0.solver == 1u;
+    auto wanted = [&](uint32_t s) {
+        if (one && tolerance) return P0.max_it;
+        return which == 0 ? B.S[s].iters_rho : B.S[s].iters_div;
+    };
+    if (threadIdx.x == 0) s_limit = 0;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(R.barrier + 1, 1u) == gridDim.x - 1) {
-            R.barrier[0] = 0;
-            R.barrier[1] = 0;
+    uint32_t most = 0;
+    for (uint32_t s = threadIdx.x; s < B.n_scenes; s += kBlock) most = max(most, wanted(s));
+    atomicMax(&s_limit, most);
+    __syncthreads();
+    const uint32_t limit = s_limit;
+    uint32_t iter = 0;
+    bool done = limit == 0u, cap_hit = false;
+    double metric = 0.0, metric_max = 0.0;
+    if (begun && one) {
+        iter = ctl.iter;
+        done = ctl.done != 0u;
+        cap_hit = ctl.cap_hit != 0u;
+        metric = ctl.metric;
+        metric_max = ctl.metric_max;
+    } else if (begun) {
+        iter = limit != 0u && B.G->src_nonfinite == 0u ? 1u : 0u;
+        done = iter >= limit;
+    }
+    uint32_t barrier = 0;
+    while (!done) {
+        for (uint32_t c = blockIdx.x; c < B.n_chunks; c += gridDim.x) {
+            const uint4 cc = B.chunks[c];
+            if (threadIdx.x < cc.y && (one || iter < wanted(cc.z)))
+                pressure_force_particle<kBlock, true>(B, cc.x + threadIdx.x, cc.z);
+        }
+        if (!grid_barrier(B, R.barrier, ++barrier)) break;
+        for (uint32_t c = blockIdx.x; c < B.n_chunks; c += gridDim.x) {
+            const uint4 cc = B.chunks[c];
+            const uint32_t i = cc.x + threadIdx.x;
+            double e = 0.0;
+            if (threadIdx.x < cc.y && (one || iter < wanted(cc.z)))
+                e = pressure_update_particle(B, B.P[cc.z], i, which,
+                                             pressure_update_sum<kBlock, true>(B, B.P[cc.z], i));
+            if (tolerance) solve_chunk_partials(B, c, e, smem);
+        }
+        if (!grid_barrier(B, R.barrier, ++barrier)) break;
+        ++iter;
+        done = iter >= limit;
+        if (tolerance) {
+            double sum, mx;
+            sum_chunks(B, smem, sum, mx);
+            finish_metric(P0, which, sum, mx, metric, metric_max);
+            if (iter >= P0.min_it && metric <= (double)(which == 0 ? P0.tol_d : P0.tol_v))
+                done = true;
+            else
+                cap_hit = done;
         }
     }
+    if (blockIdx.x == 0) {
+        for (uint32_t s = threadIdx.x; s < B.n_scenes; s += kBlock) {
+            const uint32_t K = which == 0 ? B.S[s].iters_rho : B.S[s].iters_div;
+            end_scene(B, which, s, K, one ? iter : min(iter, K), done, cap_hit, metric, metric_max);
+        }
+        if (threadIdx.x == 0) end_solve(B, which);
+    }
+    leave(R.barrier);
 }
 
 template __global__ void k_solve_resident<256>(Bufs, ResidentScratch, int, int, uint32_t);

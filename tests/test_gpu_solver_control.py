@@ -77,16 +77,16 @@ def test_frame_solve_is_the_solve_pass_by_pass(mode, n, iters, non_finite):
     data.close()
 
 
-@pytest.mark.parametrize("n", [9472, 9473, 18945, 28417])
+@pytest.mark.parametrize("n", [9472, 9473, 18945, 28417, 56832, 56833])
 @pytest.mark.parametrize("cap", [100, 3])
 def test_resident_solve_of_every_block_size(oracle_mod, n, cap):
-    """The solve of few particles as one kernel, around the sizes where its
-    block grows: iterations to a tolerance (the FP64 sums over warps and chunks)
+    """The solve as one kernel, around the sizes where its block grows and where
+    it goes over to striding over chunks: iterations to a tolerance (the FP64 sums over warps and chunks)
     and to a cap, against the oracle."""
     p = scene.dam_break_params((0, 0, 0), (4.0, 4.0, 4.0), mode=_abi.FE_MODE_FIXED,
                                solver=_abi.FE_SOLVER_TOLERANCE)
     p.max_iterations = cap
-    pos, _ = scene.lattice((0, 0, 0), (31, 31, 31), 0.025, 1000.0, 0.05, 0.03, 5)
+    pos, _ = scene.lattice((0, 0, 0), (39, 39, 39), 0.025, 1000.0, 0.05, 0.03, 5)
     pos = pos[:n]
     vel = np.random.default_rng(n).normal(0, 0.3, pos.shape).astype(np.float32)
     sim, orc = Simulation(pos, p, velocities=vel), oracle_mod.Oracle(p, pos, vel)
@@ -101,3 +101,47 @@ def test_resident_solve_of_every_block_size(oracle_mod, n, cap):
         x, y = sim.data.download(f).view(np.uint32), orc.field(f).view(np.uint32)
         assert np.array_equal(x, y), f
     sim.close()
+
+
+@pytest.mark.parametrize("solvers", ["fixed", "mixed"])
+def test_batch_solves_resident_or_iterated(solvers):
+    """Scenes that all iterate a fixed number of times are solved in one kernel,
+    others iteration by iteration; after a change of parameters too.  Either
+    way each as it is alone, one of them with a source that is not finite."""
+    w = scene.batch_workload(n_scenes=5, seed=6, lo=300, hi=900)
+    params = w.params()
+    for k, p in enumerate(params):
+        p.density_solver_iterations, p.divergence_solver_iterations = 2 + k, 5 - k
+    pos = w.positions()
+    batch = BatchSimulation(pos, params)
+    singles = [Simulation(a, q) for a, q in zip(pos, params)]
+    for frame in range(3):
+        if frame == 1 and solvers == "mixed":
+            for s in (1, 3):
+                params[s].solver = _abi.FE_SOLVER_TOLERANCE
+                batch.data.set_scene_params(s, params[s])
+                singles[s].data.sync_with_scene(params[s])
+        if frame == 2:
+            v = batch.data.download(_abi.FE_FIELD_VELOCITY_B)
+            first, n = int(batch.data.scene_first[2]), int(batch.data.scene_count[2])
+            v[first + n // 2, 1] = np.inf
+            batch.data.upload(_abi.FE_FIELD_VELOCITY_B, v)
+            singles[2].data.upload(_abi.FE_FIELD_VELOCITY_B, v[first:first + n])
+        batch.step(1, want_stats=False)
+        for sim in singles:
+            sim.step(1, want_stats=False)
+        for s, sim in enumerate(singles):
+            for f in FIELDS:
+                a, b = batch.data.scene(batch.data.download(f), s), sim.data.download(f)
+                assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (frame, s, f)
+            a, b = None, None
+            try:
+                a, b = batch.data.read_scene_stats(s), sim.data.read_stats()
+            except _abi.FluidStepError:
+                pass
+            if a and b:
+                assert (a.density_iterations, a.divergence_iterations) == (
+                    b.density_iterations, b.divergence_iterations), (frame, s)
+    batch.close()
+    for sim in singles:
+        sim.close()
