@@ -395,7 +395,10 @@ struct fe_ctx {
     StatsSnapshot* stats_dev = nullptr;      // the same memory as the device sees it
     cudaEvent_t stats_done[2] = {nullptr, nullptr};
     uint64_t stats_tickets = 0;
-    cudaEvent_t copy_done[2] = {nullptr, nullptr};
+    // ticket t's copy: event t % kTicketEvents, so that a wait for a ticket does
+    // not wait for the copies after it (until as many have followed)
+    static constexpr int kTicketEvents = 16;
+    cudaEvent_t copy_done[kTicketEvents] = {};
     uint64_t tickets = 0;
     uint64_t slot_ticket[2] = {0, 0};
 
@@ -465,9 +468,10 @@ void release(fe_ctx* c) {
     }
     for (int k = 0; k < 2; ++k) {
         if (c->snap_ready[k]) cudaEventDestroy(c->snap_ready[k]);
-        if (c->copy_done[k]) cudaEventDestroy(c->copy_done[k]);
         if (c->stats_done[k]) cudaEventDestroy(c->stats_done[k]);
     }
+    for (cudaEvent_t e : c->copy_done)
+        if (e) cudaEventDestroy(e);
     if (c->stats_host) cudaFreeHost(c->stats_host);
     if (c->stream) cudaStreamDestroy(c->stream);
 }
@@ -1596,10 +1600,10 @@ fe_status fe_download_async(fe_ctx* c, fe_field f, void* dst, size_t bytes, uint
     FE_CUDA(cudaSetDevice(c->device));
     if (!c->copy_stream) {
         FE_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < 2; ++k)
             FE_CUDA(cudaEventCreateWithFlags(&c->snap_ready[k], cudaEventDisableTiming));
-            FE_CUDA(cudaEventCreateWithFlags(&c->copy_done[k], cudaEventDisableTiming));
-        }
+        for (cudaEvent_t& e : c->copy_done)
+            FE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     if (need > c->snap_cap) {
         // earlier snapshots may still be copied out of the old buffers
@@ -1617,7 +1621,8 @@ fe_status fe_download_async(fe_ctx* c, fe_field f, void* dst, size_t bytes, uint
     const int slot = (int)(t & 1u);
     // the slot's previous copy must have left the snapshot before it is
     // overwritten
-    if (c->slot_ticket[slot]) FE_CUDA(cudaStreamWaitEvent(c->stream, c->copy_done[slot], 0));
+    if (const uint64_t before = c->slot_ticket[slot])
+        FE_CUDA(cudaStreamWaitEvent(c->stream, c->copy_done[before % fe_ctx::kTicketEvents], 0));
     float w = 0.0f;
     const bool fix_w = field_fixed_w(f, &w);
     if (elem == 16) {
@@ -1632,7 +1637,7 @@ fe_status fe_download_async(fe_ctx* c, fe_field f, void* dst, size_t bytes, uint
     FE_CUDA(cudaEventRecord(c->snap_ready[slot], c->stream));
     FE_CUDA(cudaStreamWaitEvent(c->copy_stream, c->snap_ready[slot], 0));
     FE_CUDA(cudaMemcpyAsync(dst, c->snap[slot], need, cudaMemcpyDeviceToHost, c->copy_stream));
-    FE_CUDA(cudaEventRecord(c->copy_done[slot], c->copy_stream));
+    FE_CUDA(cudaEventRecord(c->copy_done[t % fe_ctx::kTicketEvents], c->copy_stream));
     c->slot_ticket[slot] = t;
     *ticket = t;
     return FE_OK;
@@ -1644,10 +1649,9 @@ fe_status fe_download_wait(fe_ctx* c, uint64_t ticket) {
         return FE_ERR_INVALID_ARGUMENT;
     }
     FE_CUDA(cudaSetDevice(c->device));
-    // A slot serves tickets in increasing order, and each copy out of a slot
-    // follows the one before it: waiting for the slot's latest copy covers
-    // this ticket as well.
-    FE_CUDA(cudaEventSynchronize(c->copy_done[ticket & 1u]));
+    // The copies run in ticket order, so an event that has gone on to a later
+    // ticket covers this one as well.
+    FE_CUDA(cudaEventSynchronize(c->copy_done[ticket % fe_ctx::kTicketEvents]));
     return FE_OK;
 }
 
