@@ -219,9 +219,11 @@ __global__ void __launch_bounds__(kThreads, pass_min_blocks<kBits, kItems>()) k_
             // Look back kLook predecessors per step: their status words are
             // loaded together, then consumed nearest first until an
             // inclusive prefix is found; an unpublished one (flag 0) is
-            // re-polled from there.  Each step costs one memory latency
-            // instead of kLook.
-            constexpr int kLook = 8;
+            // re-polled from there.  Two: most words polled are not there
+            // yet, and the polls of a wave of tiles get in one another's way
+            // (4M pairs: 1 / 2 / 4 / 8 / 16 / 32 per step 224 / 226 / 230 /
+            // 243 / 257 / 300 us; 1M 101 / 97 / 97 / 97 / 113 / 133).
+            constexpr int kLook = 2;
             int pred = (int)tile - 1;
             int spins = 0;
             bool done = false;
