@@ -101,10 +101,24 @@ struct Recorder {
     cudaGraph_t graph = nullptr;  // null: eager
     cudaGraph_t root = nullptr;   // graph owning conditional handles
     cudaGraphNode_t last = nullptr;
+    bool early = false;           // eager: kernels begin with stage_begin()
 
     // cooperative: all blocks resident at once (the kernel has grid barriers)
     cudaError_t launch(const void* func, dim3 grid, dim3 block, size_t smem, void** args,
                        bool cooperative = false) {
+        if (!graph && early && !cooperative) {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = grid;
+            cfg.blockDim = block;
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = stream;
+            cudaLaunchAttribute attr{};
+            attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr.val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+            return cudaLaunchKernelExC(&cfg, func, args);
+        }
         if (!graph)
             return cooperative ? cudaLaunchCooperativeKernel(func, grid, block, args, smem, stream)
                                : cudaLaunchKernel(func, grid, block, args, smem, stream);
@@ -1655,12 +1669,19 @@ fe_status fe_download_wait(fe_ctx* c, uint64_t ticket) {
     return FE_OK;
 }
 
+// Stage calls of so few particles (a 64-thread block per SM) launch early: their
+// kernels' blocks fit beside the running ones.  Ten harness substeps of 1.4k
+// particles 2300 -> 1861 us, 4.8k 2754 -> 2529; 16k 2949 / 3001, as the waiting
+// blocks then take places.
+constexpr uint32_t kEarlyParticles = 148 * 64;
+
 #define FE_STAGE(name, body)                                 \
     fe_status name(fe_ctx* c) {                              \
         NvtxRange range_(#name);                             \
         fe_status s_ = need_prepared(c, #name);              \
         if (s_ != FE_OK) return s_;                          \
         Recorder R = eager(c);                               \
+        R.early = c->n <= kEarlyParticles;                   \
         body;                                                \
     }
 

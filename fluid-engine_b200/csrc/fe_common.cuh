@@ -117,6 +117,15 @@ __device__ __forceinline__ float pressure_over_rho2(float p, float rho) {
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
+// The start of a kernel of the stage calls.  With few particles the calls'
+// launches allow the next kernel's blocks to take their places while this one
+// runs (programmatic dependent launch): they then wait here until everything
+// before them is done and written.  Launched in the ordinary way it is no wait.
+__device__ __forceinline__ void stage_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // position_b and pressure acceleration of particle i (see Bufs).
 __device__ __forceinline__ float4* posb(const Bufs& B, uint32_t i) { return B.pos_b + i; }
 __device__ __forceinline__ float4* rec_pos(const Bufs& B, uint32_t i) {

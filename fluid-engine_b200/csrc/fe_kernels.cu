@@ -34,6 +34,7 @@ __global__ void k_fill_u32(uint32_t* p, uint32_t v, size_t count) {
 }
 
 __global__ void k_fill_cells(uint2* p, size_t count) {
+    stage_begin();
     size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride)
         p[i] = make_uint2(kEmpty, kEmpty);
@@ -42,6 +43,7 @@ __global__ void k_fill_cells(uint2* p, size_t count) {
 // spatial_hash.comp:23-36 (the sentinel tail is written once at creation and
 // never changes).
 __global__ void __launch_bounds__(kBlock) k_hash(Bufs B) {
+    stage_begin();
     uint32_t i, s, c;
     if (!chunk_of(B, i, s, c)) return;
     const DevParams& P = B.P[s];
@@ -55,6 +57,7 @@ __global__ void __launch_bounds__(kBlock) k_hash(Bufs B) {
 // grid_offsets.comp:20-33, also recording where each bucket ends so that the
 // walk needs no hash comparison.
 __global__ void k_offsets(Bufs B) {
+    stage_begin();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= B.n_total) return;
     uint32_t key = B.keys[i];
@@ -106,10 +109,12 @@ __device__ __forceinline__ void reorder_body(const Bufs& B, int carry_pressure,
 }
 
 __global__ void __launch_bounds__(kBlock) k_reorder(Bufs B, int carry_pressure) {
+    stage_begin();
     reorder_body<false>(B, carry_pressure, LearnArgs{});
 }
 __global__ void __launch_bounds__(kBlock) k_reorder_carry(Bufs B, int carry_pressure,
                                                           LearnArgs L) {
+    stage_begin();
     reorder_body<true>(B, carry_pressure, L);
 }
 
@@ -155,6 +160,7 @@ __device__ __forceinline__ void cell_count(const CellSort& C, uint32_t i, uint32
 }
 
 __global__ void __launch_bounds__(kBlock) k_cell_count(Bufs B, CellSort C) {
+    stage_begin();
     uint32_t i, s, c;
     const bool live = chunk_of(B, i, s, c);
     const DevParams& P = B.P[s];
@@ -170,6 +176,7 @@ constexpr unsigned long long kScanSum = 1ull << 32, kScanPrefix = 2ull << 32;
 // A thread owns 8 slots, 32 bytes of counters and 64 of bounds, so every access
 // is to whole sectors (16 slots a thread: 15.7 us at 2^20 slots; 8: 9 us).
 __global__ void __launch_bounds__(kScanThreads) k_cell_scan(Bufs B, CellSort C) {
+    stage_begin();
     constexpr int kWarps = kScanThreads / 32;
     __shared__ uint32_t s_warp[kWarps], s_base;
     __shared__ unsigned long long s_ticket;
@@ -284,6 +291,7 @@ __global__ void __launch_bounds__(kScanThreads) k_cell_scan(Bufs B, CellSort C) 
 }
 
 __global__ void __launch_bounds__(kBlock) k_cell_scatter(Bufs B, CellSort C) {
+    stage_begin();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= B.n_total) return;
     const uint32_t at = B.cells[C.key[i]].x + C.place[i];
@@ -309,11 +317,13 @@ __device__ __forceinline__ void cell_reorder(const Bufs& B, const CellSort& C, i
     reorder_slot<kCarry>(B, carry_pressure, L, i, src);
 }
 __global__ void __launch_bounds__(kBlock) k_cell_reorder(Bufs B, CellSort C, int carry_pressure) {
+    stage_begin();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < B.n_total) cell_reorder<false>(B, C, carry_pressure, LearnArgs{}, t);
 }
 __global__ void __launch_bounds__(kBlock) k_cell_reorder_carry(Bufs B, CellSort C,
                                                                int carry_pressure, LearnArgs L) {
+    stage_begin();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < B.n_total) cell_reorder<true>(B, C, carry_pressure, L, t);
 }
@@ -334,9 +344,11 @@ __device__ __forceinline__ void take_pressure_body(const Bufs& B, const LearnArg
 }
 
 __global__ void __launch_bounds__(kBlock) k_take_pressure(Bufs B) {
+    stage_begin();
     take_pressure_body<false>(B, LearnArgs{});
 }
 __global__ void __launch_bounds__(kBlock) k_take_pressure_carry(Bufs B, LearnArgs L) {
+    stage_begin();
     take_pressure_body<true>(B, L);
 }
 
@@ -813,6 +825,7 @@ __device__ __forceinline__ void density_particle(const Bufs& B, F&& f) {
 
 template <int kLanes>
 __global__ void __launch_bounds__(kDensityThreads, kDensityBlocks) k_density_alpha(Bufs B) {
+    stage_begin();
     __shared__ DensityScratch scratch[kDensityThreads / 32];
     DensityScratch& S = scratch[threadIdx.x >> 5];
     density_particle<kLanes>(B, [&](uint32_t i, uint32_t s, bool live) {
@@ -882,6 +895,7 @@ __device__ __forceinline__ void viscosity_particle(const Bufs& B, uint32_t i, ui
 
 template <int kThreads, bool kPersist>
 __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>) k_viscosity(Bufs B) {
+    stage_begin();
     for_each_particle<kThreads, kPersist>(B, [&](uint32_t i, uint32_t s, bool live) {
         if (live) viscosity_particle<kThreads>(B, i, s);
     });
@@ -925,6 +939,7 @@ __device__ __forceinline__ void density_source_body(const Bufs& B, const LearnAr
 
 template <int kThreads, bool kPersist>
 __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>) k_density_source(Bufs B) {
+    stage_begin();
     for_each_particle<kThreads, kPersist>(B, [&](uint32_t i, uint32_t s, bool live) {
         if (live) density_source_body<kThreads, false>(B, LearnArgs{}, i, s);
     });
@@ -964,6 +979,7 @@ __device__ __forceinline__ void divergence_source_body(const Bufs& B, int fixed,
 template <int kThreads, bool kPersist>
 __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>) k_divergence_source(Bufs B,
                                                                                       int fixed) {
+    stage_begin();
     for_each_particle<kThreads, kPersist>(B, [&](uint32_t i, uint32_t s, bool live) {
         if (live) divergence_source_body<kThreads>(B, fixed, i, s);
     });
@@ -976,6 +992,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>) k_divergence_s
 template <int kThreads, bool kPersist>
 __global__ void __launch_bounds__(kThreads, kMinBlocks<kThreads>) k_pressure_force(Bufs B,
                                                                                    int which) {
+    stage_begin();
     for_each_particle<kThreads, kPersist>(B, [&](uint32_t i, uint32_t s, bool live) {
         if (live && !(which >= 0 && B.S[s].solve[which].done))
             pressure_force_particle<kThreads>(B, i, s);
@@ -1084,6 +1101,7 @@ __global__ void __launch_bounds__(kBlock) k_solve_finish(Bufs B, int which,
 // The stage call for few particles: no control, so no chunk partials.
 __global__ void __launch_bounds__(kFewThreads, kMinBlocks<kFewThreads>)
     k_pressure_update_few(Bufs B) {
+    stage_begin();
     for_each_particle<kFewThreads, false>(B, [&](uint32_t i, uint32_t s, bool live) {
         if (!live) return;
         const DevParams& P = B.P[s];
@@ -1278,6 +1296,7 @@ __device__ __forceinline__ void pressure_integration_body(const Bufs& B, const L
 }
 
 __global__ void __launch_bounds__(kBlock) k_pressure_integration(Bufs B) {
+    stage_begin();
     pressure_integration_body<false>(B, LearnArgs{});
 }
 // + the density solve's after-solve bookkeeping of the learned warm start
@@ -1300,6 +1319,7 @@ __device__ __forceinline__ void divergence_integration_body(const Bufs& B, int f
 }
 
 __global__ void __launch_bounds__(kBlock) k_divergence_integration(Bufs B, int fixed) {
+    stage_begin();
     divergence_integration_body<false>(B, fixed, LearnArgs{});
 }
 __global__ void __launch_bounds__(kBlock) k_divergence_integration_learn(Bufs B, int fixed,
@@ -1423,6 +1443,7 @@ __device__ __forceinline__ void stats_chunk(Bufs B, uint4* upart, bool valid, ui
 }
 
 __global__ void __launch_bounds__(kBlock) k_stats(Bufs B, int fixed, uint4* upart) {
+    stage_begin();
     uint32_t i, s, c;
     const bool valid = chunk_of(B, i, s, c);
     const float4* vel = fixed ? velb(B, 0) : vela(B, 0);

@@ -24,6 +24,7 @@ namespace fe {
 // carry_tmp); FIXED mode does this inside k_take_pressure_carry, and after a
 // substep's re-sort k_density_alpha_div_learn does it.
 __global__ void __launch_bounds__(kBlock) k_carry_take(Bufs B, LearnArgs L) {
+    stage_begin();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= B.n_total) return;
     L.carry[i] = L.carry_tmp[i];

@@ -25,6 +25,7 @@
 
 #include <cstdint>
 
+#include "fe_common.cuh"
 #include "fe_sort.h"
 
 namespace fe {
@@ -431,6 +432,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
 // (bitonic_sort.comp:19-43).
 __global__ void k_bitonic_global(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t h,
                                  uint32_t step) {
+    stage_begin();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n / 2) return;
     uint32_t left = (i / step) * step * 2 + (i % step);
@@ -462,6 +464,7 @@ template <int kBlocks>
 __global__ void __cluster_dims__(kBlocks, 1, 1) __launch_bounds__(kBitonicTile / 2)
     k_bitonic_local(uint32_t* keys, uint32_t* vals, uint32_t tile, uint32_t h_lo, uint32_t h_hi) {
     __shared__ uint2 s[kBitonicTile];
+    stage_begin();
     const uint32_t base = blockIdx.x * tile, i = threadIdx.x, half = tile / 2;
     const bool on = i < half;   // (a tile of 2 to 32 entries has idle lanes)
     if (on) {
