@@ -511,10 +511,7 @@ auto pick(void (*k128)(KArgs...), void (*k256)(KArgs...), void (*k512)(KArgs...)
 // 7.9/7.0, 8.6/8.3; 25k 10.6/9.7, 8.1/7.4, 8.9/9.0; 50k 13.4/12.2, 9.3/8.8,
 // 11.4/11.2 with whole frames slower (347/390); 80k 15.4/19.1, 10.3/12.6,
 // 14.5/17.0.
-#ifndef FE_FEW_PARTICLES
-#define FE_FEW_PARTICLES (148 * 128)
-#endif
-constexpr uint32_t kFewParticles = FE_FEW_PARTICLES;
+constexpr uint32_t kFewParticles = 148 * 128;
 bool few(const fe_ctx* c) { return c->n <= kFewParticles; }
 #define NBR_KERNEL(name, g)               \
     (few(c) ? name<kFewThreads, false>    \
@@ -585,14 +582,12 @@ fe_status rec_nbr(fe_ctx* c, Recorder& R, int g, void (*func)(KArgs...), Args...
 // again, else 32.  Times in a graph of launches (us, 8 / 16 / 32 per warp, a
 // fall after 40 frames): 4.8k particles 28/43/58, 25k 43/60/65, 50k 72/63/68,
 // 80k 99/78/70, 131k 152/112/80.
-#ifndef FE_LANES8
-#define FE_LANES8 (148 * 32 * 8)
-#define FE_LANES16 (148 * 32 * 12)
-#endif
+constexpr uint32_t kLanes8Particles = 148 * 32 * 8;
+constexpr uint32_t kLanes16Particles = 148 * 32 * 12;
 template <class... KArgs, class... Args>
 fe_status rec_density(fe_ctx* c, Recorder& R, void (*k8)(KArgs...), void (*k16)(KArgs...),
                       void (*k32)(KArgs...), Args... args) {
-    const uint32_t lanes = c->n <= FE_LANES8 ? 8u : c->n <= FE_LANES16 ? 16u : 32u;
+    const uint32_t lanes = c->n <= kLanes8Particles ? 8u : c->n <= kLanes16Particles ? 16u : 32u;
     const uint32_t blocks = c->B.n_chunks * (kBlock / lanes) / (kFewThreads / 32);
     REC(R.k(lanes == 8 ? k8 : lanes == 16 ? k16 : k32, dim3(blocks), dim3(kFewThreads), args...));
     return FE_OK;
@@ -767,23 +762,19 @@ fe_status rec_solve_resident_many(fe_ctx* c, Recorder& R, int which) {
 // as many list entries in shared memory as fit (all 64 up to 192 threads).
 // The line: 16k particles' frame of 4 + 4 iterations 272 -> 156 us, 25k 301 ->
 // 171, 50k (37 entries fit) 325 -> 251; with 512 threads 27 entries fit.
-#ifndef FE_RESIDENT_MAX
-#define FE_RESIDENT_MAX (148 * kResidentMaxThreads)
-#endif
-#ifndef FE_RESIDENT_MANY_MAX
-#define FE_RESIDENT_MANY_MAX (1u << 20)
-#endif
+constexpr uint32_t kResidentParticles = 148 * kResidentMaxThreads;
+constexpr uint32_t kResidentManyParticles = 1u << 20;
 fe_status choose_resident(fe_ctx* c) {
     int smem_max = 0, cooperative = 0, blocks = 0;
     FE_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
     FE_CUDA(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, c->device));
-    if (cooperative && c->n <= FE_RESIDENT_MANY_MAX) {
+    if (cooperative && c->n <= kResidentManyParticles) {
         FE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_solve_resident_many,
                                                               kBlock, 0));
         c->resident_many_blocks =
             std::min<uint32_t>(c->B.n_chunks, (uint32_t)(blocks * c->num_sms));
     }
-    if (c->B.n_scenes != 1 || c->n > FE_RESIDENT_MAX) return FE_OK;
+    if (c->B.n_scenes != 1 || c->n > kResidentParticles) return FE_OK;
     uint32_t threads = 64;
     while ((c->n + threads - 1) / threads > (uint32_t)c->num_sms) threads += 64;
     if (!cooperative || threads > (uint32_t)kResidentMaxThreads) return FE_OK;

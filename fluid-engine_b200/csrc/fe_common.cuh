@@ -121,6 +121,9 @@ __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 // launches allow the next kernel's blocks to take their places while this one
 // runs (programmatic dependent launch): they then wait here until everything
 // before them is done and written.  Launched in the ordinary way it is no wait.
+// Every kernel that a stage call can launch begins with it: one that did not
+// would run beside the kernel before it.  Loads of what that kernel wrote come
+// after a plain load or a bounds test, so that none can be moved above the wait.
 __device__ __forceinline__ void stage_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -1485,6 +1485,7 @@ __global__ void __launch_bounds__(kBlock) k_divergence_integration_stats_learn(B
 }
 
 __global__ void __launch_bounds__(kBlock) k_stats_finish(Bufs B, uint4* upart) {
+    stage_begin();
     __shared__ double smem[8];
     __shared__ uint32_t s_u[3][8];
     const uint32_t sc = blockIdx.x;

@@ -1,4 +1,6 @@
-// fe_sort.cu — key/value sorts for the neighbour search.
+// fe_sort.cu — key/value sorts: fe_sort_pairs, and the entry order of a context
+// whose params ask for the bitonic network (the radix choice is a counting sort
+// over the hash table there: k_cell_count and what follows it).
 //
 // Radix: stable LSD radix sort with b-bit digits (b = 8 or 10),
 // ceil(key_bits / b) passes.  The reference runs count -> single-workgroup
@@ -19,8 +21,8 @@
 //
 // Bitonic: the compare-exchange network of bitonic_sort.comp driven by the
 // (h, step) loops of GpuSorter::execute (sorter.rs:73-115).  Stages whose
-// pairs lie inside a 2048-entry tile, or a cluster of 8, run in shared memory, several per
-// launch; the network and therefore the result are unchanged.
+// pairs lie inside a 2048-entry tile, or a cluster of 8, run in shared memory,
+// several per launch; the network and therefore the result are unchanged.
 #include <cuda_runtime.h>
 
 #include <cstdint>

@@ -1,10 +1,12 @@
 """The shapes of the neighbour passes: every one gives the same bits."""
+import ctypes
+
 import numpy as np
 import pytest
 
 from fluid_step import _abi, scene
-from fluid_step.pipelines import (CommandBufferBuilder, ComputePipelines, GpuPhysicsData,
-                                  Simulation)
+from fluid_step.pipelines import (BatchSimulation, CommandBufferBuilder, ComputePipelines,
+                                  GpuPhysicsData, Simulation)
 
 pytestmark = pytest.mark.gpu
 
@@ -63,3 +65,38 @@ def test_tuned_shapes_above_the_line():
         _same(sim.data.download, ref.data.download, (threads, persistent))
         sim.close()
     ref.close()
+
+
+@pytest.mark.parametrize("scenes", [2, 7])
+def test_stage_calls_of_a_small_batch(scenes):
+    """Every stage call of a batch of few particles, its per-scene statistics
+    included, against one context per scene."""
+    pos, par = [], []
+    for k in range(scenes):
+        p, x = _scene(300 + 97 * k, _abi.FE_MODE_FIXED)
+        pos.append(x)
+        par.append(p)
+    batch = BatchSimulation(pos, par)
+    singles = [Simulation(x, p) for x, p in zip(pos, par)]
+    names = ["neighbor_search", "density_alpha", "viscosity", "density_source",
+             "pressure_force", "pressure_update", "pressure_integration", "neighbor_search",
+             "density_alpha", "divergence_source", "pressure_force", "pressure_update",
+             "divergence_integration", "stats_pass"]
+    for sim in [batch] + singles:
+        lib, h = sim.data._lib, sim.data.handle
+        for _ in range(4):
+            for name in names:
+                _abi.check(lib, getattr(lib, "fe_" + name)(h), name)
+    lib = batch.data._lib
+    for k, sim in enumerate(singles):
+        a, b = _abi.FeStats(), _abi.FeStats()
+        _abi.check(lib, lib.fe_read_scene_stats(batch.data.handle, k, ctypes.byref(a)), "stats")
+        _abi.check(lib, lib.fe_read_stats(sim.data.handle, ctypes.byref(b)), "stats")
+        assert bytes(a) == bytes(b), k
+    x = batch.data.download(_abi.FE_FIELD_POSITION_A).view(np.uint32)
+    y = np.concatenate([s.data.download(_abi.FE_FIELD_POSITION_A).view(np.uint32)
+                        for s in singles])
+    assert np.array_equal(x, y)
+    batch.close()
+    for sim in singles:
+        sim.close()
