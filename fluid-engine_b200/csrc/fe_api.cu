@@ -358,7 +358,7 @@ struct fe_ctx {
     CellSort cell_sort{};
     // resident solve: its scratch and launch shape (threads 0: not used)
     ResidentScratch resident{};
-    uint32_t resident_threads = 0, resident_rows = 0;
+    bool resident_single = false;  // solves by k_solve_resident
     uint32_t resident_many_blocks = 0;   // of k_solve_resident_many
     uint4* upart = nullptr;
     uint32_t key_bits = 32;
@@ -714,9 +714,8 @@ fe_status rec_solve_begin(fe_ctx* c, Recorder& R, int which, cudaGraphConditiona
     return FE_OK;
 }
 
-auto resident_kernel(uint32_t threads) {
-    return threads <= 256 ? k_solve_resident<256> : k_solve_resident<kResidentMaxThreads>;
-}
+// All 64 list entries of a block's particles (three contexts' blocks an SM).
+constexpr size_t kResidentSmem = (size_t)kNbrCap * kResidentThreads * sizeof(float4);
 
 // A solve in one resident launch, its begin and end included (of the density
 // solve from the plain start, all but the first iteration).
@@ -727,11 +726,9 @@ fe_status rec_solve_resident(fe_ctx* c, Recorder& R, int which) {
                 0));
         begun = 1;
     }
-    const uint32_t threads = c->resident_threads;
-    const size_t smem = (size_t)c->resident_rows * threads * sizeof(float4);
-    void* args[] = {&c->B, &c->resident, &which, &begun, &c->resident_rows};
-    REC(R.launch((const void*)resident_kernel(threads), dim3((c->n + threads - 1) / threads), dim3(threads),
-                 smem, args, true));
+    void* args[] = {&c->B, &c->resident, &which, &begun};
+    REC(R.launch((const void*)k_solve_resident, dim3((c->n + kResidentThreads - 1) / kResidentThreads),
+                 dim3(kResidentThreads), kResidentSmem, args, true));
     return FE_OK;
 }
 
@@ -758,36 +755,45 @@ fe_status rec_solve_resident_many(fe_ctx* c, Recorder& R, int which) {
     return FE_OK;
 }
 
-// The shape of the resident solve: one particle per thread, a block per SM,
-// as many list entries in shared memory as fit (all 64 up to 192 threads).
-// The line: 16k particles' frame of 4 + 4 iterations 272 -> 156 us, 25k 301 ->
-// 171, 50k (37 entries fit) 325 -> 251; with 512 threads 27 entries fit.
-constexpr uint32_t kResidentParticles = 148 * kResidentMaxThreads;
-constexpr uint32_t kResidentManyParticles = 1u << 20;
+// Which solves run resident.  A cooperative launch waits until all its blocks
+// find a place: alone it saves the iterations' launches and the WHILE node, but
+// beside other contexts' frames it waits and leaves places idle.  Microseconds
+// per frame of 4 + 4 iterations, one context / two / four / sixteen on streams
+// of their own:
+//             a particle per thread   strided chunks      iterated (WHILE)
+//   4.1k      133 /  70 /  37 /  18   195/ 98/ 51/ 17     232/125/ 67/ 35
+//   16k       152 /  88 /  69 /  66   207/111/ 70/ 48     262/145/ 85/ 64
+//   32k       179 / 142 / 135 / 135   218/140/103/ 96     282/168/115/ 92
+//   50k       220 / 179 / 176 / 178   240/161/134/134     300/192/132/117
+//   65k                               243/176/170/171     301/207/149/139
+//   131k                              355/338/353/360     410/311/279/290
+//   262k                              681/695/711/719     770/575/576/604
+// Contexts of mixed sizes at once, 16 of 4k to 60k particles (ms per frame of
+// all) and 64 of 4k to 262k: a particle per thread up to 18.9k particles, chunks
+// up to 56.8k 1.25 and 13.6; up to 9.5k and 37.9k, as here, 0.97 and 10.3;
+// iterated throughout - and 10.1.
+// Several scenes in one context, which are what one has instead of several
+// contexts: 256 scenes of 1k to 8k particles 3.2 -> 1.9 ms.
+constexpr uint32_t kResidentParticles = 148 * kResidentThreads;   // a block per SM
+constexpr uint32_t kStridedParticles = 148 * kBlock;              // a chunk per SM
+constexpr uint32_t kStridedBatchParticles = 1u << 20;
 fe_status choose_resident(fe_ctx* c) {
-    int smem_max = 0, cooperative = 0, blocks = 0;
-    FE_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+    int cooperative = 0, blocks = 0;
     FE_CUDA(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, c->device));
-    if (cooperative && c->n <= kResidentManyParticles) {
+    if (!cooperative) return FE_OK;
+    if (c->n <= (c->B.n_scenes == 1 ? kStridedParticles : kStridedBatchParticles)) {
         FE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_solve_resident_many,
                                                               kBlock, 0));
         c->resident_many_blocks =
             std::min<uint32_t>(c->B.n_chunks, (uint32_t)(blocks * c->num_sms));
     }
     if (c->B.n_scenes != 1 || c->n > kResidentParticles) return FE_OK;
-    uint32_t threads = 64;
-    while ((c->n + threads - 1) / threads > (uint32_t)c->num_sms) threads += 64;
-    if (!cooperative || threads > (uint32_t)kResidentMaxThreads) return FE_OK;
-    const uint32_t fit = ((uint32_t)smem_max - 1024u) / (threads * (uint32_t)sizeof(float4));
-    const uint32_t rows = std::min(fit, kNbrCap);
-    const size_t smem = (size_t)rows * threads * sizeof(float4);
-    const auto kernel = resident_kernel(threads);
-    FE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 smem_max - 1024));
-    FE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, (int)threads, smem));
-    if (blocks < 1) return FE_OK;
-    c->resident_threads = threads;
-    c->resident_rows = rows;
+    FE_CUDA(cudaFuncSetAttribute(k_solve_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kResidentSmem));
+    FE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_solve_resident,
+                                                          kResidentThreads, kResidentSmem));
+    c->resident_single =
+        (c->n + kResidentThreads - 1) / kResidentThreads <= (uint32_t)(blocks * c->num_sms);
     return FE_OK;
 }
 
@@ -795,7 +801,7 @@ fe_status choose_resident(fe_ctx* c) {
 // finish when the context holds several scenes, guard}, end kernel.  Eager:
 // the same kernels with a host loop on the device flag.
 fe_status rec_solve(fe_ctx* c, Recorder& R, int which) {
-    if (c->resident_threads) return rec_solve_resident(c, R, which);
+    if (c->resident_single) return rec_solve_resident(c, R, which);
     if (resident_many(c)) return rec_solve_resident_many(c, R, which);
     Bufs B = c->B;
     fe_status st;
@@ -1301,7 +1307,7 @@ fe_status create_ctx(const fe_params* params, const uint32_t* counts, uint32_t n
         return fail(s);
     ResidentScratch& rs = c->resident;
     if ((s = dev_alloc(c, &rs.barrier, 2))) return fail(s);
-    if (c->resident_threads) {
+    if (c->resident_single) {
         if ((s = dev_alloc(c, &rs.pr, n)) || (s = dev_alloc(c, &rs.sums, 16 * (size_t)nchunks)))
             return fail(s);
         rs.maxes = rs.sums + 8 * (size_t)nchunks;

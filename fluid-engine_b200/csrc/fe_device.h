@@ -131,7 +131,7 @@ struct CellSort {
 };
 
 // Scratch of the resident solve (k_solve_resident).
-constexpr int kResidentMaxThreads = 384;
+constexpr int kResidentThreads = 64;
 constexpr int kResidentBlocks = 4;   // per SM, of k_solve_resident_many
 struct ResidentScratch {
     float* pr;               // p / rho^2 per particle

@@ -56,8 +56,7 @@ __global__ void k_pressure_first(Bufs B, cudaGraphConditionalHandle handle, int 
 __global__ void k_solve_end(Bufs B, int which);
 // A whole solve of few particles in one cooperative launch (fe_resident.cu).
 __global__ void k_solve_resident_many(Bufs B, ResidentScratch R, int which, int begun);
-template <int kMaxThreads>
-__global__ void k_solve_resident(Bufs B, ResidentScratch R, int which, int begun, uint32_t rows);
+__global__ void k_solve_resident(Bufs B, ResidentScratch R, int which, int begun);
 __global__ void k_loop_guard(Bufs B, int which, cudaGraphConditionalHandle handle);
 __global__ void k_pressure_integration(Bufs B);
 __global__ void k_pressure_integration_learn(Bufs B, LearnArgs L);

@@ -5,8 +5,7 @@
 // rest the chain parameters -> count -> list words -> neighbours, and the graph's
 // WHILE node adds 7 us between iterations (16k particles: 24 us an iteration,
 // here 8.6).
-// Here every particle keeps a thread, and every SM a block, for all the
-// iterations.  The pair gradients, which do not change during a solve, stay in
+// Here every particle keeps a thread for all the iterations.  The pair gradients, which do not change during a solve, stay in
 // shared memory with the neighbours' indices, so an iteration is two gathers
 // (4 bytes of p / rho^2, 16 of acceleration), all of a thread's loads in flight
 // together, and two grid-wide barriers.
@@ -57,8 +56,8 @@ __device__ __forceinline__ bool grid_barrier(const Bufs& B, uint32_t* count, uin
 }
 
 struct Particle {
-    const float4* cache;   // [rows][blockDim.x]: gradient, neighbour index
-    uint32_t i, cnt, rows;
+    const float4* cache;   // [cnt][kResidentThreads]: gradient, neighbour index
+    uint32_t i, cnt;
     f3 pi;
 };
 
@@ -75,22 +74,18 @@ __device__ __forceinline__ void for_each_cached(const Bufs& B, const DevParams& 
         });
         return;
     }
-    for (uint32_t k = 0; k < q.rows; k += kBatch) {
+    for (uint32_t k = 0; k < q.cnt; k += kBatch) {
         float4 e[kBatch];
         decltype(load(0u)) d[kBatch];
 #pragma unroll
         for (int t = 0; t < kBatch; ++t)
-            if (k + t < q.rows) {
-                e[t] = q.cache[(k + t) * blockDim.x];
+            if (k + t < q.cnt) {
+                e[t] = q.cache[(k + t) * kResidentThreads];
                 d[t] = load(__float_as_uint(e[t].w));
             }
 #pragma unroll
         for (int t = 0; t < kBatch; ++t)
-            if (k + t < q.rows) f(xyz(e[t]), d[t]);
-    }
-    for (uint32_t k = q.rows; k < q.cnt; ++k) {   // beyond the shared memory
-        const uint2 v = __ldg(B.nbr + (size_t)k * B.n_total + q.i);
-        f(scale(__uint_as_float(v.y), sub(q.pi, xyz(__ldg(posb(B, v.x))))), load(v.x));
+            if (k + t < q.cnt) f(xyz(e[t]), d[t]);
     }
 }
 
@@ -203,16 +198,13 @@ __device__ __forceinline__ void leave(uint32_t* barrier) {
 
 // A solve of a single-scene context: iterations from the current pressures (or
 // from where k_pressure_first left the density solve: begun != 0) until the
-// solver's control says done.  `rows` list entries per thread fit the dynamic
-// shared memory.
-// kMaxThreads: bounds the block, and with it the registers a thread may take
-// for its loads in flight.  16 entries at a time in the force and 8 in the
-// update; all 36 and 18 at once made an iteration 2.8 us longer at 16k
-// particles (more predicated instructions than latencies saved).
-template <int kMaxThreads>
-__global__ void __launch_bounds__(kMaxThreads, 1)
-    k_solve_resident(Bufs B, ResidentScratch R, int which, int begun, uint32_t rows) {
-    constexpr int kForceBatch = kMaxThreads <= 256 ? 16 : 8, kUpdateBatch = 8;
+// solver's control says done.
+// 16 entries at a time in the force and 8 in the update; all 36 and 18 at once
+// made an iteration 2.8 us longer at 16k particles (more predicated
+// instructions than latencies saved).
+__global__ void __launch_bounds__(kResidentThreads, 3)
+    k_solve_resident(Bufs B, ResidentScratch R, int which, int begun) {
+    constexpr int kForceBatch = 16, kUpdateBatch = 8;
     extern __shared__ float4 s_cache[];
     __shared__ double s_sum[16];
     const DevParams& P = B.P[0];
@@ -235,7 +227,6 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     const uint32_t i = q.i;
     const bool live = i < B.n_total;
     q.cnt = 0;
-    q.rows = 0;
     float4 p4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float rho_i = 0.0f, alpha_i = 0.0f, s_i = 0.0f, p_i = 0.0f;
     uint32_t barrier = 0;
@@ -251,7 +242,6 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         p4 = *posb(B, i);
         q.pi = xyz(p4);
         q.cnt = B.nbr_count[i];
-        q.rows = q.cnt <= kNbrCap ? min(q.cnt, rows) : 0u;
         rho_i = B.rho[i];
         alpha_i = B.alpha[i];
         s_i = B.src[i];
@@ -269,9 +259,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
                 B, i, q.cnt, [&](uint32_t j) { return *posb(B, j); },
                 [&](uint2 v, float4 pj) {
                     const f3 grad = scale(__uint_as_float(v.y), sub(q.pi, xyz(pj)));
-                    if (k < rows)
-                        s_cache[k * blockDim.x + threadIdx.x] =
-                            make_float4(grad.x, grad.y, grad.z, __uint_as_float(v.x));
+                    s_cache[k * kResidentThreads + threadIdx.x] =
+                        make_float4(grad.x, grad.y, grad.z, __uint_as_float(v.x));
                     ++k;
                     force(grad, pj.w);
                 });
@@ -435,9 +424,5 @@ __global__ void __launch_bounds__(kBlock, kResidentBlocks)
     }
     leave(R.barrier);
 }
-
-template __global__ void k_solve_resident<256>(Bufs, ResidentScratch, int, int, uint32_t);
-template __global__ void k_solve_resident<kResidentMaxThreads>(Bufs, ResidentScratch, int, int,
-                                                               uint32_t);
 
 }  // namespace fe
