@@ -46,15 +46,17 @@ PASS_BYTES = {
 }
 
 
-def ns_bytes(passes: int) -> int:
-    # hash 20 + sort (4 + 16 P) + offsets 12 + reorder 52
-    return 20 + 4 + 16 * passes + 12 + 52
+# The neighbour search, a counting sort over the hash table: position read, key
+# and place written 20; count read, zeroed and {start, end} written per slot 16;
+# key, place and start read, index written 16; index, key, bounds and the
+# particle's state read, keys, index and state written 72.
+NS_BYTES = 20 + 16 + 16 + 72
 
 
-def step_bytes(iters: float, passes: int) -> float:
+def step_bytes(iters: float) -> float:
     b = (PASS_BYTES["viscosity"] + PASS_BYTES["density_source"] + PASS_BYTES["pressure_integration"]
          + PASS_BYTES["density_alpha"] + PASS_BYTES["divergence_source"]
-         + PASS_BYTES["divergence_integration"] + PASS_BYTES["stats"] + ns_bytes(passes))
+         + PASS_BYTES["divergence_integration"] + PASS_BYTES["stats"] + NS_BYTES)
     return b + iters * (PASS_BYTES["pressure_force"] + PASS_BYTES["pressure_update"])
 
 
@@ -236,23 +238,26 @@ def barrier(world: int):
         dist.barrier()
 
 
-def launches_per_frame(stats, passes: int, fixed_mode: bool, learned: bool = False) -> float:
-    """Kernels of one frame with one substep (the frame graph's nodes)."""
-    # neighbour search: hash, scratch fill, histogram, P passes, table fill,
-    # offsets, reorder (density_alpha takes the gathered pressure and
-    # learned state current)
-    ns = 1 + 1 + 1 + passes + 1 + 1 + 1
-    # viscosity, density source, 2 x (solve begin + end), integration,
-    # density/alpha (with the divergence source summed in), divergence
-    # integration, substep counter
-    fixed = 1 + 1 + 4 + 1 + 1 + 1 + 1
-    # per Jacobi iteration: force, update, loop guard
-    iters = 3 * (stats.density_iterations + stats.divergence_iterations)
-    # learned: 2 x the network (which also applies the start); features,
-    # after-solve bookkeeping and the carry permutation ride in the source,
-    # integration and reorder passes
-    extra = 2 if learned else 0
-    return 1 + ns + fixed + iters + extra   # + prologue (the stats ride in the last integration)
+def launches_per_frame(stats, n: int, learned: bool = False) -> float:
+    """Kernels of one single-scene frame with one substep (the frame graph's)."""
+    # neighbour search: count, scan, scatter, reorder
+    search = 4
+    # prologue, viscosity, density source, integration, density/alpha (with the
+    # divergence source summed in), divergence integration (with the stats),
+    # substep counter
+    fixed = 7
+    # the plain density solve's first iteration; learned: 2 x the network
+    # (features, after-solve bookkeeping and the carry permutation ride in the
+    # source, integration and reorder passes)
+    start = 2 if learned else 1
+    if n <= 148 * 256:
+        solves = 2          # each solve one resident kernel
+    else:
+        # begin (of the plain density solve the first iteration) and end of
+        # each, and per further iteration force, update and loop guard
+        its = stats.density_iterations + stats.divergence_iterations - (0 if learned else 1)
+        solves = (4 if learned else 3) + 3 * its
+    return search + fixed + start + solves
 
 
 # ---------------------------------------------------------------------------
@@ -279,7 +284,6 @@ def measure_arm(args, w, params, model, world, local, build="parity"):
         tune_report = sim.data.autotune().as_dict()
     else:
         tune_report = None
-    tuning = sim.data.tuning()
     stream = torch.cuda.ExternalStream(lib.fe_get_stream(h), device=local)
     # --eager launches each frame's kernels directly (FE_STEP_NO_GRAPH); the
     # kernels and their work are the same as in the graph replay.
@@ -382,15 +386,12 @@ def measure_arm(args, w, params, model, world, local, build="parity"):
         if name == "neighbor_search":
             lib.fe_density_alpha(h)
     lib.fe_synchronize(h)
-    key_bits = max(1, int(np.ceil(np.log2(max(sim.data.table_size, 2)))))
-    passes = -(-key_bits // tuning.radix_digit_bits)
-    fixed_mode = params.mode == _abi.FE_MODE_FIXED
     avg = type("S", (), {"density_iterations": iters_d, "divergence_iterations": iters_v})
-    launches = launches_per_frame(avg, passes, fixed_mode, model is not None) * args.steps
+    launches = launches_per_frame(avg, n, model is not None) * args.steps
     sim.close()
     return {"n": n, "dev_ms": dev_ms_max, "value": n * args.steps * world / (dev_ms_max / 1e3),
             "e2e": n * args.steps * world / e2e_s, "iters": (iters_d, iters_v),
-            "kern": kern, "passes": passes, "launches": int(round(launches)),
+            "kern": kern, "launches": int(round(launches)),
             "clocks": clocks.summary(), "residual": (st.density_residual, st.divergence_residual),
             "tuning": tune_report}
 
@@ -816,8 +817,8 @@ def run_gpu(args) -> None:
             "issue_roofline": issue,
             "fp32_roofline": fp32,
             "kernel_ms": kern,
-            "step_roofline": {"algorithmic_bytes_per_step": step_bytes(it_total, head["passes"]) * n,
-                              "frac": step_bytes(it_total, head["passes"]) * n
+            "step_roofline": {"algorithmic_bytes_per_step": step_bytes(it_total) * n,
+                              "frac": step_bytes(it_total) * n
                               / (head["dev_ms"] / args.steps / 1e3) / 1e9 / peak},
             "sort": {**sort, "roofline_frac": 68 * sort["n"] / (sort["ms"] / 1e3) / 1e9 / peak},
             "gpu_launches": head["launches"],

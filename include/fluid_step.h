@@ -441,8 +441,8 @@ FE_API fe_status fe_debug_bounded_wait(int device, uint32_t limit, uint32_t* fla
  *                  divergence source, divergence solve,
  *                  divergence integration };
  *   stats.
- * The frame is replayed from a CUDA graph (conditional WHILE nodes for the
- * tolerance solver) unless FE_STEP_NO_GRAPH.  `out` may be NULL; when given,
+ * The frame is replayed from a CUDA graph (its solves conditional WHILE nodes,
+ * or for few particles one kernel each) unless FE_STEP_NO_GRAPH.  `out` may be NULL; when given,
  * the call synchronises and fills it. */
 FE_API fe_status fe_step(fe_ctx* ctx, uint32_t n_substeps, uint32_t flags, fe_stats* out);
 
@@ -457,8 +457,9 @@ FE_API fe_status fe_step(fe_ctx* ctx, uint32_t n_substeps, uint32_t flags, fe_st
  *     `cpu_radix_sort` (sorter.rs:465-559).  `key_bits` (1..32) bounds the
  *     key range: keys must be < 2^key_bits; 32 sorts any keys.  Digit width
  *     and keys per thread are those fe_autotune_sort chose for this device
- *     and size class, else 8-bit digits and 16 keys per thread; the result
- *     does not depend on them.
+ *     and size class, else 8-bit digits and 16 keys per thread; up to 65536
+ *     pairs are sorted by one cluster instead.  The result does not depend
+ *     on any of it.
  *   FE_SORT_BITONIC: the compare-exchange network of bitonic_sort.comp;
  *     n must be a power of two; not stable (same network, same result as
  *     the reference for the same input).
@@ -488,14 +489,17 @@ FE_API fe_status fe_sort_flags(uint32_t* flags_out, void* stream);
 /* Tunable shapes; none of them changes a result.
  *   radix_digit_bits, radix_items: onesweep digit width (8 or 10) and keys
  *     per thread (4, 8, 16; the pairs (8,4) (8,8) (8,16) (10,8) (10,16)).
+ *     A context's neighbour search is a counting sort, which has no shape;
+ *     they are kept for the report.
  *   mlp_ctas_per_sm: blocks per SM of the learned warm start's inference
  *     grid (1..6; at most 4 fit on an SM, larger values act as 4).
  *   nbr_threads[g]: threads per block of neighbour group g, 128, 256 or 512
  *     (a block covers half a 256-particle chunk per pass, one chunk, or two
  *     chunks at a time; particles per thread = 256 / threads per chunk);
- *     FE_NBR_DENSITY_ALPHA 128 or 256 (its per-warp shared scratch),
+ *     FE_NBR_DENSITY_ALPHA 128 or 256 (of no effect: its blocks have 64),
  *     FE_NBR_PRESSURE_UPDATE 256 only, its FP64 sums being per chunk.  0
  *     means 256.
+ *     The other groups' apply above 18944 particles.
  *   nbr_persistent[g]: 1 = persistent grid (as many blocks as fit on the
  *     GPU at once, each striding over the chunk table of all scenes); 0 =
  *     one block per chunk (or chunk pair). */
