@@ -4,11 +4,14 @@
 // pressure_update each take some 7 us of which 2 are the launch and most of the
 // rest the chain parameters -> count -> list words -> neighbours, and the graph's
 // WHILE node adds 7 us between iterations (16k particles: 24 us an iteration,
-// here 8.6).
-// Here every particle keeps a thread for all the iterations.  The pair gradients, which do not change during a solve, stay in
-// shared memory with the neighbours' indices, so an iteration is two gathers
-// (4 bytes of p / rho^2, 16 of acceleration), all of a thread's loads in flight
-// together, and two grid-wide barriers.
+// with a particle per thread 8.6).
+// Here every particle keeps a thread for all the iterations.  The pair
+// gradients, which do not change during a solve, stay in shared memory with the
+// neighbours' indices, so an iteration is two gathers (4 bytes of p / rho^2, 16
+// of acceleration), a thread's loads in flight together, and two grid-wide
+// barriers: 4.1k particles' frame of 4 + 4 iterations 232 -> 133 us.  More
+// particles take chunks (k_solve_resident_many): 16k 262 -> 207 us, 32k 282 ->
+// 218.  How far each goes is decided in choose_resident.
 //
 // The arithmetic is that of k_pressure_force and k_pressure_update in the same
 // order (the same bits), and so are the tolerance solver's FP64 sums, which
