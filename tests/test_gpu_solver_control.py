@@ -80,9 +80,9 @@ def test_frame_solve_is_the_solve_pass_by_pass(mode, n, iters, non_finite):
 @pytest.mark.parametrize("n", [9472, 9473, 18945, 28417, 37888, 37889, 56832, 56833])
 @pytest.mark.parametrize("cap", [100, 3])
 def test_resident_solve_around_its_lines(oracle_mod, n, cap):
-    """The solve as one kernel, around the sizes where its block grows and where
-    it goes over to striding over chunks: iterations to a tolerance (the FP64 sums over warps and chunks)
-    and to a cap, against the oracle."""
+    """The solve as one kernel, around the sizes where a particle per thread goes
+    over to chunks and chunks to the iterated passes: iterations to a tolerance
+    (the FP64 sums over warps and chunks) and to a cap, against the oracle."""
     p = scene.dam_break_params((0, 0, 0), (4.0, 4.0, 4.0), mode=_abi.FE_MODE_FIXED,
                                solver=_abi.FE_SOLVER_TOLERANCE)
     p.max_iterations = cap
