@@ -33,6 +33,7 @@
 #include "fe_mlp.h"
 #include "fe_model.h"
 #include "fe_sort.h"
+#include "fe_sort_scratch.h"
 #include "fe_raymarch.h"
 #include "fe_splat.h"
 #include "fe_tune.h"
@@ -437,10 +438,8 @@ namespace {
 std::atomic<uint32_t> g_fail_countdown{0};
 std::atomic<int> g_poison{0};
 
-template <class T>
-fe_status dev_alloc(fe_ctx* c, T** out, size_t count) {
-    void* p = nullptr;
-    size_t bytes = std::max<size_t>(count * sizeof(T), 16);
+// cudaMalloc, counted by the hook that makes one fail.
+fe_status raw_alloc(void** out, size_t bytes) {
     uint32_t k = g_fail_countdown.load();
     while (k != 0 && !g_fail_countdown.compare_exchange_weak(k, k - 1)) {
     }
@@ -448,11 +447,20 @@ fe_status dev_alloc(fe_ctx* c, T** out, size_t count) {
         set_error("device allocation of %zu bytes failed (injected)", bytes);
         return FE_ERR_OUT_OF_MEMORY;
     }
-    cudaError_t e = cudaMalloc(&p, bytes);
+    cudaError_t e = cudaMalloc(out, bytes);
     if (e != cudaSuccess) {
         set_error("cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
         return FE_ERR_OUT_OF_MEMORY;
     }
+    return FE_OK;
+}
+
+template <class T>
+fe_status dev_alloc(fe_ctx* c, T** out, size_t count) {
+    void* p = nullptr;
+    size_t bytes = std::max<size_t>(count * sizeof(T), 16);
+    fe_status s = raw_alloc(&p, bytes);
+    if (s != FE_OK) return s;
     if (g_poison.load() && cudaMemset(p, 0xFF, bytes) != cudaSuccess) {
         cudaFree(p);
         set_error("poisoning a new allocation failed");
@@ -2124,14 +2132,7 @@ FE_API fe_status fe_debug_read_trace(fe_ctx* c, uint32_t slot, uint16_t* rows, f
 // an event serialises users of the same scratch across streams.
 // ---------------------------------------------------------------------------
 namespace {
-struct SortScratch {
-    int device = -1;
-    uint32_t cap = 0;
-    uint32_t* tk = nullptr;
-    uint32_t* tv = nullptr;
-    uint32_t* words = nullptr;
-    size_t nwords = 0;
-    uint32_t* flags = nullptr;
+struct SortScratch : SortBuffers {
     cudaEvent_t done = nullptr;
 };
 std::mutex g_sort_mutex;
@@ -2181,19 +2182,19 @@ fe_status sort_pairs_impl(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t k
     std::lock_guard<std::mutex> lock(g_sort_mutex);
     SortScratch& S = g_sort[dev];
     const uint32_t kb = key_bits ? key_bits : 32;
+    if (!S.done) FE_CUDA(cudaEventCreateWithFlags(&S.done, cudaEventDisableTiming));
+    if (S.flags) {
+        FE_CUDA(cudaStreamWaitEvent(stream, S.done, 0));
+    } else {
+        fe_status st = raw_alloc((void**)&S.flags, kSortFlagWords * 4);
+        if (st != FE_OK) return st;
+        FE_CUDA(cudaMemsetAsync(S.flags, 0, kSortFlagWords * 4, stream));
+    }
     // Few pairs: one cluster sorts them in one launch, whatever shape is tuned
     // (us, 32-bit keys, copies of the input included; onesweep at its default
     // shape / this: 1k 48/24, 32k 60/31, 64k 62/43).  An explicit shape is taken
     // as it is.
     if (!forced && n <= kSmallSortMax) {
-        if (S.flags) {
-            FE_CUDA(cudaStreamWaitEvent(stream, S.done, 0));
-        } else {   // the error word alone: its scratch grows when a sort needs it
-            if (!S.done) FE_CUDA(cudaEventCreateWithFlags(&S.done, cudaEventDisableTiming));
-            FE_CUDA(cudaMalloc(&S.words, 32));
-            S.flags = S.words;
-            S.device = dev;
-        }
         const cudaError_t e = radix_sort_small(keys, vals, n, kb, S.flags, stream);
         if (e == cudaSuccess) {
             FE_CUDA(cudaEventRecord(S.done, stream));
@@ -2206,29 +2207,14 @@ fe_status sort_pairs_impl(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t k
         cfg = *forced;
     else
         sort_tuning_lookup(dev, n, kb, &cfg);
-    size_t words = radix_scratch_words(n, kb, cfg);
-    if (S.cap < n || S.nwords < words) {
-        if (S.done) FE_CUDA(cudaEventSynchronize(S.done));
-        cudaFree(S.tk);
-        cudaFree(S.tv);
-        cudaFree(S.words);
-        S.tk = S.tv = S.words = S.flags = nullptr;
-        uint32_t cap = std::max(n, S.cap);
-        size_t nw = std::max(words, S.nwords);
-        FE_CUDA(cudaMalloc(&S.tk, (size_t)cap * 4));
-        FE_CUDA(cudaMalloc(&S.tv, (size_t)cap * 4));
-        FE_CUDA(cudaMalloc(&S.words, (nw + 8) * 4));
-        S.cap = cap;
-        S.nwords = nw;
-        S.flags = S.words + nw;
-        FE_CUDA(cudaMemset(S.flags, 0, 32));
-        if (!S.done) FE_CUDA(cudaEventCreateWithFlags(&S.done, cudaEventDisableTiming));
-        S.device = dev;
-    } else {
-        FE_CUDA(cudaStreamWaitEvent(stream, S.done, 0));
+    const size_t words = radix_scratch_words(n, kb, cfg);
+    if (!sort_buffers_hold(S, n, words)) {
+        FE_CUDA(cudaEventSynchronize(S.done));   // nothing uses the old ones any more
+        fe_status st = sort_buffers_grow(S, n, words, raw_alloc, cudaFree);
+        if (st != FE_OK) return st;
     }
     // the error word reports this call only (fe_sort_flags reads it)
-    REC(R.fill_u32(S.flags, 0u, 8));
+    REC(R.fill_u32(S.flags, 0u, kSortFlagWords));
     bool in_tmp = false;
     REC(radix_sort(L, keys, vals, S.tk, S.tv, n, kb, S.words, S.flags, &in_tmp, cfg));
     if (in_tmp) {

@@ -99,3 +99,30 @@ def test_bounded_wait_runs_out_and_the_device_stays_usable(lib):
                                   5000, 32, _abi.FE_SORT_RADIX) == _abi.FE_OK
     order = np.argsort(keys, kind="stable")
     assert np.array_equal(k, keys[order]) and np.array_equal(v, vals[order])
+
+
+@pytest.mark.parametrize("k", [1, 2, 3])
+def test_sorts_after_a_failed_growth_of_their_buffers(lib, k):
+    """The k-th allocation of a growing sort fails: small sorts (which need the
+    error word alone), sorts that fitted before the growth and the same sort
+    again are right."""
+    import torch
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def sort(n):
+        keys = torch.randint(0, 1 << 30, (n,), dtype=torch.int32, device="cuda")
+        vals = torch.arange(n, dtype=torch.int32, device="cuda")
+        ref = torch.sort(keys, stable=True)
+        rc = lib.fe_sort_pairs(ctypes.c_void_p(keys.data_ptr()), ctypes.c_void_p(vals.data_ptr()),
+                               n, 32, _abi.FE_SORT_RADIX, st)
+        if rc == _abi.FE_OK:
+            assert torch.equal(keys, ref.values) and torch.equal(vals.long(), ref.indices)
+        return rc
+
+    grown = (8 + k) << 20          # beyond every other test's
+    assert sort(1000) == _abi.FE_OK and sort(200_000) == _abi.FE_OK
+    lib.fe_debug_fail_allocation(k)
+    assert sort(grown) == _abi.FE_ERR_OUT_OF_MEMORY
+    assert b"injected" in lib.fe_last_error()
+    for n in (1000, 200_000, 65_537, grown):
+        assert sort(n) == _abi.FE_OK
