@@ -83,8 +83,9 @@ __device__ __forceinline__ void for_each_particle(const Bufs& B, F&& f) {
 
 // The bucket walk of the shaders (e.g. density_and_alpha.comp:31-63) over the
 // {start, end} table.  f(j, r_vec, r2) is called for each candidate with
-// r2 <= h*h, in walk order.
-template <class F>
+// r2 <= h*h, in walk order.  kCoherent: see for_each_neighbor (the table is
+// the search's, so its loads are read-only ones either way).
+template <bool kCoherent = false, class F>
 __device__ __forceinline__ void walk(const Bufs& B, const DevParams& P, f3 pi, F&& f) {
     const float h = P.h;
     const float h2 = h * h;
@@ -99,7 +100,7 @@ __device__ __forceinline__ void walk(const Bufs& B, const DevParams& P, f3 pi, F
                 const uint2 cell = __ldg(B.cells + k);
                 if (cell.x == kEmpty) continue;
                 for (uint32_t j = cell.x; j < cell.y; ++j) {
-                    f3 rv = sub(pi, xyz(__ldg(posb(B, j))));
+                    f3 rv = sub(pi, xyz(kCoherent ? *posb(B, j) : __ldg(posb(B, j))));
                     float r2 = dot(rv, rv);
                     if (r2 > h2) continue;
                     f(j, rv, r2);
@@ -189,7 +190,7 @@ __device__ __forceinline__ void for_each_neighbor(const Bufs& B, const DevParams
             [&](uint2 v, float4 q) { f(sub(pi, xyz(q)), __uint_as_float(v.y), q); });
     } else {
         const float h = P.h;
-        walk(B, P, pi, [&](uint32_t j, f3 rv, float r2) {
+        walk<kCoherent>(B, P, pi, [&](uint32_t j, f3 rv, float r2) {
             float r = sqrtf(r2);
             if (r > kEpsR)
                 f(rv, kernel_grad_scale(r, h), kCoherent ? *posb(B, j) : __ldg(posb(B, j)));
@@ -227,7 +228,7 @@ __device__ __forceinline__ void for_each_neighbor_pair(const Bufs& B, const DevP
             });
     } else {
         const float h = P.h;
-        walk(B, P, pi, [&](uint32_t j, f3 rv, float r2) {
+        walk<kCoherent>(B, P, pi, [&](uint32_t j, f3 rv, float r2) {
             float r = sqrtf(r2);
             const float4* data = recs + 2 * (size_t)j + 1;
             if (r > kEpsR) f(rv, kernel_grad_scale(r, h), kCoherent ? *data : __ldg(data));

@@ -71,7 +71,7 @@ __device__ __forceinline__ void for_each_cached(const Bufs& B, const DevParams& 
                                                 const Particle& q, Load&& load, F&& f) {
     if (q.cnt > kNbrCap) {
         const float h = P.h;
-        walk(B, P, q.pi, [&](uint32_t j, f3 rv, float r2) {
+        walk<true>(B, P, q.pi, [&](uint32_t j, f3 rv, float r2) {
             const float r = sqrtf(r2);
             if (r > kEpsR) f(scale(kernel_grad_scale(r, h), rv), load(j));
         });

@@ -145,3 +145,58 @@ def test_batch_solves_resident_or_iterated(solvers):
     batch.close()
     for sim in singles:
         sim.close()
+
+
+def _with_clumps(n, per_clump, seed):
+    """A lattice of n particles and, above it, four clumps whose particles have
+    more neighbours than the list holds."""
+    pos, _ = scene.lattice((0, 0, 0), (40, 20, 48), 0.025, 1000.0, 0.05, 0.02, seed)
+    rng = np.random.default_rng(seed)
+    at = np.array([[0.55, 2.0, 0.55], [1.55, 2.0, 0.55], [0.55, 2.0, 1.55], [0.6, 2.0, 0.6]])
+    clumps = np.repeat(at, per_clump, 0) + rng.uniform(-0.04, 0.04, (4 * per_clump, 3))
+    return np.concatenate([pos[:n], clumps]).astype(np.float32)
+
+
+@pytest.mark.parametrize("per_clump", [64, 90])
+@pytest.mark.parametrize("solver", [_abi.FE_SOLVER_TOLERANCE, _abi.FE_SOLVER_FIXED_ITERS])
+@pytest.mark.parametrize("n", [11000, 30011])
+def test_strided_resident_solve_past_the_neighbour_list(oracle_mod, n, solver, per_clump):
+    """Particles with more neighbours than the list holds walk the buckets in
+    every half iteration, between whose barriers other blocks write what the walk
+    reads: several iterations over strided chunks against the oracle."""
+    p = scene.dam_break_params((0, 0, 0), (4.0, 4.0, 4.0), mode=_abi.FE_MODE_FIXED, solver=solver)
+    p.density_solver_iterations, p.divergence_solver_iterations = 9, 7
+    p.min_iterations, p.max_iterations = 5, 12
+    p.dt = 0.0002
+    pos = _with_clumps(n, per_clump, 3)
+    sim, orc = Simulation(pos, p), oracle_mod.Oracle(p, pos)
+    for _ in range(2):
+        a, b = sim.step(1), orc.step(1)
+        assert a.flags & _abi.FE_STATS_NEIGHBOR_OVERFLOW
+        assert (a.density_iterations, a.divergence_iterations) == (b.density_iterations,
+                                                                   b.divergence_iterations)
+        for f in FIELDS:
+            x, y = sim.data.download(f).view(np.uint32), orc.field(f).view(np.uint32)
+            assert np.array_equal(x, y), f
+    sim.close()
+
+
+def test_batch_resident_solve_past_the_neighbour_list(oracle_mod):
+    """The same in the scenes of a fixed-iteration batch."""
+    pos = [_with_clumps(900, 90, 1), _with_clumps(2500, 70, 2), _with_clumps(700, 0, 3)]
+    params = []
+    for k in range(3):
+        p = scene.dam_break_params((0, 0, 0), (4.0, 4.0, 4.0), mode=_abi.FE_MODE_FIXED)
+        p.density_solver_iterations, p.divergence_solver_iterations = 6 + k, 5
+        p.dt = 0.0002
+        params.append(p)
+    batch = BatchSimulation(pos, params)
+    oracles = [oracle_mod.Oracle(p, a) for p, a in zip(params, pos)]
+    for _ in range(2):
+        batch.step(1, want_stats=False)
+        for s, orc in enumerate(oracles):
+            orc.step(1)
+            for f in FIELDS:
+                x = batch.data.scene(batch.data.download(f), s)
+                assert np.array_equal(x.view(np.uint32), orc.field(f).view(np.uint32)), (s, f)
+    batch.close()
