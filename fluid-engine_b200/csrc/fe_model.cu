@@ -275,10 +275,11 @@ FE_API fe_status fe_model_train_step(fe_model* m, const float* d_x, const float*
     }
     cudaStream_t s = (cudaStream_t)stream;
     M_CUDA(cudaSetDevice(m->device));
-    m->step += 1;
+    const uint32_t step = m->step + 1;   // counted once it has been launched
     M_CUDA(mlp::train_step(m->params(), d_x, d_y, m->norm, n, m->grad_part, m->flags, m->master,
                            m->adam_m, m->adam_v, m->wbf16, m->grad + mlp::kParams, lr, 0.9f,
-                           0.999f, 1e-8f, m->step, weight_decay, s, m->num_sms));
+                           0.999f, 1e-8f, step, weight_decay, s, m->num_sms));
+    m->step = step;
     if (h_loss) {
         M_CUDA(cudaMemcpyAsync(h_loss, m->grad + mlp::kParams, 4, cudaMemcpyDeviceToHost, s));
         M_CUDA(cudaStreamSynchronize(s));

@@ -68,3 +68,43 @@ def reference_gradients(ref, p, xs, e):
     dz1 = (dz2b @ q(w2)) * ref.silu_grad(z1)
     return np.concatenate([(q(dz1).T @ X).reshape(-1), (dz2b.T @ h1).reshape(-1),
                            (dob.T @ h2).reshape(-1), dz1.sum(0), dz2.sum(0), do.sum(0)])
+
+
+def test_a_step_that_failed_is_not_counted():
+    """A step whose launches were refused (its stream's capture had been given up)
+    has not updated the weights, so the next one's bias correction is that of a
+    run without it."""
+    import torch
+    rng = np.random.default_rng(2)
+    x = torch.from_numpy(rng.normal(size=(300, 12)).astype(np.float32)).cuda()
+    y = torch.from_numpy(rng.normal(size=(300, 2)).astype(np.float32)).cuda()
+    torch.cuda.synchronize()
+    models = [Model(seed=3), Model(seed=3)]
+    lib = models[0].lib
+    rt = ctypes.CDLL("libcudart.so.12")      # the one torch has loaded
+
+    def step(m, stream=None):
+        return lib.fe_model_train_step(m.handle, ctypes.c_void_p(x.data_ptr()),
+                                       ctypes.c_void_p(y.data_ptr()), 300, 1e-2, 0.0, stream, None)
+
+    def refused(m):
+        stream, graph = ctypes.c_void_p(), ctypes.c_void_p()
+        assert rt.cudaStreamCreateWithFlags(ctypes.byref(stream), 1) == 0
+        assert rt.cudaStreamBeginCapture(stream, 1) == 0          # thread-local
+        assert rt.cudaStreamSynchronize(stream) != 0              # gives the capture up
+        rc = step(m, stream)
+        assert rt.cudaStreamEndCapture(stream, ctypes.byref(graph)) != 0
+        rt.cudaGetLastError()
+        assert rt.cudaStreamDestroy(stream) == 0
+        return rc
+
+    for m, fail in zip(models, (False, True)):
+        assert step(m) == _abi.FE_OK
+        if fail:
+            assert refused(m) == _abi.FE_ERR_CUDA
+        assert step(m) == _abi.FE_OK
+    torch.cuda.synchronize()
+    a, b = models[0].parameters(), models[1].parameters()
+    assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    for m in models:
+        m.close()
