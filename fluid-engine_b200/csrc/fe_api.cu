@@ -438,28 +438,11 @@ namespace {
 std::atomic<uint32_t> g_fail_countdown{0};
 std::atomic<int> g_poison{0};
 
-// cudaMalloc, counted by the hook that makes one fail.
-fe_status raw_alloc(void** out, size_t bytes) {
-    uint32_t k = g_fail_countdown.load();
-    while (k != 0 && !g_fail_countdown.compare_exchange_weak(k, k - 1)) {
-    }
-    if (k == 1) {
-        set_error("device allocation of %zu bytes failed (injected)", bytes);
-        return FE_ERR_OUT_OF_MEMORY;
-    }
-    cudaError_t e = cudaMalloc(out, bytes);
-    if (e != cudaSuccess) {
-        set_error("cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
-        return FE_ERR_OUT_OF_MEMORY;
-    }
-    return FE_OK;
-}
-
 template <class T>
 fe_status dev_alloc(fe_ctx* c, T** out, size_t count) {
     void* p = nullptr;
     size_t bytes = std::max<size_t>(count * sizeof(T), 16);
-    fe_status s = raw_alloc(&p, bytes);
+    fe_status s = fe_device_alloc(&p, bytes);
     if (s != FE_OK) return s;
     if (g_poison.load() && cudaMemset(p, 0xFF, bytes) != cudaSuccess) {
         cudaFree(p);
@@ -1108,6 +1091,22 @@ void fe_set_error_message(const char* fmt, ...) {
     va_start(ap, fmt);
     set_error_v(fmt, ap);
     va_end(ap);
+}
+
+fe_status fe_device_alloc(void** out, size_t bytes) {
+    uint32_t k = g_fail_countdown.load();
+    while (k != 0 && !g_fail_countdown.compare_exchange_weak(k, k - 1)) {
+    }
+    if (k == 1) {
+        set_error("device allocation of %zu bytes failed (injected)", bytes);
+        return FE_ERR_OUT_OF_MEMORY;
+    }
+    cudaError_t e = cudaMalloc(out, bytes);
+    if (e != cudaSuccess) {
+        set_error("cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
+        return FE_ERR_OUT_OF_MEMORY;
+    }
+    return FE_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -2186,7 +2185,7 @@ fe_status sort_pairs_impl(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t k
     if (S.flags) {
         FE_CUDA(cudaStreamWaitEvent(stream, S.done, 0));
     } else {
-        fe_status st = raw_alloc((void**)&S.flags, kSortFlagWords * 4);
+        fe_status st = fe_device_alloc((void**)&S.flags, kSortFlagWords * 4);
         if (st != FE_OK) return st;
         FE_CUDA(cudaMemsetAsync(S.flags, 0, kSortFlagWords * 4, stream));
     }
@@ -2210,7 +2209,7 @@ fe_status sort_pairs_impl(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_t k
     const size_t words = radix_scratch_words(n, kb, cfg);
     if (!sort_buffers_hold(S, n, words)) {
         FE_CUDA(cudaEventSynchronize(S.done));   // nothing uses the old ones any more
-        fe_status st = sort_buffers_grow(S, n, words, raw_alloc, cudaFree);
+        fe_status st = sort_buffers_grow(S, n, words, fe_device_alloc, cudaFree);
         if (st != FE_OK) return st;
     }
     // the error word reports this call only (fe_sort_flags reads it)

@@ -67,8 +67,10 @@ fe_status fe_model::ensure_scratch(uint32_t n) {
     if (n <= scratch_rows) return FE_OK;
     cudaFree(xb);
     xb = nullptr;
+    scratch_rows = 0;   // until they are there
     uint32_t rows = n + 1024;
-    M_CUDA(cudaMalloc(&xb, (size_t)rows * 16 * sizeof(__nv_bfloat16)));
+    const fe_status st = fe_device_alloc((void**)&xb, (size_t)rows * 16 * sizeof(__nv_bfloat16));
+    if (st != FE_OK) return st;
     scratch_rows = rows;
     return FE_OK;
 }

@@ -414,9 +414,9 @@ FE_API fe_status fe_state_import(fe_ctx* ctx, const void* src, size_t bytes);
  * without faulting a GPU.  They are process-wide and not thread-safe with
  * respect to concurrent context creation.
  * fe_debug_fail_allocation(k): the k-th device allocation of a context
- *   (fe_create, fe_batch_create and the buffers contexts add later) or of
- *   fe_sort_pairs' buffers from now on fails with FE_ERR_OUT_OF_MEMORY; 0
- *   turns the hook off.
+ *   (fe_create, fe_batch_create and the buffers contexts add later), of
+ *   fe_sort_pairs' buffers or of a model's rows from now on fails with
+ *   FE_ERR_OUT_OF_MEMORY; 0 turns the hook off.
  * fe_debug_poison_allocations(on): new context allocations are filled with
  *   0xFF bytes (NaN as floats, 0xFFFFFFFF as indices), so that a read of
  *   memory no pass has written shows up in the results.

@@ -126,3 +126,29 @@ def test_sorts_after_a_failed_growth_of_their_buffers(lib, k):
     assert b"injected" in lib.fe_last_error()
     for n in (1000, 200_000, 65_537, grown):
         assert sort(n) == _abi.FE_OK
+
+
+def test_forward_after_a_failed_growth_of_its_rows(lib):
+    """A forward call whose larger row buffer could not be allocated: calls that
+    fitted the buffer before and the same call again give what they gave."""
+    import torch
+    from fluid_step.learned import Model
+    m = Model(seed=2)
+    x = torch.randn(50_000, 12, device="cuda")
+
+    def forward(n):
+        y = torch.zeros(n, 2, device="cuda")
+        rc = lib.fe_model_forward(m.handle, ctypes.c_void_p(x.data_ptr()),
+                                  ctypes.c_void_p(y.data_ptr()), n,
+                                  ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        return rc, y
+
+    rc, before = forward(900)
+    assert rc == _abi.FE_OK
+    lib.fe_debug_fail_allocation(1)
+    assert forward(50_000)[0] == _abi.FE_ERR_OUT_OF_MEMORY
+    rc, after = forward(900)
+    assert rc == _abi.FE_OK and torch.equal(before, after)
+    rc, whole = forward(50_000)
+    assert rc == _abi.FE_OK and torch.equal(whole[:900], before)
+    m.close()
