@@ -389,8 +389,10 @@ __global__ void __launch_bounds__(kBlock) k_refresh_pr(Bufs B) {
 // particles share a cell also shares that cell's 27 buckets.
 //  * Few runs (bulk fluid, several particles per cell): cell-cooperative.  A
 //    run's buckets laid end to end in walk order (z, y, x offsets, each
-//    bucket's entries in sorted order) are its row of candidates.  The warp
-//    takes all its runs' rows a slab of 32 candidates at a time: it stages the
+//    bucket's entries in sorted order) are its row of candidates.  The rows
+//    are taken a window of kMaxSlabs slabs at a time, phase 1 and 2 for each
+//    (mostly there is one).  Of a window the warp takes all its runs'
+//    candidates a slab of 32 at a time: it stages the
 //    slab's positions (each loaded once per run) in shared memory, and every
 //    lane then tests its own particle against the 32 candidates of its run
 //    and keeps the mask.  The test is a superset of the exact one, in packed
@@ -401,15 +403,20 @@ __global__ void __launch_bounds__(kBlock) k_refresh_pr(Bufs B) {
 //    particle index.
 //  * Many runs (spray, sparse cells): each lane walks its own 27 buckets and
 //    records its in-range candidates, kStage of them at a time.
-// A run whose row is longer than kMaxSlabs * 32 does everything in a
-// single-phase walk.
 // ---------------------------------------------------------------------------
-// In-range candidates a lane can keep in the per-lane form; row length and runs
-// of the cooperative form: what fits 5.6 KB per warp, 32 warps an SM.  A
+// In-range candidates a lane can keep in the per-lane form; window and runs of
+// the cooperative form: what fits 5.6 KB per warp, 32 warps an SM.  A
 // moving dam break has 5 to 8 runs in the mean warp and more than 10 in 5 to
-// 15 % of them; its rows are 70 to 320 candidates long.
+// 15 % of them; its rows are 70 to 320 candidates long.  Rows longer than a window
+// come with a denser fluid, a larger h, and buckets that cells share (12,000
+// particles at rest, 0.1 % of them with 385 to 392 candidates: 89 us when those
+// walked in one phase, 36 in windows).  1M particles in motion, ms, walked /
+// windows: h of 2.0 spacings 0.41 / 0.42, 2.42 1.62 / 0.73, 2.9 1.31 / 0.97.  Only
+// where every candidate is in range, thousands of particles on one spot, does the
+// test cost more than it saves (16k there: 5.7 / 7.1).
 constexpr int kStage = 44;
 constexpr int kMaxSlabs = 12;
+constexpr uint32_t kWindow = kMaxSlabs * 32;
 constexpr int kCoopRuns = 10;
 
 // The near test in half precision, in units of h, relative to the first
@@ -427,14 +434,15 @@ constexpr float kCoopMinH = 1e-15f, kCoopMaxH = 1e15f;
 union DensityScratch {
     struct {
         uint32_t mask[kMaxSlabs][32];
-        // the row of each run: where non-empty buckets start (bit c of word w:
-        // at candidate 32 w + c), how many start before a word, each bucket's
-        // first entry minus its place in the row, and the row's length (0: too
-        // long)
+        // the window of each run's row: where non-empty buckets start (bit c of
+        // word w: at candidate 32 w + c; a bucket that goes on from the window
+        // before starts at 0), how many start before a word, each bucket's
+        // first entry minus its place in the window, and the candidates in it
         uint32_t starts[kCoopRuns][kMaxSlabs];
         uint8_t before[kCoopRuns][kMaxSlabs];
         uint32_t first[kCoopRuns][27];
         uint32_t total[kCoopRuns];
+        int3 cell[kCoopRuns];
         alignas(16) float4 head[kCoopRuns];   // position of the run's first particle
         // a slab of each run: x, y, z as 16 pairs (candidate k, candidate
         // k + 16).  208 bytes apart, so that eight runs' 16-byte reads fall
@@ -508,23 +516,19 @@ __device__ __forceinline__ uint32_t row_entry(const uint32_t* first, uint32_t st
     return first[slot] + (sl << 5) + bit;
 }
 
-// Cooperative phase 1 over the runs of one warp (see above), given by their
-// first lanes.  Returns the calling lane's run, or -1 if its row is too long,
-// and the number of candidates that passed the near test.  All 32 lanes.
-__device__ __forceinline__ int coop_candidates(const Bufs& B, const DevParams& P,
-                                               DensityScratch& S, uint32_t heads, bool live,
-                                               int cx, int cy, int cz, float4 p4,
-                                               uint32_t& n_in) {
+// Candidates [from, from + kWindow) of the rows of the warp's runs (see above;
+// S.cell and S.head are set): the calling lane's masks, and in n_in the number
+// that passed the near test.  Returns whether a row goes on.  All 32 lanes.
+__device__ __forceinline__ bool coop_candidates(const Bufs& B, const DevParams& P,
+                                                DensityScratch& S, int runs, int run, bool live,
+                                                float4 p4, uint32_t from, uint32_t& n_in) {
     constexpr int kGroup = 4;   // runs whose loads are in flight together
-    constexpr uint32_t kLong = 2047u;   // stands for any longer bucket: 27 fit 16 bits
     const uint32_t lane = (uint32_t)lane_id();
     const uint32_t lt_mask = (1u << lane) - 1u;
-    const int runs = __popc(heads);
-    const int run = __popc(heads & (lt_mask | (1u << lane))) - 1;
+    bool more = false;
+    n_in = 0;
     for (uint32_t t = lane; t < kCoopRuns * kMaxSlabs; t += 32) (&S.starts[0][0])[t] = 0u;
-    if ((heads >> lane) & 1u) S.head[run] = p4;
     __syncwarp();
-    uint32_t left = heads;
 #pragma unroll 1
     for (int r0 = 0; r0 < runs; r0 += kGroup) {
         uint32_t start[kGroup], len[kGroup];
@@ -532,60 +536,53 @@ __device__ __forceinline__ int coop_candidates(const Bufs& B, const DevParams& P
         for (int q = 0; q < kGroup; ++q) {
             start[q] = len[q] = 0;
             if (r0 + q >= runs) continue;
-            const int h0 = __ffs(left) - 1;
-            left &= left - 1;
-            const int rx = __shfl_sync(kFull, cx, h0), ry = __shfl_sync(kFull, cy, h0),
-                      rz = __shfl_sync(kFull, cz, h0);
+            const int3 cell3 = S.cell[r0 + q];
             if (lane < 27u) {   // lane t: bucket t of the walk
                 const int t = (int)lane;
                 const int x = t % 3 - 1, y = (t / 3) % 3 - 1, z = t / 9 - 1;
                 const uint2 cell = B.cells[P.table_base +
-                                           cell_hash_pow2((int)((uint32_t)rx + (uint32_t)x),
-                                                          (int)((uint32_t)ry + (uint32_t)y),
-                                                          (int)((uint32_t)rz + (uint32_t)z),
+                                           cell_hash_pow2((int)((uint32_t)cell3.x + (uint32_t)x),
+                                                          (int)((uint32_t)cell3.y + (uint32_t)y),
+                                                          (int)((uint32_t)cell3.z + (uint32_t)z),
                                                           P.T - 1u)];
                 start[q] = cell.x;
-                len[q] = cell.x != kEmpty ? min(cell.y - cell.x, kLong) : 0u;
+                len[q] = cell.x != kEmpty ? cell.y - cell.x : 0u;
             }
         }
 #pragma unroll
-        for (int q = 0; q < kGroup; q += 2) {
-            if (r0 + q >= runs) continue;
-            uint32_t both = len[q] | len[q + 1] << 16;   // two runs' sums in one
+        for (int q = 0; q < kGroup; ++q) {
+            const int r = r0 + q;
+            if (r >= runs) continue;
+            uint32_t incl = len[q];
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t v = __shfl_up_sync(kFull, both, d);
-                if (lane >= (uint32_t)d) both += v;
+                const uint32_t v = __shfl_up_sync(kFull, incl, d);
+                if (lane >= (uint32_t)d) incl += v;
             }
-            const uint32_t totals = __shfl_sync(kFull, both, 31);
-#pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                const int r = r0 + q + w;
-                if (r >= runs) continue;
-                const uint32_t l = len[q + w];
-                const uint32_t total = w ? totals >> 16 : totals & 0xFFFFu;
-                const uint32_t nonempty = __ballot_sync(kFull, l != 0);
-                const bool fits = total <= (uint32_t)kMaxSlabs * 32u;
-                if (l != 0 && fits) {
-                    const uint32_t incl = w ? both >> 16 : both & 0xFFFFu, excl = incl - l;
-                    const uint32_t slot = __popc(nonempty & lt_mask);
-                    S.first[r][slot] = start[q + w] - excl;
-                    atomicOr(&S.starts[r][excl >> 5], 1u << (excl & 31u));
-                    // words that begin after this bucket's first entry and not
-                    // after its last have slot + 1 starts before them
-                    for (uint32_t k = (excl >> 5) + 1; k <= incl >> 5 && k < kMaxSlabs; ++k)
-                        S.before[r][k] = (uint8_t)(slot + 1);
-                }
-                if (lane == 0) {
-                    S.total[r] = fits ? total : 0u;   // (a row is never empty)
-                    S.before[r][0] = 0;
-                }
+            const uint32_t total = __shfl_sync(kFull, incl, 31);
+            more |= total > from + kWindow;
+            // this lane's bucket within the window: places [a, b)
+            const uint32_t excl = incl - len[q];
+            const uint32_t a = max(excl, from) - from, b = min(incl, from + kWindow);
+            const bool in = max(excl, from) < b;
+            const uint32_t nonempty = __ballot_sync(kFull, in);
+            if (in) {
+                const uint32_t slot = __popc(nonempty & lt_mask), end = b - from;
+                S.first[r][slot] = start[q] - excl + from;
+                atomicOr(&S.starts[r][a >> 5], 1u << (a & 31u));
+                // words that begin after this bucket's first entry and not
+                // after its last have slot + 1 starts before them
+                for (uint32_t k = (a >> 5) + 1; k <= end >> 5 && k < kMaxSlabs; ++k)
+                    S.before[r][k] = (uint8_t)(slot + 1);
+            }
+            if (lane == 0) {
+                S.total[r] = total > from ? min(total - from, kWindow) : 0u;
+                S.before[r][0] = 0;
             }
         }
     }
     __syncwarp();
     const uint32_t my_total = live ? S.total[run] : 0u;
-    const int my_run = my_total ? run : -1;
     const uint32_t my_slabs = (my_total + 31u) >> 5;
     const uint32_t slabs = __reduce_max_sync(kFull, my_slabs);
     const float inv_h = P.inv_h;
@@ -648,7 +645,7 @@ __device__ __forceinline__ int coop_candidates(const Bufs& B, const DevParams& P
             __syncwarp();
         }
     }
-    return my_run;
+    return more;
 }
 
 // The candidates of a lane that passed the near test, in walk order.
@@ -707,29 +704,22 @@ __device__ __forceinline__ void density_alpha_particle(const Bufs& B, DensityScr
               pz = __shfl_up_sync(kFull, cz, 1);
     const bool head = live && (lane == 0 || cx != px || cy != py || cz != pz);
     const uint32_t heads = __ballot_sync(kFull, head);
-    const bool coop = __popc(heads) <= kCoopRuns && h > kCoopMinH && h < kCoopMaxH;
-    int my_run = -1;
-    uint32_t n1 = 0;
-    if (coop) {
-        my_run = coop_candidates(B, P, S, heads, live, cx, cy, cz, p4, n1);
-    } else if (live) {
-        walk(B, P, pi, [&](uint32_t j, f3, float) {
-            if (n1 < (uint32_t)kStage) S.cand[n1][lane] = j;
-            ++n1;
-        });
-    }
-    __syncwarp();
-    if (!live) return;
-
+    const int runs = __popc(heads);
+    const bool coop = runs <= kCoopRuns && h > kCoopMinH && h < kCoopMaxH;
     const uint32_t stride = B.n_total;
     DensityAcc a;
-    a.op = B.nbr + i;
-    const f3 vi = kDiv ? xyz(__ldg(kDiv == 1 ? velb(B, i) : vela(B, i))) : f3{0.0f, 0.0f, 0.0f};
+    // (the particle's velocity and next list slot are fetched again for every
+    // batch of pairs: kept through phase 1, they are registers it needs)
+    auto velocity = [&] {
+        return kDiv ? xyz(__ldg(kDiv == 1 ? velb(B, i) : vela(B, i))) : f3{0.0f, 0.0f, 0.0f};
+    };
     float4 vj = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     // n candidates in order, the next one's position on its way while this one's
     // terms are computed
     auto sums = [&](uint32_t n, auto&& next) {
         if (n == 0) return;
+        const f3 vi = velocity();
+        a.op = B.nbr + i + (size_t)min(a.cnt, kNbrCap) * stride;
         uint32_t j = next();
         f3 pj = neighbour_pos<kDiv>(B, j, vj);
         for (uint32_t k = 1; k <= n; ++k) {
@@ -746,34 +736,49 @@ __device__ __forceinline__ void density_alpha_particle(const Bufs& B, DensityScr
             density_term<kDiv>(a, m, P, kn, j0, rv, r2, stride, vi, v0);
         }
     };
-    if (my_run >= 0) {
-        RowWalk w(S, my_run, lane);
-        sums(n1, [&] { return w.next(S, my_run, lane); });
-    } else if (!coop && n1 <= (uint32_t)kStage) {
-        uint32_t k = 0;
-        sums(n1, [&] { return S.cand[k++][lane]; });
-    } else if (!coop) {
-        // more candidates than the scratch holds: kStage of them at a time
-        for (uint32_t from = 0; from < n1; from += kStage) {
-            uint32_t seen = 0;
-            walk(B, P, pi, [&](uint32_t j, f3, float) {
-                const uint32_t at = seen++ - from;
-                if (at < (uint32_t)kStage) S.cand[at][lane] = j;
-            });
-            const uint32_t n = min(n1 - from, (uint32_t)kStage);
+    uint32_t n1 = 0;
+    if (coop) {
+        const int run = __popc(heads & ((2u << lane) - 1u)) - 1;
+        if (head) {
+            S.cell[run] = make_int3(cx, cy, cz);
+            S.head[run] = p4;
+        }
+        __syncwarp();
+        bool more = true;
 #pragma unroll 1
-            for (uint32_t k = 0; k < n; ++k) {
-                const uint32_t j = S.cand[k][lane];
-                const f3 rv = sub(pi, neighbour_pos<kDiv>(B, j, vj));
-                density_term<kDiv>(a, m, P, kn, j, rv, dot(rv, rv), stride, vi, vj);
+        for (uint32_t from = 0; more; from += kWindow) {
+            more = coop_candidates(B, P, S, runs, run, live, p4, from, n1);
+            __syncwarp();
+            if (live && n1) {
+                RowWalk w(S, run, lane);
+                sums(n1, [&] { return w.next(S, run, lane); });
             }
+            __syncwarp();
         }
     } else {
-        walk(B, P, pi, [&](uint32_t j, f3 rv, float r2) {
-            if (kDiv) vj = __ldg(kDiv == 1 ? velb(B, j) : vela(B, j));
-            density_term<kDiv>(a, m, P, kn, j, rv, r2, stride, vi, vj);
-        });
+        if (live)
+            walk(B, P, pi, [&](uint32_t j, f3, float) {
+                if (n1 < (uint32_t)kStage) S.cand[n1][lane] = j;
+                ++n1;
+            });
+        __syncwarp();
+        if (n1 <= (uint32_t)kStage) {
+            uint32_t k = 0;
+            sums(n1, [&] { return S.cand[k++][lane]; });
+        } else {
+            // more candidates than the scratch holds: kStage of them at a time
+            for (uint32_t from = 0; from < n1; from += kStage) {
+                uint32_t seen = 0;
+                walk(B, P, pi, [&](uint32_t j, f3, float) {
+                    const uint32_t at = seen++ - from;
+                    if (at < (uint32_t)kStage) S.cand[at][lane] = j;
+                });
+                uint32_t k = 0;
+                sums(min(n1 - from, (uint32_t)kStage), [&] { return S.cand[k++][lane]; });
+            }
+        }
     }
+    if (!live) return;
     if (kDiv) B.src[i] = -a.div;   // divergence_source_term.comp:58-60
     B.rho[i] = a.density;
     // velocity_b.w carries m / rho (the factor viscosity applies to each
@@ -800,7 +805,7 @@ __device__ __forceinline__ void density_alpha_particle(const Bufs& B, DensityScr
         // the substep's density-source moments, as the re-sort gathered them
         const float4 m4 = L.mom_tmp[i];
         const float fm[kMoments] = {m4.x, m4.y, m4.z, m4.w, cr.z};
-        emit_features(B, L, P, i, s, 1, a.div, vi, fm);
+        emit_features(B, L, P, i, s, 1, a.div, velocity(), fm);
     }
 }
 

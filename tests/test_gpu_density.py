@@ -101,3 +101,51 @@ def test_particles_per_warp(oracle_mod, n):
         a, b = sim.data.download(f).view(np.uint32), orc.field(f).view(np.uint32)
         assert np.array_equal(a, b), f
     sim.close()
+
+
+def _row_of(total, h, seed, scattered=0):
+    """3^3 cells whose particles make the centre cell's row exactly `total` long,
+    and `scattered` particles in the cells around them."""
+    rng = np.random.default_rng(seed)
+    ijk = np.stack(np.meshgrid(*[np.arange(3)] * 3, indexing="ij"), -1).reshape(-1, 3) + 2
+    per = np.full(27, total // 27)
+    per[: total - per.sum()] += 1
+    rng.shuffle(per)
+    at = np.repeat(ijk, per, 0)
+    if scattered:
+        at = np.concatenate([at, rng.integers(0, 7, (scattered, 3))])
+    return ((at + rng.uniform(0.02, 0.98, at.shape)) * h).astype(np.float32)
+
+
+@pytest.mark.parametrize("mode", [_abi.FE_MODE_REFERENCE, _abi.FE_MODE_FIXED])
+@pytest.mark.parametrize("total", [383, 384, 385, 416, 767, 768, 769, 1153, 4000])
+def test_rows_of_several_windows(oracle_mod, total, mode):
+    """Rows that end at, before and after the 384 candidates of a window, buckets
+    that go on from one window to the next, and warps whose runs need different
+    numbers of windows."""
+    p = scene.dam_break_params((0, 0, 0), (1.3, 1.3, 1.3), mode=mode)
+    p.dt = 0.0002
+    pos = _row_of(total, 0.1, total, scattered=200)
+    sim, orc = Simulation(pos, p), oracle_mod.Oracle(p, pos)
+    for k in range(2):
+        sim.step(1)
+        orc.step(1)
+        for f in FIELDS:
+            a, b = sim.data.download(f).view(np.uint32), orc.field(f).view(np.uint32)
+            assert np.array_equal(a, b), (k, f)
+    sim.close()
+
+
+def test_rows_of_several_windows_with_32_particles_per_warp(oracle_mod):
+    """The same in a context large enough for whole warps."""
+    p = scene.dam_break_params((0, 0, 0), (4.0, 4.0, 4.0), mode=_abi.FE_MODE_FIXED)
+    p.dt = 0.0002
+    rest, _ = scene.lattice((1.2, 0, 1.2), (40, 39, 39), 0.025, 1000.0, 0.05, 0.04, 5)
+    pos = np.concatenate([_row_of(1000, 0.1, 7, scattered=300), rest])
+    sim, orc = Simulation(pos, p), oracle_mod.Oracle(p, pos)
+    sim.step(1)
+    orc.step(1)
+    for f in FIELDS:
+        a, b = sim.data.download(f).view(np.uint32), orc.field(f).view(np.uint32)
+        assert np.array_equal(a, b), f
+    sim.close()
