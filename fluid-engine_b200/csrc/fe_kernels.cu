@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(kBlock) k_refresh_pr(Bufs B) {
 // come with a denser fluid, a larger h, and buckets that cells share (12,000
 // particles at rest, 0.1 % of them with 385 to 392 candidates: 89 us when those
 // walked in one phase, 36 in windows).  1M particles in motion, ms, walked /
-// windows: h of 2.0 spacings 0.41 / 0.42, 2.42 1.62 / 0.73, 2.9 1.31 / 0.97.  Only
+// windows: h of 2.0 spacings 0.41 / 0.40, 2.42 1.62 / 0.71, 2.9 1.31 / 0.95.  Only
 // where every candidate is in range, thousands of particles on one spot, does the
 // test cost more than it saves (16k there: 5.7 / 7.1).
 constexpr int kStage = 44;
@@ -648,6 +648,47 @@ __device__ __forceinline__ bool coop_candidates(const Bufs& B, const DevParams& 
     return more;
 }
 
+// The per-lane form: the next in-range candidates of the lane's walk, at most
+// kStage, to S.cand; returns their number.  t: the bucket to go on with (27: none
+// left), next: the candidate in it (0: its first).
+__device__ __forceinline__ uint32_t lane_candidates(const Bufs& B, const DevParams& P,
+                                                    DensityScratch& S, f3 pi, int cx, int cy,
+                                                    int cz, uint32_t& t, uint32_t& next) {
+    const float h2 = P.h * P.h;
+    const int lane = lane_id();
+    uint32_t n = 0;
+#pragma unroll 1
+    for (uint32_t r = t / 3u; r < 9u; ++r) {   // three buckets' bounds in flight
+        const uint32_t y = (uint32_t)cy + r % 3u - 1u, z = (uint32_t)cz + r / 3u - 1u;
+        uint2 cell[3];
+#pragma unroll
+        for (uint32_t x = 0; x < 3u; ++x)
+            cell[x] = __ldg(B.cells + P.table_base +
+                            cell_hash_pow2((int)((uint32_t)cx + x - 1u), (int)y, (int)z, P.T - 1u));
+#pragma unroll
+        for (uint32_t x = 0; x < 3u; ++x) {
+            uint32_t j = cell[x].x, end = j == kEmpty ? 0u : cell[x].y;
+            if (3u * r + x < t) continue;
+            if (next) {
+                j = next;
+                next = 0;
+            }
+            for (; j < end; ++j) {
+                const f3 rv = sub(pi, xyz(__ldg(posb(B, j))));
+                if (dot(rv, rv) > h2) continue;
+                S.cand[n][lane] = j;
+                if (++n == (uint32_t)kStage) {
+                    t = 3u * r + x;
+                    next = j + 1;
+                    return n;
+                }
+            }
+        }
+    }
+    t = 27u;
+    return n;
+}
+
 // The candidates of a lane that passed the near test, in walk order.
 struct RowWalk {
     uint32_t sl = 0, bits = 0, starts = 0, before = 0;
@@ -761,21 +802,18 @@ __device__ __forceinline__ void density_alpha_particle(const Bufs& B, DensityScr
                 if (n1 < (uint32_t)kStage) S.cand[n1][lane] = j;
                 ++n1;
             });
-        __syncwarp();
-        if (n1 <= (uint32_t)kStage) {
+        // A lane with more than fit starts again, kStage at a time, going on with
+        // its walk where it left it.  (Walking from the start for every kStage of
+        // them took 118 ms beside cells of 4000 particles, this 16; a walk that
+        // stops at kStage from the beginning is slower for the lanes with fewer.)
+        uint32_t t = n1 > (uint32_t)kStage ? 0u : 27u, next = 0;
+        if (t == 0u) n1 = 0;
+        for (;;) {
+            __syncwarp();
             uint32_t k = 0;
             sums(n1, [&] { return S.cand[k++][lane]; });
-        } else {
-            // more candidates than the scratch holds: kStage of them at a time
-            for (uint32_t from = 0; from < n1; from += kStage) {
-                uint32_t seen = 0;
-                walk(B, P, pi, [&](uint32_t j, f3, float) {
-                    const uint32_t at = seen++ - from;
-                    if (at < (uint32_t)kStage) S.cand[at][lane] = j;
-                });
-                uint32_t k = 0;
-                sums(min(n1 - from, (uint32_t)kStage), [&] { return S.cand[k++][lane]; });
-            }
+            if (!__any_sync(kFull, t < 27u)) break;
+            n1 = lane_candidates(B, P, S, pi, cx, cy, cz, t, next);
         }
     }
     if (!live) return;

@@ -149,3 +149,25 @@ def test_rows_of_several_windows_with_32_particles_per_warp(oracle_mod):
         a, b = sim.data.download(f).view(np.uint32), orc.field(f).view(np.uint32)
         assert np.array_equal(a, b), f
     sim.close()
+
+
+@pytest.mark.parametrize("mode", [_abi.FE_MODE_REFERENCE, _abi.FE_MODE_FIXED])
+def test_many_runs_beside_crowded_cells(oracle_mod, mode):
+    """Warps with a cell per particle, some of whose particles have one, two or
+    more stages of candidates in a crowded cell beside theirs."""
+    p = scene.dam_break_params((0, 0, 0), (4.0, 4.0, 4.0), mode=mode)
+    p.dt = 0.0002
+    pos = [_cells(1, 38, 0.1, 11)]
+    rng = np.random.default_rng(12)
+    for m in (30, 44, 45, 60, 90, 150, 400):
+        for at in rng.integers(2, 38, (5, 3)):
+            pos.append((at + rng.uniform(0.02, 0.98, (m, 3))) * 0.1)
+    pos = np.concatenate(pos).astype(np.float32)
+    assert len(pos) > 56832          # 32 particles per warp
+    sim, orc = Simulation(pos, p), oracle_mod.Oracle(p, pos)
+    sim.step(1)
+    orc.step(1)
+    for f in FIELDS:
+        a, b = sim.data.download(f).view(np.uint32), orc.field(f).view(np.uint32)
+        assert np.array_equal(a, b), f
+    sim.close()
