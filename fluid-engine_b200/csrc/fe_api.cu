@@ -385,8 +385,9 @@ struct fe_ctx {
     int splat_res[3] = {0, 0, 0};  // resolution of the last splat
     SplatWeights splat_weights{};
     bool splat_ready = false;
-    uint32_t* splat_hist = nullptr;    // particles per centre voxel
+    uint32_t* splat_hist = nullptr;    // particles per centre voxel, then the grid's bits
     size_t splat_hist_cap = 0;
+    uint32_t* splat_bits_at = nullptr; // in splat_hist, of the last splat
 
     // raymarched image and its sky
     float4* sky = nullptr;
@@ -395,9 +396,8 @@ struct fe_ctx {
     float4* image = nullptr;
     size_t image_cap = 0;
     int image_w = 0, image_h = 0;
-    uint32_t* ray_bits = nullptr;   // raymarch scratch, by grid size
-    uint8_t* ray_coarse = nullptr;
-    size_t ray_bits_cap = 0, ray_coarse_cap = 0;
+    uint8_t* ray_coarse = nullptr;  // raymarch scratch, by grid size
+    size_t ray_coarse_cap = 0;
 
     // fe_download_async: two device snapshots, the copy stream, and which
     // ticket each snapshot slot serves (0: none)
@@ -976,7 +976,7 @@ size_t field_bytes(const fe_ctx* c, fe_field f, void** dptr, size_t* elem, size_
         case FE_FIELD_GRID_START: *dptr = c->B.cells; *elem = 4; *pitch = 8; n = c->T; break;
         case FE_FIELD_STATS: *dptr = c->B.S; *elem = 4; n = 3; break;
         case FE_FIELD_DENSITY_GRID:
-            if (!c->splat_grid) {
+            if (!c->splat_bits_at) {
                 set_error("no density grid yet: call fe_density_splat first");
                 return 0;
             }
@@ -1548,6 +1548,10 @@ fe_status fe_upload(fe_ctx* c, fe_field f, const void* src, size_t bytes) {
         FE_CUDA(cudaMemcpy2DAsync(c->B.pa, 32, src, 16, 16, c->n, cudaMemcpyHostToDevice,
                                   c->stream));
     }
+    if (f == FE_FIELD_DENSITY_GRID)   // and what the water pass keeps of the grid
+        FE_CUDA(splat_bits(c->splat_grid,
+                           make_int3(c->splat_res[0], c->splat_res[1], c->splat_res[2]),
+                           c->splat_bits_at, c->stream));
     // pos_b.w caches p / rho^2 for pressure_force, the velocities' w rho.
     if (f == FE_FIELD_PRESSURE || f == FE_FIELD_DENSITY || f == FE_FIELD_POSITION_B ||
         f == FE_FIELD_VELOCITY_A || f == FE_FIELD_VELOCITY_B)
@@ -1764,24 +1768,27 @@ fe_status fe_density_splat(fe_ctx* c) {
             }
         c->splat_ready = true;
     }
-    c->splat_res[0] = rx;
-    c->splat_res[1] = ry;
-    c->splat_res[2] = rz;
     // Counts per centre voxel, then the convolution with the weights
     // (fe_splat.cu).
     const int3 res = make_int3(rx, ry, rz);
     const size_t hist_n = (size_t)(rx + 1) * (ry + 1) * (rz + 1);
-    if (hist_n > c->splat_hist_cap) {
-        fe_status st0 = dev_alloc(c, &c->splat_hist, hist_n);
+    const size_t hist_words = hist_n + splat_bit_words(res);
+    if (hist_words > c->splat_hist_cap) {
+        fe_status st0 = dev_alloc(c, &c->splat_hist, hist_words);
         if (st0 != FE_OK) return st0;
-        c->splat_hist_cap = hist_n;
+        c->splat_hist_cap = hist_words;
     }
+    c->splat_res[0] = rx;
+    c->splat_res[1] = ry;
+    c->splat_res[2] = rz;
+    c->splat_bits_at = c->splat_hist + hist_n;
     const float3 b0 = make_float3(p.box_min[0], p.box_min[1], p.box_min[2]);
     const float3 b1 = make_float3(p.box_max[0], p.box_max[1], p.box_max[2]);
     FE_CUDA(cudaMemsetAsync(c->splat_grid, 0, voxels * 4, c->stream));
-    FE_CUDA(cudaMemsetAsync(c->splat_hist, 0, hist_n * 4, c->stream));
+    FE_CUDA(cudaMemsetAsync(c->splat_hist, 0, hist_words * 4, c->stream));
     FE_CUDA(splat_histogram(c->B.pos_a, c->n, b0, b1, res, c->splat_hist, c->stream));
-    FE_CUDA(splat_convolve(c->splat_hist, res, c->splat_weights, c->splat_grid, c->stream));
+    FE_CUDA(splat_convolve(c->splat_hist, res, c->splat_weights, c->splat_grid, c->splat_bits_at,
+                           c->stream));
     return FE_OK;
 }
 
@@ -1818,7 +1825,7 @@ fe_status fe_raymarch(fe_ctx* c, const fe_camera* cam) {
         set_error("NULL argument");
         return FE_ERR_INVALID_ARGUMENT;
     }
-    if (!c->splat_grid) {
+    if (!c->splat_bits_at) {
         set_error("fe_raymarch: no density grid yet (fe_density_splat first)");
         return FE_ERR_INVALID_ARGUMENT;
     }
@@ -1845,17 +1852,13 @@ fe_status fe_raymarch(fe_ctx* c, const fe_camera* cam) {
     RaymarchArgs a;
     a.grid = c->splat_grid;
     a.res = make_int3(c->splat_res[0], c->splat_res[1], c->splat_res[2]);
-    const size_t bit_words = raymarch_bit_words(a.res), coarse_bytes = raymarch_coarse_bytes(a.res);
-    fe_status st;
-    if (bit_words > c->ray_bits_cap) {
-        if ((st = dev_alloc(c, &c->ray_bits, bit_words)) != FE_OK) return st;
-        c->ray_bits_cap = bit_words;
-    }
+    const size_t coarse_bytes = raymarch_coarse_bytes(a.res);
     if (coarse_bytes > c->ray_coarse_cap) {
-        if ((st = dev_alloc(c, &c->ray_coarse, coarse_bytes)) != FE_OK) return st;
+        fe_status st = dev_alloc(c, &c->ray_coarse, coarse_bytes);
+        if (st != FE_OK) return st;
         c->ray_coarse_cap = coarse_bytes;
     }
-    a.bits = c->ray_bits;
+    a.bits = c->splat_bits_at;
     a.coarse = c->ray_coarse;
     a.sky = c->sky;
     a.sky_w = c->sky_w;

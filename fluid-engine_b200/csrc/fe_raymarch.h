@@ -16,13 +16,12 @@ struct RaymarchArgs {
     float3 cam;
     float3 box_min, box_max;   // sim box (the water model's bounds)
     int width, height;
-    uint32_t* bits;    // scratch: which texels are above the offset
-    uint8_t* coarse;   // scratch: what holds for every texel around 4^3 voxels
+    const uint32_t* bits;      // the grid's bits (fe_splat.h)
+    uint8_t* coarse;           // scratch: what holds for every texel around 4^3 voxels
     float4* out;               // [height][width] RGBA, alpha 0 where the shader discards
 };
 
-// Sizes of RaymarchArgs::bits (words) and ::coarse (bytes) for a grid.
-size_t raymarch_bit_words(int3 res);
+// Bytes of RaymarchArgs::coarse for a grid.
 size_t raymarch_coarse_bytes(int3 res);
 
 cudaError_t raymarch(const RaymarchArgs& a, cudaStream_t stream);

@@ -157,9 +157,12 @@ __global__ void __launch_bounds__(256) k_splat_hist(const float4* __restrict__ p
 }
 
 // One block per output tile; a window without particles leaves the grid at 0.
+// The bits of kSurfaceCount go out with the grid: the water pass would read 32
+// times as much to find them (512^3 voxels: 0.48 ms).
 __global__ void __launch_bounds__(kThreads, 2) k_splat_conv(const uint32_t* __restrict__ hist,
                                                             int3 res, SplatWeights W,
-                                                            uint32_t* __restrict__ grid) {
+                                                            uint32_t* __restrict__ grid,
+                                                            uint32_t* __restrict__ bits) {
     extern __shared__ __align__(16) uint32_t win[];  // [kWinZ][kWinY][kRow]
     const int tdx = (res.x + kTileX - 1) / kTileX, tdy = (res.y + kTileY - 1) / kTileY;
     const int tx = blockIdx.x % tdx, ty = (blockIdx.x / tdx) % tdy, tz = blockIdx.x / (tdx * tdy);
@@ -184,11 +187,31 @@ __global__ void __launch_bounds__(kThreads, 2) k_splat_conv(const uint32_t* __re
     add_classes<kReach>(acc, at, 0, kNarrow, W);
     add_classes<4>(acc, at, kNarrow, kClassTable.n, W);
     const int x = tx * kTileX + lx, y = ty * kTileY + ly, z = tz * kTileZ + lz;
+    // a row of the tile is one word of bits, four threads' bytes
+    static_assert(kTileX == 32 && kPer == 8, "a tile row per word");
+    uint32_t word = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i)
+        word |= (x + i < res.x && acc[i] > kSurfaceCount ? 1u : 0u) << (lx + i);
+    word |= __shfl_xor_sync(0xFFFFFFFFu, word, 1);
+    word |= __shfl_xor_sync(0xFFFFFFFFu, word, 2);
     if (y >= res.y || z >= res.z) return;
+    if (lx == 0) bits[((size_t)z * res.y + y) * tdx + tx] = word;
     uint32_t* out = grid + ((size_t)z * res.y + y) * res.x + x;
 #pragma unroll
     for (int i = 0; i < kPer; ++i)
         if (x + i < res.x) out[i] = acc[i];
+}
+
+__global__ void __launch_bounds__(256) k_splat_bits(const uint32_t* __restrict__ grid, int3 res,
+                                                    uint32_t* __restrict__ bits) {
+    const int words = (res.x + 31) / 32;
+    const size_t w = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (w >= (size_t)words * res.y * res.z) return;
+    const int x = (int)(w % words) * 32 + (int)(threadIdx.x & 31u);
+    const bool above = x < res.x && __ldg(grid + w / words * res.x + x) > kSurfaceCount;
+    const uint32_t b = __ballot_sync(0xFFFFFFFFu, above);
+    if ((threadIdx.x & 31u) == 0) bits[w] = b;
 }
 
 }  // namespace
@@ -201,13 +224,19 @@ cudaError_t splat_histogram(const float4* pos, uint32_t n, float3 box_min, float
 }
 
 cudaError_t splat_convolve(const uint32_t* hist, int3 res, const SplatWeights& w, uint32_t* grid,
-                           cudaStream_t stream) {
+                           uint32_t* bits, cudaStream_t stream) {
     const int tdx = (res.x + kTileX - 1) / kTileX, tdy = (res.y + kTileY - 1) / kTileY,
               tdz = (res.z + kTileZ - 1) / kTileZ;
     cudaError_t e = cudaFuncSetAttribute(k_splat_conv, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kWinBytes);
     if (e != cudaSuccess) return e;
-    k_splat_conv<<<tdx * tdy * tdz, kThreads, kWinBytes, stream>>>(hist, res, w, grid);
+    k_splat_conv<<<tdx * tdy * tdz, kThreads, kWinBytes, stream>>>(hist, res, w, grid, bits);
+    return cudaGetLastError();
+}
+
+cudaError_t splat_bits(const uint32_t* grid, int3 res, uint32_t* bits, cudaStream_t stream) {
+    const size_t words = splat_bit_words(res);
+    k_splat_bits<<<(unsigned)((words + 7) / 8), 256, 0, stream>>>(grid, res, bits);
     return cudaGetLastError();
 }
 
