@@ -763,16 +763,20 @@ fe_status rec_solve_resident_many(fe_ctx* c, Recorder& R, int which) {
 // all) and 64 of 4k to 262k: a particle per thread up to 18.9k particles, chunks
 // up to 56.8k 1.25 and 13.6; up to 9.5k and 37.9k, as here, 0.97 and 10.3;
 // iterated throughout - and 10.1.
-// Several scenes in one context, which are what one has instead of several
-// contexts: 256 scenes of 1k to 8k particles 3.2 -> 1.9 ms.
+// Batches of scenes that iterate a fixed number of times go by the same line
+// (resident / iterated, us per frame of one context / two / four / eight):
+//   17k 195/106/65/49 and 257/146/87/65, 38k 218/134/102/98 and 288/180/112/85,
+//   50k 237/151/137/142 and 316/195/131/110, 97k 300/279/280/289 and
+//   372/262/202/197, 153k 536/555/576/589 and 552/374/312/314, 590k
+//   1359/1409/1455/1473 and 1396/1238/1203/1220, 944k 2027/2093/2155/2158 and
+//   2135/1968/1937/1984.
 constexpr uint32_t kResidentParticles = 148 * kResidentThreads;   // a block per SM
 constexpr uint32_t kStridedParticles = 148 * kBlock;              // a chunk per SM
-constexpr uint32_t kStridedBatchParticles = 1u << 20;
 fe_status choose_resident(fe_ctx* c) {
     int cooperative = 0, blocks = 0;
     FE_CUDA(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, c->device));
     if (!cooperative) return FE_OK;
-    if (c->n <= (c->B.n_scenes == 1 ? kStridedParticles : kStridedBatchParticles)) {
+    if (c->n <= kStridedParticles) {
         FE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_solve_resident_many,
                                                               kBlock, 0));
         c->resident_many_blocks =

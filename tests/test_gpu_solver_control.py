@@ -200,3 +200,30 @@ def test_batch_resident_solve_past_the_neighbour_list(oracle_mod):
                 x = batch.data.scene(batch.data.download(f), s)
                 assert np.array_equal(x.view(np.uint32), orc.field(f).view(np.uint32)), (s, f)
     batch.close()
+
+
+@pytest.mark.parametrize("last", [9000, 10000])
+def test_batch_solves_around_their_line(last):
+    """Fixed-iteration batches below and above the size up to which their solves
+    are one kernel: each scene as it is alone."""
+    rng = np.random.default_rng(last)
+    pos, params = [], []
+    for k, n in enumerate((14000, 14400, last)):       # 37400 and 38400 particles
+        a, _ = scene.lattice((0, 0, 0), (25, 24, 24), 0.025, 1000.0, 0.05, 0.03, k)
+        pos.append(a[:n])
+        p = scene.dam_break_params((0, 0, 0), (2.0, 2.0, 2.0), mode=_abi.FE_MODE_FIXED)
+        p.density_solver_iterations, p.divergence_solver_iterations = 3 + 2 * k, 4 - k
+        params.append(p)
+    vel = [rng.normal(0, 0.3, a.shape).astype(np.float32) for a in pos]
+    batch = BatchSimulation(pos, params, scene_velocities=vel)
+    batch.step(2)
+    for s, (a, p, v) in enumerate(zip(pos, params, vel)):
+        st = batch.data.read_scene_stats(s)
+        assert (st.density_iterations, st.divergence_iterations) == (3 + 2 * s, 4 - s)
+        one = Simulation(a, p, velocities=v)
+        one.step(2)
+        for f in FIELDS:
+            x = batch.data.scene(batch.data.download(f), s)
+            assert np.array_equal(x.view(np.uint32), one.data.download(f).view(np.uint32)), (s, f)
+        one.close()
+    batch.close()
