@@ -238,8 +238,9 @@ def barrier(world: int):
         dist.barrier()
 
 
-def launches_per_frame(stats, n: int, learned: bool = False) -> float:
-    """Kernels of one single-scene frame with one substep (the frame graph's)."""
+def launches_per_frame(stats, n: int, sms: int, learned: bool = False) -> float:
+    """Kernels of one single-scene frame with one substep (the frame graph's) on
+    a device of `sms` multiprocessors."""
     # neighbour search: count, scan, scatter, reorder
     search = 4
     # prologue, viscosity, density source, integration, density/alpha (with the
@@ -250,7 +251,7 @@ def launches_per_frame(stats, n: int, learned: bool = False) -> float:
     # (features, after-solve bookkeeping and the carry permutation ride in the
     # source, integration and reorder passes)
     start = 2 if learned else 1
-    if n <= 148 * 256:
+    if n <= sms * 256:      # a chunk of particles per multiprocessor
         solves = 2          # each solve one resident kernel
     else:
         # begin (of the plain density solve the first iteration) and end of
@@ -387,7 +388,8 @@ def measure_arm(args, w, params, model, world, local, build="parity"):
             lib.fe_density_alpha(h)
     lib.fe_synchronize(h)
     avg = type("S", (), {"density_iterations": iters_d, "divergence_iterations": iters_v})
-    launches = launches_per_frame(avg, n, model is not None) * args.steps
+    sms = torch.cuda.get_device_properties(local).multi_processor_count
+    launches = launches_per_frame(avg, n, sms, model is not None) * args.steps
     sim.close()
     return {"n": n, "dev_ms": dev_ms_max, "value": n * args.steps * world / (dev_ms_max / 1e3),
             "e2e": n * args.steps * world / e2e_s, "iters": (iters_d, iters_v),

@@ -423,7 +423,7 @@ struct fe_ctx {
     // neighbour kernels, per FE_NBR_* group: threads per block, persistent
     uint32_t nbr_threads[FE_NBR_GROUPS] = {256, 256, 256, 256};
     uint32_t nbr_persistent[FE_NBR_GROUPS] = {0, 0, 0, 0};
-    int num_sms = 148;
+    int num_sms = 1;   // of the device; the sizes where shapes change go by it
 
     bool learned() const { return params[0].warm_start == FE_WARM_LEARNED && model != nullptr; }
     bool carries() const { return L.carry != nullptr && (learned() || capture); }
@@ -502,8 +502,7 @@ auto pick(void (*k128)(KArgs...), void (*k256)(KArgs...), void (*k512)(KArgs...)
 // 7.9/7.0, 8.6/8.3; 25k 10.6/9.7, 8.1/7.4, 8.9/9.0; 50k 13.4/12.2, 9.3/8.8,
 // 11.4/11.2 with whole frames slower (347/390); 80k 15.4/19.1, 10.3/12.6,
 // 14.5/17.0.
-constexpr uint32_t kFewParticles = 148 * 128;
-bool few(const fe_ctx* c) { return c->n <= kFewParticles; }
+bool few(const fe_ctx* c) { return c->n <= c->num_sms * 128u; }
 #define NBR_KERNEL(name, g)               \
     (few(c) ? name<kFewThreads, false>    \
             : NBR_KERNEL_P(name, c->nbr_threads[g], c->nbr_persistent[g]))
@@ -573,12 +572,11 @@ fe_status rec_nbr(fe_ctx* c, Recorder& R, int g, void (*func)(KArgs...), Args...
 // again, else 32.  Times in a graph of launches (us, 8 / 16 / 32 per warp, a
 // fall after 40 frames): 4.8k particles 28/43/58, 25k 43/60/65, 50k 72/63/68,
 // 80k 99/78/70, 131k 152/112/80.
-constexpr uint32_t kLanes8Particles = 148 * 32 * 8;
-constexpr uint32_t kLanes16Particles = 148 * 32 * 12;
 template <class... KArgs, class... Args>
 fe_status rec_density(fe_ctx* c, Recorder& R, void (*k8)(KArgs...), void (*k16)(KArgs...),
                       void (*k32)(KArgs...), Args... args) {
-    const uint32_t lanes = c->n <= kLanes8Particles ? 8u : c->n <= kLanes16Particles ? 16u : 32u;
+    const uint32_t warps = c->num_sms * 32u;
+    const uint32_t lanes = c->n <= warps * 8u ? 8u : c->n <= warps * 12u ? 16u : 32u;
     const uint32_t blocks = c->B.n_chunks * (kBlock / lanes) / (kFewThreads / 32);
     REC(R.k(lanes == 8 ? k8 : lanes == 16 ? k16 : k32, dim3(blocks), dim3(kFewThreads), args...));
     return FE_OK;
@@ -658,8 +656,8 @@ fe_status rec_neighbor_search(fe_ctx* c, Recorder& R, bool take = true) {
     } else {
         REC(R.k(k_hash, chunk_grid(c), dim3(kBlock), B));
         REC(bitonic_sort(R.sort_launch(), B.keys, B.vals, c->T));
-        REC(R.k(k_fill_cells, dim3(std::min<uint32_t>((c->T + 255) / 256, 148 * 8)), dim3(256),
-                B.cells, (size_t)c->T));
+        REC(R.k(k_fill_cells, dim3(std::min<uint32_t>((c->T + 255) / 256, c->num_sms * 8u)),
+                dim3(256), B.cells, (size_t)c->T));
         REC(R.k(k_offsets, flat_grid(c->n), dim3(kBlock), B));
         if (c->carries())
             REC(R.k(k_reorder_carry, flat_grid(c->n), dim3(kBlock), B, fixed, c->L));
@@ -770,19 +768,19 @@ fe_status rec_solve_resident_many(fe_ctx* c, Recorder& R, int which) {
 //   372/262/202/197, 153k 536/555/576/589 and 552/374/312/314, 590k
 //   1359/1409/1455/1473 and 1396/1238/1203/1220, 944k 2027/2093/2155/2158 and
 //   2135/1968/1937/1984.
-constexpr uint32_t kResidentParticles = 148 * kResidentThreads;   // a block per SM
-constexpr uint32_t kStridedParticles = 148 * kBlock;              // a chunk per SM
 fe_status choose_resident(fe_ctx* c) {
+    const uint32_t resident_particles = c->num_sms * kResidentThreads,   // a block per SM
+                   strided_particles = c->num_sms * kBlock;              // a chunk per SM
     int cooperative = 0, blocks = 0;
     FE_CUDA(cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, c->device));
     if (!cooperative) return FE_OK;
-    if (c->n <= kStridedParticles) {
+    if (c->n <= strided_particles) {
         FE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_solve_resident_many,
                                                               kBlock, 0));
         c->resident_many_blocks =
             std::min<uint32_t>(c->B.n_chunks, (uint32_t)(blocks * c->num_sms));
     }
-    if (c->B.n_scenes != 1 || c->n > kResidentParticles) return FE_OK;
+    if (c->B.n_scenes != 1 || c->n > resident_particles) return FE_OK;
     FE_CUDA(cudaFuncSetAttribute(k_solve_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kResidentSmem));
     FE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_solve_resident,
@@ -1685,7 +1683,7 @@ fe_status fe_download_wait(fe_ctx* c, uint64_t ticket) {
 // kernels' blocks fit beside the running ones.  Ten harness substeps of 1.4k
 // particles 2300 -> 1861 us, 4.8k 2754 -> 2529; 16k 2949 / 3001, as the waiting
 // blocks then take places.
-constexpr uint32_t kEarlyParticles = 148 * 64;
+bool early(const fe_ctx* c) { return c->n <= c->num_sms * 64u; }
 
 #define FE_STAGE(name, body)                                 \
     fe_status name(fe_ctx* c) {                              \
@@ -1693,7 +1691,7 @@ constexpr uint32_t kEarlyParticles = 148 * 64;
         fe_status s_ = need_prepared(c, #name);              \
         if (s_ != FE_OK) return s_;                          \
         Recorder R = eager(c);                               \
-        R.early = c->n <= kEarlyParticles;                   \
+        R.early = early(c);                   \
         body;                                                \
     }
 
@@ -2419,11 +2417,9 @@ fe_status fe_autotune(fe_ctx* c, fe_tune_report* report) {
     fill_radix_report(&r, ms);
     int ctas = c->mlp_ctas;
     if (c->model && c->L.xb && c->L.out) {
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
         float mms[kMlpCtaCandidates] = {};
         e = tune_mlp(c->stream, c->model->params(), static_cast<const __nv_bfloat16*>(c->L.xb),
-                     c->L.out, c->n, &c->B.G->flags, sms, 7, &ctas, mms);
+                     c->L.out, c->n, &c->B.G->flags, c->num_sms, 7, &ctas, mms);
         if (e != cudaSuccess) {
             set_error("network tuning: %s", cudaGetErrorString(e));
             return FE_ERR_CUDA;

@@ -129,7 +129,7 @@ __device__ __forceinline__ uint2 ld_list(const uint2* p, uint64_t pol) {
 // entries at a time, all their loads issued before the arithmetic, which runs
 // strictly in list order.
 // kAhead: also the next batch's list words are loaded before this batch's
-// gathers are used.  The shape for few particles (see kFewParticles), where a
+// gathers are used.  The shape for few particles (see few() in fe_api.cu), where a
 // pass is one chain of load latencies per thread and nothing else hides them;
 // with many particles the passes are bound by the gathers' throughput and the
 // registers cost more than the order gains.
