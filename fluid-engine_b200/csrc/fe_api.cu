@@ -2819,19 +2819,36 @@ FE_API void fe_debug_fail_allocation(uint32_t k) { g_fail_countdown.store(k); }
 
 FE_API void fe_debug_poison_allocations(int on) { g_poison.store(on ? 1 : 0); }
 
-FE_API fe_status fe_debug_bounded_wait(int device, uint32_t limit, uint32_t* flags) {
-    if (!flags || limit == 0) {
-        set_error("fe_debug_bounded_wait needs flags and a non-zero limit");
+FE_API fe_status fe_debug_bounded_wait_in(int device, uint32_t wait, uint32_t limit,
+                                          uint32_t* flags) {
+    if (!flags || limit == 0 || wait > FE_WAIT_SOLVE) {
+        set_error("fe_debug_bounded_wait needs one of the waits, flags and a non-zero limit");
         return FE_ERR_INVALID_ARGUMENT;
     }
     *flags = 0;
     FE_CUDA(cudaSetDevice(device));
-    FE_CUDA(lookback_wait_selftest((int)std::min<uint32_t>(limit, 1u << 30), flags));
+    const int polls = (int)std::min<uint32_t>(limit, 1u << 30);
+    uint32_t* d = nullptr;   // the word waited for (8 bytes), the flags
+    FE_CUDA(cudaMalloc(&d, 16));
+    cudaError_t e = cudaMemset(d, 0, 16);
+    if (e == cudaSuccess)
+        e = wait == FE_WAIT_SORT ? lookback_wait_on(d, d + 2, polls, nullptr)
+            : wait == FE_WAIT_SEARCH
+                ? scan_wait_on(reinterpret_cast<unsigned long long*>(d), d + 2, polls, nullptr)
+                : grid_barrier_wait_on(d, d + 2, polls, nullptr);
+    if (e == cudaSuccess) e = cudaMemcpy(flags, d + 2, 4, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    FE_CUDA(e);
     if (*flags & 0x4u) {
-        set_error("a bounded device wait timed out (look-back)");
+        set_error("a bounded device wait timed out (%s)",
+                  wait == FE_WAIT_SOLVE ? "grid barrier" : "look-back");
         return FE_ERR_TIMEOUT;
     }
     return FE_OK;
+}
+
+FE_API fe_status fe_debug_bounded_wait(int device, uint32_t limit, uint32_t* flags) {
+    return fe_debug_bounded_wait_in(device, FE_WAIT_SORT, limit, flags);
 }
 
 }  // extern "C"

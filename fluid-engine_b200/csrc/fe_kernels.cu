@@ -173,6 +173,45 @@ __global__ void __launch_bounds__(kBlock) k_cell_count(Bufs B, CellSort C) {
 // to its state, so nothing has to be cleared between searches; the counters
 // are left at zero for the next one.
 constexpr unsigned long long kScanSum = 1ull << 32, kScanPrefix = 2ull << 32;
+
+// The sum of the tiles before `tile` of this launch: 32 status words at a time,
+// nearest last, until one holds a whole prefix.  A word that has not come within
+// `limit` looks raises the flag and ends the wait.  One warp.
+__device__ __forceinline__ uint32_t scan_look_back(const volatile unsigned long long* st, int tile,
+                                                   unsigned long long epoch, int limit,
+                                                   uint32_t* flags) {
+    const int lane = lane_id();
+    uint32_t base = 0;
+    int spins = 0;
+    for (int last = tile - 1; last >= 0;) {
+        const int pred = last - lane;
+        unsigned long long v = epoch | kScanPrefix;   // before tile 0: 0
+        if (pred >= 0) v = st[pred];
+        const bool ready = (v >> 34) == (epoch >> 34);
+        const uint32_t not_ready = __ballot_sync(kFull, !ready);
+        const uint32_t whole = __ballot_sync(kFull, ready && (v & kScanPrefix));
+        // usable: the words up to the nearest whole prefix, or up to the
+        // first one that is not there yet
+        const uint32_t stop = whole ? __ffs(whole) : 33u;           // count to take
+        const uint32_t gap = not_ready ? __ffs(not_ready) - 1u : 32u;
+        const uint32_t take = min(stop, gap);
+        uint32_t part = (uint32_t)lane < take ? (uint32_t)v : 0u;
+#pragma unroll
+        for (int m = 16; m >= 1; m >>= 1) part += __shfl_xor_sync(kFull, part, m);
+        base += part;
+        if (stop <= gap) break;
+        last -= (int)take;
+        if (take == 0) {
+            if (++spins > limit) {
+                if (lane == 0) atomicOr(flags, 0x4u);
+                break;
+            }
+            __nanosleep(32);
+        }
+    }
+    return base;
+}
+
 // A thread owns 8 slots, 32 bytes of counters and 64 of bounds, so every access
 // is to whole sectors (16 slots a thread: 15.7 us at 2^20 slots; 8: 9 us).
 __global__ void __launch_bounds__(kScanThreads) k_cell_scan(Bufs B, CellSort C) {
@@ -227,41 +266,13 @@ __global__ void __launch_bounds__(kScanThreads) k_cell_scan(Bufs B, CellSort C) 
         }
         if (lane < kWarps) s_warp[lane] = total - w;
         total = __shfl_sync(kFull, total, 31);
-        // this tile's sum, then the sums of the tiles before it: 32 status
-        // words at a time, nearest last, until one holds a whole prefix
+        // this tile's sum, then the sums of the tiles before it
         volatile unsigned long long* st = C.status;
         if (lane == 0) {
             st[tile] = epoch | (tile == 0 ? kScanPrefix : kScanSum) | total;
         }
-        uint32_t base = 0;
-        int pred = (int)tile - 1 - lane;
-        int spins = 0;
-        bool ok = true;
-        for (int last = (int)tile - 1; ok && last >= 0;) {
-            pred = last - lane;
-            unsigned long long v = epoch | kScanPrefix;   // before tile 0: 0
-            if (pred >= 0) v = st[pred];
-            const bool ready = (v >> 34) == (epoch >> 34);
-            const uint32_t not_ready = __ballot_sync(kFull, !ready);
-            const uint32_t whole = __ballot_sync(kFull, ready && (v & kScanPrefix));
-            // usable: the words up to the nearest whole prefix, or up to the
-            // first one that is not there yet
-            const uint32_t stop = whole ? __ffs(whole) : 33u;           // count to take
-            const uint32_t gap = not_ready ? __ffs(not_ready) - 1u : 32u;
-            const uint32_t take = min(stop, gap);
-            uint32_t part = (uint32_t)lane < take ? (uint32_t)v : 0u;
-#pragma unroll
-            for (int m = 16; m >= 1; m >>= 1) part += __shfl_xor_sync(kFull, part, m);
-            base += part;
-            if (stop <= gap) break;
-            last -= (int)take;
-            if (take == 0) {
-                if (++spins > kScanSpins) ok = false;
-                __nanosleep(32);
-            }
-        }
+        const uint32_t base = scan_look_back(st, (int)tile, epoch, kScanSpins, &B.G->flags);
         if (lane == 0) {
-            if (!ok) atomicOr(&B.G->flags, 0x4u);
             if (tile) st[tile] = epoch | kScanPrefix | (unsigned long long)(base + total);
             s_base = base;
         }
@@ -288,6 +299,16 @@ __global__ void __launch_bounds__(kScanThreads) k_cell_scan(Bufs B, CellSort C) 
         for (int q = 0; q < kPer; ++q)
             if (k0 + q < B.T_total) B.cells[k0 + q] = cell[q];
     }
+}
+
+// Waits for the tile before tile 1, which nothing publishes.
+__global__ void k_scan_selftest(const unsigned long long* status, uint32_t* flags, int limit) {
+    scan_look_back(status, 1, 1ull << 34, limit, flags);
+}
+cudaError_t scan_wait_on(const unsigned long long* status, uint32_t* flags, int limit,
+                         cudaStream_t stream) {
+    k_scan_selftest<<<1, 32, 0, stream>>>(status, flags, limit < kScanSpins ? limit : kScanSpins);
+    return cudaGetLastError();
 }
 
 __global__ void __launch_bounds__(kBlock) k_cell_scatter(Bufs B, CellSort C) {

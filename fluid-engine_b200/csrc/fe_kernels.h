@@ -76,4 +76,11 @@ __global__ void k_stats_snapshot(Bufs B, StatsSnapshot* dst, uint32_t scene);
 __global__ void k_snapshot4(float4* dst, const float4* src, uint32_t stride, uint32_t n,
                             int fix_w, float w);
 
+// One wait of the cell scan and of the resident solves' barrier for something
+// that never comes: gives up after `limit` polls (or the kernel's own bound) and
+// raises bit 0x4 of *flags.  status, count: a zeroed word.
+cudaError_t scan_wait_on(const unsigned long long* status, uint32_t* flags, int limit,
+                         cudaStream_t stream);
+cudaError_t grid_barrier_wait_on(uint32_t* count, uint32_t* flags, int limit, cudaStream_t stream);
+
 }  // namespace fe

@@ -32,12 +32,14 @@ namespace {
 constexpr int kBarrierSpins = 1 << 22;
 
 // Barrier number `k` (1, 2, ...) of the launch over all blocks.  False, with
-// the flag raised, if it did not come about.  Whole block.  Every thread's
-// stores before it come before every thread's loads after it (release and
-// acquire by one thread, bar.sync for the others), so the gathers are plain
-// loads, which the neighbours that a cell's particles share make L1 hits
-// (through L2 alone an iteration took 14.0 us instead of 11.2 at 37k particles).
-__device__ __forceinline__ bool grid_barrier(const Bufs& B, uint32_t* count, uint32_t k) {
+// the flag raised, if it did not come about within `limit` polls.  Whole block.
+// Every thread's stores before it come before every thread's loads after it
+// (release and acquire by one thread, bar.sync for the others), so the gathers
+// are plain loads, which the neighbours that a cell's particles share make L1
+// hits (through L2 alone an iteration took 14.0 us instead of 11.2 at 37k
+// particles).
+__device__ __forceinline__ bool grid_barrier(uint32_t* flags, uint32_t* count, uint32_t k,
+                                             int limit = kBarrierSpins) {
     __syncthreads();
     int ok = 1;
     if (threadIdx.x == 0) {
@@ -48,8 +50,8 @@ __device__ __forceinline__ bool grid_barrier(const Bufs& B, uint32_t* count, uin
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
             if (seen >= target) break;
-            if (++spins > kBarrierSpins) {
-                atomicOr(&B.G->flags, 0x4u);
+            if (++spins > limit) {
+                atomicOr(flags, 0x4u);
                 ok = 0;
                 break;
             }
@@ -275,7 +277,7 @@ __global__ void __launch_bounds__(kResidentThreads, 3)
         // every thread has its acceleration from the current pressures
         const f3 ai = {-acc.x, -acc.y, -acc.z};
         if (live) *accp(B, i) = make_float4(ai.x, ai.y, ai.z, 0.0f);
-        if (!(ok = grid_barrier(B, R.barrier, ++barrier))) break;
+        if (!(ok = grid_barrier(&B.G->flags, R.barrier, ++barrier))) break;
         double e_sum = 0.0;
         if (live) {
             float sum_ap = 0.0f;
@@ -313,7 +315,7 @@ __global__ void __launch_bounds__(kResidentThreads, 3)
                 R.maxes[i >> 5] = b;
             }
         }
-        if (!(ok = grid_barrier(B, R.barrier, ++barrier))) break;
+        if (!(ok = grid_barrier(&B.G->flags, R.barrier, ++barrier))) break;
         ++iter;
         if (tolerance) {
             double sum, mx;
@@ -395,7 +397,7 @@ __global__ void __launch_bounds__(kBlock, kResidentBlocks)
             if (threadIdx.x < cc.y && (one || iter < wanted(cc.z)))
                 pressure_force_particle<kBlock, true>(B, cc.x + threadIdx.x, cc.z);
         }
-        if (!grid_barrier(B, R.barrier, ++barrier)) break;
+        if (!grid_barrier(&B.G->flags, R.barrier, ++barrier)) break;
         for (uint32_t c = blockIdx.x; c < B.n_chunks; c += gridDim.x) {
             const uint4 cc = B.chunks[c];
             const uint32_t i = cc.x + threadIdx.x;
@@ -405,7 +407,7 @@ __global__ void __launch_bounds__(kBlock, kResidentBlocks)
                                              pressure_update_sum<kBlock, true>(B, B.P[cc.z], i));
             if (tolerance) solve_chunk_partials(B, c, e, smem);
         }
-        if (!grid_barrier(B, R.barrier, ++barrier)) break;
+        if (!grid_barrier(&B.G->flags, R.barrier, ++barrier)) break;
         ++iter;
         done = iter >= limit;
         if (tolerance) {
@@ -426,6 +428,19 @@ __global__ void __launch_bounds__(kBlock, kResidentBlocks)
         if (threadIdx.x == 0) end_solve(B, which);
     }
     leave(R.barrier);
+}
+
+namespace {
+// Waits for a barrier that this launch alone cannot complete.
+__global__ void k_barrier_selftest(uint32_t* count, uint32_t* flags, int limit) {
+    grid_barrier(flags, count, 2, limit);
+}
+}  // namespace
+
+cudaError_t grid_barrier_wait_on(uint32_t* count, uint32_t* flags, int limit, cudaStream_t stream) {
+    k_barrier_selftest<<<1, kResidentThreads, 0, stream>>>(
+        count, flags, limit < kBarrierSpins ? limit : kBarrierSpins);
+    return cudaGetLastError();
 }
 
 }  // namespace fe

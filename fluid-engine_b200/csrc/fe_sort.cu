@@ -686,19 +686,6 @@ __global__ void k_lookback_selftest(const uint32_t* status, uint32_t* error_flag
 }
 }  // namespace
 
-cudaError_t lookback_wait_selftest(int limit, uint32_t* flags_out) {
-    uint32_t* d = nullptr;
-    cudaError_t e = cudaMalloc(&d, 8);
-    if (e != cudaSuccess) return e;
-    if ((e = cudaMemset(d, 0, 8)) == cudaSuccess) {
-        k_lookback_selftest<<<1, 1>>>(d, d + 1, limit < kMaxSpins ? limit : kMaxSpins);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpy(flags_out, d + 1, 4, cudaMemcpyDeviceToHost);
-    }
-    cudaFree(d);
-    return e;
-}
-
 cudaError_t lookback_wait_on(uint32_t* status, uint32_t* error_flags, int limit,
                              cudaStream_t stream) {
     k_lookback_selftest<<<1, 1, 0, stream>>>(status, error_flags,

@@ -71,13 +71,9 @@ cudaError_t radix_sort_small(uint32_t* keys, uint32_t* vals, uint32_t n, uint32_
 // In-place bitonic network; n must be a power of two.
 cudaError_t bitonic_sort(const SortLaunch& L, uint32_t* keys, uint32_t* vals, uint32_t n);
 
-// Runs one look-back wait on a status word that is never published, with at
-// most `limit` polls (clamped to the radix pass's own limit), on the current
-// device; *flags_out receives the error flags it raised (0x4 = timed out).
-cudaError_t lookback_wait_selftest(int limit, uint32_t* flags_out);
-
-// The same wait, enqueued on `stream`, on a caller's status word (which must
-// hold no published flag) with the timeout flag raised in *error_flags.
+// One look-back wait of the radix pass, enqueued on `stream`, on a status word
+// that is never published (it must hold no published flag): gives up after at
+// most `limit` polls (or the pass's own bound) and raises 0x4 in *error_flags.
 cudaError_t lookback_wait_on(uint32_t* status, uint32_t* error_flags, int limit,
                              cudaStream_t stream);
 

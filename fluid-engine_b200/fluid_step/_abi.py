@@ -79,6 +79,8 @@ FE_STATS_NEIGHBOR_OVERFLOW = 0x2
 FE_STATS_LOOKBACK_TIMEOUT = 0x4
 FE_STATS_NON_FINITE = 0x8
 
+FE_WAIT_SORT, FE_WAIT_SEARCH, FE_WAIT_SOLVE = 0, 1, 2
+
 FE_MAX_PARTICLES = 1 << 26
 FE_MAX_SCENES = 65536
 
@@ -367,6 +369,7 @@ SIGNATURES = {
     "fe_debug_fail_allocation": (None, [c_uint32]),
     "fe_debug_poison_allocations": (None, [c_int]),
     "fe_debug_bounded_wait": (c_int, [c_int, c_uint32, POINTER(c_uint32)]),
+    "fe_debug_bounded_wait_in": (c_int, [c_int, c_uint32, c_uint32, POINTER(c_uint32)]),
     "fe_state_size": (c_int, [CTX, POINTER(c_size_t)]),
     "fe_state_export": (c_int, [CTX, c_void_p, c_size_t]),
     "fe_state_import": (c_int, [CTX, c_void_p, c_size_t]),

@@ -423,10 +423,19 @@ FE_API fe_status fe_state_import(fe_ctx* ctx, const void* src, size_t bytes);
  * fe_debug_bounded_wait(device, limit, flags): runs one look-back wait of
  *   the radix pass on a status word that is never published, giving up
  *   after `limit` polls; returns FE_ERR_TIMEOUT with FE_STATS_LOOKBACK_TIMEOUT
- *   in *flags, and the device stays usable. */
+ *   in *flags, and the device stays usable.
+ * fe_debug_bounded_wait_in(device, wait, limit, flags): the same for any of the
+ *   waits on other blocks: the radix pass's look-back (FE_WAIT_SORT), the cell
+ *   scan's look-back of the neighbour search (FE_WAIT_SEARCH), the grid barrier
+ *   of the resident solves (FE_WAIT_SOLVE). */
+#define FE_WAIT_SORT   0u
+#define FE_WAIT_SEARCH 1u
+#define FE_WAIT_SOLVE  2u
 FE_API void fe_debug_fail_allocation(uint32_t k);
 FE_API void fe_debug_poison_allocations(int on);
 FE_API fe_status fe_debug_bounded_wait(int device, uint32_t limit, uint32_t* flags);
+FE_API fe_status fe_debug_bounded_wait_in(int device, uint32_t wait, uint32_t limit,
+                                          uint32_t* flags);
 
 /* ------------------------------------------------------------------------- */
 /* Whole step                                                                */

@@ -152,3 +152,24 @@ def test_forward_after_a_failed_growth_of_its_rows(lib):
     rc, whole = forward(50_000)
     assert rc == _abi.FE_OK and torch.equal(whole[:900], before)
     m.close()
+
+
+@pytest.mark.parametrize("wait", [_abi.FE_WAIT_SORT, _abi.FE_WAIT_SEARCH, _abi.FE_WAIT_SOLVE])
+def test_every_wait_on_other_blocks_runs_out(lib, wait):
+    """The look-backs of the sort and the cell scan and the resident solves' grid
+    barrier, each on something that never comes: a status, and the search and the
+    solve still work."""
+    p, pos = _scene(n_drop=3)
+    sim = Simulation(pos, p)
+    sim.step(1)
+    flags = ctypes.c_uint32(7)
+    t0 = time.perf_counter()
+    rc = lib.fe_debug_bounded_wait_in(0, wait, 2000, ctypes.byref(flags))
+    assert time.perf_counter() - t0 < 5.0
+    assert rc == _abi.FE_ERR_TIMEOUT and flags.value == _abi.FE_STATS_LOOKBACK_TIMEOUT
+    assert b"timed out" in lib.fe_last_error()
+    assert sim.step(1).flags & _abi.FE_STATS_LOOKBACK_TIMEOUT == 0
+    sim.close()
+    for bad in ((3, 10, flags), (wait, 0, flags)):
+        assert lib.fe_debug_bounded_wait_in(0, bad[0], bad[1], ctypes.byref(bad[2])) == \
+            _abi.FE_ERR_INVALID_ARGUMENT
