@@ -2847,6 +2847,23 @@ FE_API fe_status fe_debug_bounded_wait_in(int device, uint32_t wait, uint32_t li
     return FE_OK;
 }
 
+FE_API fe_status fe_debug_sort_wait_timeout(uint32_t limit, void* stream_ptr) {
+    int dev;
+    FE_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(g_sort_mutex);
+    if (limit == 0 || dev < 0 || dev >= 16 || !g_sort[dev].flags) {
+        set_error("fe_debug_sort_wait_timeout needs a non-zero limit and a sort before it");
+        return FE_ERR_INVALID_ARGUMENT;
+    }
+    SortScratch& S = g_sort[dev];
+    cudaStream_t stream = (cudaStream_t)stream_ptr;
+    FE_CUDA(cudaStreamWaitEvent(stream, S.done, 0));
+    FE_CUDA(cudaMemsetAsync(S.flags, 0, kSortFlagWords * 4, stream));
+    FE_CUDA(lookback_wait_on(S.flags + 1, S.flags, (int)std::min<uint32_t>(limit, 1u << 30), stream));
+    FE_CUDA(cudaEventRecord(S.done, stream));
+    return FE_OK;
+}
+
 FE_API fe_status fe_debug_bounded_wait(int device, uint32_t limit, uint32_t* flags) {
     return fe_debug_bounded_wait_in(device, FE_WAIT_SORT, limit, flags);
 }

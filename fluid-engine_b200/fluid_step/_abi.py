@@ -369,6 +369,7 @@ SIGNATURES = {
     "fe_debug_fail_allocation": (None, [c_uint32]),
     "fe_debug_poison_allocations": (None, [c_int]),
     "fe_debug_bounded_wait": (c_int, [c_int, c_uint32, POINTER(c_uint32)]),
+    "fe_debug_sort_wait_timeout": (c_int, [c_uint32, c_void_p]),
     "fe_debug_bounded_wait_in": (c_int, [c_int, c_uint32, c_uint32, POINTER(c_uint32)]),
     "fe_state_size": (c_int, [CTX, POINTER(c_size_t)]),
     "fe_state_export": (c_int, [CTX, c_void_p, c_size_t]),

@@ -427,7 +427,10 @@ FE_API fe_status fe_state_import(fe_ctx* ctx, const void* src, size_t bytes);
  * fe_debug_bounded_wait_in(device, wait, limit, flags): the same for any of the
  *   waits on other blocks: the radix pass's look-back (FE_WAIT_SORT), the cell
  *   scan's look-back of the neighbour search (FE_WAIT_SEARCH), the grid barrier
- *   of the resident solves (FE_WAIT_SOLVE). */
+ *   of the resident solves (FE_WAIT_SOLVE).
+ * fe_debug_sort_wait_timeout(limit, stream): such a wait on the current device
+ *   in the order of `stream`, raising FE_STATS_LOOKBACK_TIMEOUT in the error
+ *   word that fe_sort_flags reports (after at least one radix fe_sort_pairs). */
 #define FE_WAIT_SORT   0u
 #define FE_WAIT_SEARCH 1u
 #define FE_WAIT_SOLVE  2u
@@ -436,6 +439,7 @@ FE_API void fe_debug_poison_allocations(int on);
 FE_API fe_status fe_debug_bounded_wait(int device, uint32_t limit, uint32_t* flags);
 FE_API fe_status fe_debug_bounded_wait_in(int device, uint32_t wait, uint32_t limit,
                                           uint32_t* flags);
+FE_API fe_status fe_debug_sort_wait_timeout(uint32_t limit, void* stream);
 
 /* ------------------------------------------------------------------------- */
 /* Whole step                                                                */

@@ -56,3 +56,31 @@ def test_bitonic_network_of_every_tile(oracle_mod, n, ties):
     ks, vs = sort_pairs_host(k, v, algorithm=_abi.FE_SORT_BITONIC)
     rk, rv = oracle_mod.sort_bitonic(k, v)
     assert np.array_equal(ks, rk) and np.array_equal(vs, rv)
+
+
+@pytest.mark.parametrize("n", [1000, 40000, 100000])
+def test_a_sort_clears_an_error_word_that_was_raised(n):
+    """The error word is one call's: a wait that ran out raises it, and the next
+    sort, by one cluster or in passes, clears it in stream order."""
+    import torch
+    lib = _abi.load_library()
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    k = torch.randint(0, 1 << 30, (n,), dtype=torch.int32, device="cuda")
+    v = torch.arange(n, dtype=torch.int32, device="cuda")
+
+    def sort():
+        assert lib.fe_sort_pairs(ctypes.c_void_p(k.data_ptr()), ctypes.c_void_p(v.data_ptr()), n,
+                                 32, _abi.FE_SORT_RADIX, st) == _abi.FE_OK
+
+    def word():
+        f = torch.full((1,), 7, dtype=torch.int32, device="cuda")
+        assert lib.fe_sort_flags(ctypes.c_void_p(f.data_ptr()), st) == _abi.FE_OK
+        return int(f.item())
+
+    sort()
+    assert word() == 0
+    assert lib.fe_debug_sort_wait_timeout(500, st) == _abi.FE_OK
+    assert word() == _abi.FE_STATS_LOOKBACK_TIMEOUT
+    sort()
+    assert word() == 0
+    assert lib.fe_debug_sort_wait_timeout(0, st) == _abi.FE_ERR_INVALID_ARGUMENT
