@@ -227,3 +227,38 @@ def test_batch_solves_around_their_line(last):
             assert np.array_equal(x.view(np.uint32), one.data.download(f).view(np.uint32)), (s, f)
         one.close()
     batch.close()
+
+
+@pytest.mark.parametrize("solvers", ["fixed", "mixed"])
+def test_batch_scenes_keep_their_counts_beside_a_non_finite_one(solvers):
+    """The iteration counts of every scene, resident or iterated; only the scene
+    with an infinite velocity may report an error, and only once it has it."""
+    w = scene.batch_workload(n_scenes=5, seed=6, lo=300, hi=900)
+    params = w.params()
+    for k, p in enumerate(params):
+        p.density_solver_iterations, p.divergence_solver_iterations = 2 + k, 5 - k
+        if solvers == "mixed" and k in (1, 3):
+            p.solver = _abi.FE_SOLVER_TOLERANCE
+    pos = w.positions()
+    batch = BatchSimulation(pos, params)
+    singles = [Simulation(a, q) for a, q in zip(pos, params)]
+    for frame in range(3):
+        if frame == 2:
+            v = batch.data.download(_abi.FE_FIELD_VELOCITY_B)
+            first, n = int(batch.data.scene_first[2]), int(batch.data.scene_count[2])
+            v[first + n // 2, 1] = np.inf
+            batch.data.upload(_abi.FE_FIELD_VELOCITY_B, v)
+            singles[2].data.upload(_abi.FE_FIELD_VELOCITY_B, v[first:first + n])
+        batch.step(1, want_stats=False)
+        for s, sim in enumerate(singles):
+            sim.step(1, want_stats=False)
+            if frame == 2 and s == 2:
+                continue
+            a, b = batch.data.read_scene_stats(s), sim.data.read_stats()
+            counts = (a.density_iterations, a.divergence_iterations)
+            assert counts == (b.density_iterations, b.divergence_iterations), (frame, s)
+            if params[s].solver == _abi.FE_SOLVER_FIXED_ITERS:
+                assert counts == (2 + s, 5 - s), (frame, s)
+    batch.close()
+    for sim in singles:
+        sim.close()
