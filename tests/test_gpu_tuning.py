@@ -278,3 +278,77 @@ def test_set_tuning_rejects_neighbour_shapes_outside_the_candidates():
     for t in bad:
         assert lib.fe_set_tuning(sim.data.handle, ctypes.byref(t)) == _abi.FE_ERR_INVALID_ARGUMENT
     sim.close()
+
+
+# --------------------------------------------------------------------------
+# The same above the sizes where few particles take shapes of their own and the
+# solves are one kernel (18,944 and 37,888 particles): here the tuned list passes
+# and the iterated solves run.
+# --------------------------------------------------------------------------
+def _large_frames(tuning, learned_model=None, frames=2):
+    w = scene.workload("dam_break_256k")
+    p = _abi.copy_params(w.params)
+    p.solver, p.mode = _abi.FE_SOLVER_TOLERANCE, _abi.FE_MODE_FIXED
+    if learned_model is not None:
+        p.warm_start = _abi.FE_WARM_LEARNED
+    vel = np.random.default_rng(3).normal(0, 0.3, (38011, 3)).astype(np.float32)
+    sim = Simulation(w.positions()[:38011], p, velocities=vel)
+    if learned_model is not None:
+        _abi.check(sim.data._lib, sim.data._lib.fe_set_model(sim.data.handle,
+                                                             learned_model.handle), "")
+    if tuning is not None:
+        sim.data.set_tuning(tuning)
+    for _ in range(frames):
+        st = sim.step(1)
+    out = {f: sim.data.download(f).copy() for f in
+           (_abi.FE_FIELD_POSITION_A, _abi.FE_FIELD_VELOCITY_A, _abi.FE_FIELD_VELOCITY_B,
+            _abi.FE_FIELD_DENSITY, _abi.FE_FIELD_SOURCE_TERM, _abi.FE_FIELD_PRESSURE,
+            _abi.FE_FIELD_PRESSURE_ACCEL)}
+    sim.close()
+    return out, st
+
+
+@pytest.fixture(scope="module")
+def large_reference():
+    return _large_frames(None)
+
+
+@pytest.mark.parametrize("threads,persistent", NBR_SHAPES)
+def test_iterated_frames_identical_under_every_neighbour_shape(large_reference, threads,
+                                                               persistent):
+    ref, st_ref = large_reference
+    got, st = _large_frames(_nbr_tuning(threads, persistent))
+    _same(ref, got)
+    for name in ("density_iterations", "divergence_iterations", "density_residual",
+                 "divergence_residual", "density_residual_max", "divergence_residual_max"):
+        assert getattr(st, name) == getattr(st_ref, name), name
+    assert st.density_iterations > 1
+
+
+def test_iterated_learned_frames_identical_under_neighbour_shapes():
+    m = learned.Model(seed=5)
+    ref, st_ref = _large_frames(None, m)
+    for shape in NBR_SHAPES:
+        got, st = _large_frames(_nbr_tuning(*shape), m)
+        _same(ref, got)
+        assert st.density_iterations == st_ref.density_iterations, shape
+    m.close()
+
+
+@pytest.mark.parametrize("digit_bits,items", _abi.RADIX_CANDIDATES)
+def test_sorts_identical_under_every_tuned_radix_shape(digit_bits, items):
+    """Above 65,536 pairs, where fe_sort_pairs reads the tuned shape: every shape
+    against the default one."""
+    lib = _abi.load_library()
+    n = 70_001
+    rng = np.random.default_rng(5)
+    keys = rng.integers(0, 1 << 20, n, dtype=np.uint64).astype(np.uint32)
+    out = []
+    for call in (lambda k, v: lib.fe_sort_pairs(ptr(k), ptr(v), n, 20, _abi.FE_SORT_RADIX, None),
+                 lambda k, v: lib.fe_sort_pairs_config(ptr(k), ptr(v), n, 20, digit_bits, items,
+                                                       None)):
+        k, v = dev(keys.view(np.int32)), dev(np.arange(n, dtype=np.int32))
+        assert call(k, v) == _abi.FE_OK
+        torch.cuda.synchronize()
+        out.append((k.cpu().numpy(), v.cpu().numpy()))
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
