@@ -599,6 +599,9 @@ fe_status rec_density_alpha_div(fe_ctx* c, Recorder& R) {
                            : rec_density(c, R, DENSITY_DIV(k_density_alpha_div, 2), c->B);
 }
 
+// Whether group g's launches follow its tuned shape at this context's size.
+bool nbr_shape_used(const fe_ctx* c, int g) { return g != FE_NBR_DENSITY_ALPHA && !few(c); }
+
 // Whether a shape may run group g.
 bool nbr_shape_ok(int g, uint32_t threads, uint32_t persistent) {
     if (persistent > 1) return false;
@@ -2354,6 +2357,11 @@ fe_status tune_neighbour_kernels(fe_ctx* c, fe_tune_report* r) {
         for (int k = 0; k < kNbrCands; ++k) {
             r->nbr_ms[g][k] = -1.0f;
             if (!nbr_shape_ok(g, kNbrCandThreads[k], kNbrCandPersistent[k])) continue;
+            // where all shapes are one launch, the current one alone: the
+            // others' times would differ by chance and decide by it
+            if (!nbr_shape_used(c, g) &&
+                !(kNbrCandThreads[k] == keep_t && kNbrCandPersistent[k] == keep_p))
+                continue;
             c->nbr_threads[g] = kNbrCandThreads[k];
             c->nbr_persistent[g] = kNbrCandPersistent[k];
             float ms = 0.0f;

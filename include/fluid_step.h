@@ -539,7 +539,9 @@ typedef struct fe_tune_report {
     float mlp_ms[FE_TUNE_MAX_CANDIDATES];
     /* neighbour kernels (0 candidates before the first neighbour search):
      * the shared candidate list, and per group the median time of each
-     * candidate, negative where it is not a candidate of that group */
+     * candidate, negative where it is not a candidate of that group, or where
+     * the group's launches do not follow its shape at this size and it is not
+     * the current one */
     uint32_t nbr_candidates;
     uint32_t nbr_threads[FE_TUNE_MAX_CANDIDATES];
     uint32_t nbr_persistent[FE_TUNE_MAX_CANDIDATES];

@@ -352,3 +352,26 @@ def test_sorts_identical_under_every_tuned_radix_shape(digit_bits, items):
         torch.cuda.synchronize()
         out.append((k.cpu().numpy(), v.cpu().numpy()))
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("n", [12000, 38011])
+def test_autotune_times_the_shapes_that_are_used(n):
+    """Groups whose launches do not follow their shape at this size (density_alpha
+    always, the list passes of few particles) keep the one they have."""
+    w = scene.workload("dam_break_256k")
+    p = _abi.copy_params(w.params)
+    p.mode = _abi.FE_MODE_FIXED
+    sim = Simulation(w.positions()[:n], p)
+    sim.step(1)
+    sim.data.set_tuning(_nbr_tuning(128, 1))
+    r = sim.data.autotune()
+    t = sim.data.tuning()
+    for g in range(_abi.FE_NBR_GROUPS):
+        timed = [(r.nbr_threads[k], r.nbr_persistent[k]) for k in range(r.nbr_candidates)
+                 if r.nbr_ms[g][k] >= 0]
+        if g == _abi.FE_NBR_DENSITY_ALPHA or n == 12000:
+            own = 256 if g == _abi.FE_NBR_PRESSURE_UPDATE else 128
+            assert timed == [(own, 1)] == [(t.nbr_threads[g], t.nbr_persistent[g])], g
+        else:
+            assert len(timed) == (2 if g == _abi.FE_NBR_PRESSURE_UPDATE else 6), g
+    sim.close()
