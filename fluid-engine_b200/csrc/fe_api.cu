@@ -567,16 +567,21 @@ fe_status rec_nbr(fe_ctx* c, Recorder& R, int g, void (*func)(KArgs...), Args...
 }
 
 // density_alpha: blocks of 64 threads (the shapes fe_set_tuning takes for this
-// group are accepted and make no difference).  Particles per warp: 8 while all
-// those warps are resident at once (32 an SM), 16 up to half as many particles
-// again, else 32.  Times in a graph of launches (us, 8 / 16 / 32 per warp, a
-// fall after 40 frames): 4.8k particles 28/43/58, 25k 43/60/65, 50k 72/63/68,
-// 80k 99/78/70, 131k 152/112/80.
+// group are accepted and make no difference).  Particles per warp: 8 while the
+// warps take up to 5/8 of the SMs' places (32 an SM), 16 while they take up to
+// 6/8, else 32.  Times in a graph of launches (us, 8 / 16 / 32 per warp, a fall
+// after 40 frames): 4.8k particles 28/43/58, 25k 43/60/65, 50k 72/63/68, 80k
+// 99/78/70, 131k 152/112/80.  Alone, 8 per warp are the fastest up to 38k; but
+// they are more instructions for the same particles, and beside other contexts'
+// frames those are what counts.  Frames of 25k and 37k particles of one context /
+// two / four / eight, us, 8 per warp 222/134/88/74 and 239/151/116/112, 16 per
+// warp 227/130/82/66 and 231/139/102/100 (32, without resident solves,
+// 333/191/109/72 and 350/202/125/96); of 20k 217/126/80/59 and 220/123/74/52.
 template <class... KArgs, class... Args>
 fe_status rec_density(fe_ctx* c, Recorder& R, void (*k8)(KArgs...), void (*k16)(KArgs...),
                       void (*k32)(KArgs...), Args... args) {
     const uint32_t warps = c->num_sms * 32u;
-    const uint32_t lanes = c->n <= warps * 8u ? 8u : c->n <= warps * 12u ? 16u : 32u;
+    const uint32_t lanes = c->n <= warps * 5u ? 8u : c->n <= warps * 12u ? 16u : 32u;
     const uint32_t blocks = c->B.n_chunks * (kBlock / lanes) / (kFewThreads / 32);
     REC(R.k(lanes == 8 ? k8 : lanes == 16 ? k16 : k32, dim3(blocks), dim3(kFewThreads), args...));
     return FE_OK;

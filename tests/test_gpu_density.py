@@ -171,3 +171,8 @@ def test_many_runs_beside_crowded_cells(oracle_mod, mode):
         a, b = sim.data.download(f).view(np.uint32), orc.field(f).view(np.uint32)
         assert np.array_equal(a, b), f
     sim.close()
+
+
+@pytest.mark.parametrize("n", [23680, 23681, 23700])
+def test_particles_per_warp_around_the_first_line(oracle_mod, n):
+    test_particles_per_warp(oracle_mod, n)
