@@ -262,3 +262,27 @@ def test_batch_scenes_keep_their_counts_beside_a_non_finite_one(solvers):
     batch.close()
     for sim in singles:
         sim.close()
+
+
+@pytest.mark.parametrize("mode", [_abi.FE_MODE_REFERENCE, _abi.FE_MODE_FIXED])
+@pytest.mark.parametrize("side,per_clump", [(0.24, 0), (0.4, 0), (0.4, 100)])
+def test_resident_solve_past_the_neighbour_list(oracle_mod, side, per_clump, mode):
+    """A particle per thread: particles that walk the buckets in every half
+    iteration, all of them, some, and beside ones with lists."""
+    rng = np.random.default_rng(int(side * 100))
+    pos = (rng.random((900, 3)) * side + 0.12).astype(np.float32)
+    if per_clump:
+        pos = np.concatenate([pos, _with_clumps(1500, per_clump, 4) + np.float32(0.6)])
+    p = scene.dam_break_params((0, 0, 0), (4.0, 4.0, 4.0), mode=mode)
+    p.density_solver_iterations, p.divergence_solver_iterations = 5, 6
+    p.dt = 0.0001
+    sim, orc = Simulation(pos, p), oracle_mod.Oracle(p, pos)
+    for k in range(2):
+        st = sim.step(1)
+        orc.step(1)
+        if k == 0:
+            assert st.flags & _abi.FE_STATS_NEIGHBOR_OVERFLOW
+        for f in FIELDS:
+            x, y = sim.data.download(f).view(np.uint32), orc.field(f).view(np.uint32)
+            assert np.array_equal(x, y), (k, f)
+    sim.close()
