@@ -108,6 +108,46 @@ __device__ __forceinline__ void walk(const Bufs& B, const DevParams& P, f3 pi, F
             }
 }
 
+// The same with the next candidate's position and load(j) on their way while this
+// one's terms are computed, f(r_vec, r2, load(j)): for few particles, whose threads
+// have nothing else to wait with.  20 + 20 iterations of 2.3k and 8.2k particles at
+// h = 2.6 spacings (73 neighbours each, more than the list holds): 13.2 and 15.1 ms
+// in k_solve_resident with the walk above, 9.8 and 10.4 with this one; as passes
+// of 256 threads a block 11.7 and 14.0.
+template <bool kCoherent, class Load, class F>
+__device__ __forceinline__ void walk_ahead(const Bufs& B, const DevParams& P, f3 pi, Load&& load,
+                                           F&& f) {
+    auto position = [&](uint32_t j) { return kCoherent ? *posb(B, j) : __ldg(posb(B, j)); };
+    const float h2 = P.h * P.h;
+    const int cx = cell_coord(pi.x, P.h), cy = cell_coord(pi.y, P.h), cz = cell_coord(pi.z, P.h);
+#pragma unroll 1
+    for (int z = -1; z <= 1; ++z)
+#pragma unroll 1
+        for (int y = -1; y <= 1; ++y)
+#pragma unroll 1
+            for (int x = -1; x <= 1; ++x) {
+                const uint2 cell =
+                    __ldg(B.cells + P.table_base +
+                          cell_hash_pow2((int)((uint32_t)cx + (uint32_t)x),
+                                         (int)((uint32_t)cy + (uint32_t)y),
+                                         (int)((uint32_t)cz + (uint32_t)z), P.T - 1u));
+                if (cell.x == kEmpty) continue;
+                float4 pj = position(cell.x);
+                auto d = load(cell.x);
+#pragma unroll 1
+                for (uint32_t j = cell.x; j < cell.y; ++j) {
+                    const f3 rv = sub(pi, xyz(pj));
+                    const auto d0 = d;
+                    if (j + 1 < cell.y) {
+                        pj = position(j + 1);
+                        d = load(j + 1);
+                    }
+                    const float r2 = dot(rv, rv);
+                    if (!(r2 > h2)) f(rv, r2, d0);
+                }
+            }
+}
+
 // Streaming read of a neighbour-list entry: read once per pass, so it
 // bypasses L1 and carries an evict-first L2 policy, leaving the caches to the
 // gathered neighbour data.
@@ -176,6 +216,16 @@ __device__ __forceinline__ void for_each_entry(const Bufs& B, uint32_t i, uint32
     }
 }
 
+// The walk of a pass in this shape: f(r_vec, r2, load(j)).
+template <int kThreads, bool kCoherent, class Load, class F>
+__device__ __forceinline__ void walk_for(const Bufs& B, const DevParams& P, f3 pi, Load&& load,
+                                         F&& f) {
+    if constexpr (kEntryAhead<kThreads>)
+        walk_ahead<kCoherent>(B, P, pi, load, f);
+    else
+        walk<kCoherent>(B, P, pi, [&](uint32_t j, f3 rv, float r2) { f(rv, r2, load(j)); });
+}
+
 // Neighbours with r > 1e-6 in walk order: f(r_vec, grad_scale, pos_j), where
 // pos_j = pos_b[j] (w = p_j / rho_j^2).  kCoherent: other blocks of the same
 // launch write what is gathered (between grid barriers), so the loads are not
@@ -190,10 +240,10 @@ __device__ __forceinline__ void for_each_neighbor(const Bufs& B, const DevParams
             [&](uint2 v, float4 q) { f(sub(pi, xyz(q)), __uint_as_float(v.y), q); });
     } else {
         const float h = P.h;
-        walk<kCoherent>(B, P, pi, [&](uint32_t j, f3 rv, float r2) {
-            float r = sqrtf(r2);
-            if (r > kEpsR)
-                f(rv, kernel_grad_scale(r, h), kCoherent ? *posb(B, j) : __ldg(posb(B, j)));
+        auto load = [&](uint32_t j) { return kCoherent ? *posb(B, j) : __ldg(posb(B, j)); };
+        walk_for<kThreads, kCoherent>(B, P, pi, load, [&](f3 rv, float r2, float4 q) {
+            const float r = sqrtf(r2);
+            if (r > kEpsR) f(rv, kernel_grad_scale(r, h), q);
         });
     }
 }
@@ -228,10 +278,13 @@ __device__ __forceinline__ void for_each_neighbor_pair(const Bufs& B, const DevP
             });
     } else {
         const float h = P.h;
-        walk<kCoherent>(B, P, pi, [&](uint32_t j, f3 rv, float r2) {
-            float r = sqrtf(r2);
+        auto load = [&](uint32_t j) {
             const float4* data = recs + 2 * (size_t)j + 1;
-            if (r > kEpsR) f(rv, kernel_grad_scale(r, h), kCoherent ? *data : __ldg(data));
+            return kCoherent ? *data : __ldg(data);
+        };
+        walk_for<kThreads, kCoherent>(B, P, pi, load, [&](f3 rv, float r2, float4 d) {
+            const float r = sqrtf(r2);
+            if (r > kEpsR) f(rv, kernel_grad_scale(r, h), d);
         });
     }
 }

@@ -66,46 +66,6 @@ struct Particle {
     f3 pi;
 };
 
-// The bucket walk with the next candidate's loads on their way while this one's
-// terms are computed: a thread has nothing else to wait with here (20 + 20
-// iterations of 2.3k and 8.2k particles at h = 2.6 spacings, 73 neighbours each:
-// 13.2 and 15.1 ms with the passes' walk, 9.8 and 10.4 this way; as passes of their
-// own, before there were resident solves, 11.7 and 14.0).
-// f(r_vec, r2, load(j)) for each candidate with r2 <= h*h, in walk order; plain
-// loads, as other blocks write between grid barriers.
-template <class Load, class F>
-__device__ __forceinline__ void walk_ahead(const Bufs& B, const DevParams& P, f3 pi, Load&& load,
-                                           F&& f) {
-    const float h2 = P.h * P.h;
-    const int cx = cell_coord(pi.x, P.h), cy = cell_coord(pi.y, P.h), cz = cell_coord(pi.z, P.h);
-#pragma unroll 1
-    for (int z = -1; z <= 1; ++z)
-#pragma unroll 1
-        for (int y = -1; y <= 1; ++y)
-#pragma unroll 1
-            for (int x = -1; x <= 1; ++x) {
-                const uint2 cell =
-                    __ldg(B.cells + P.table_base +
-                          cell_hash_pow2((int)((uint32_t)cx + (uint32_t)x),
-                                         (int)((uint32_t)cy + (uint32_t)y),
-                                         (int)((uint32_t)cz + (uint32_t)z), P.T - 1u));
-                if (cell.x == kEmpty) continue;
-                float4 pj = *posb(B, cell.x);
-                auto d = load(cell.x);
-#pragma unroll 1
-                for (uint32_t j = cell.x; j < cell.y; ++j) {
-                    const f3 rv = sub(pi, xyz(pj));
-                    const auto d0 = d;
-                    if (j + 1 < cell.y) {
-                        pj = *posb(B, j + 1);
-                        d = load(j + 1);
-                    }
-                    const float r2 = dot(rv, rv);
-                    if (!(r2 > h2)) f(rv, r2, d0);
-                }
-            }
-}
-
 // f(gradient, load(j)) over particle q's neighbours in list order, kBatch loads
 // in flight.
 template <int kBatch, class Load, class F>
@@ -113,7 +73,7 @@ __device__ __forceinline__ void for_each_cached(const Bufs& B, const DevParams& 
                                                 const Particle& q, Load&& load, F&& f) {
     if (q.cnt > kNbrCap) {
         const float h = P.h;
-        walk_ahead(B, P, q.pi, load, [&](f3 rv, float r2, auto d) {
+        walk_ahead<true>(B, P, q.pi, load, [&](f3 rv, float r2, auto d) {
             const float r = sqrtf(r2);
             if (r > kEpsR) f(scale(kernel_grad_scale(r, h), rv), d);
         });

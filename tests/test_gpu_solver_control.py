@@ -286,3 +286,27 @@ def test_resident_solve_past_the_neighbour_list(oracle_mod, side, per_clump, mod
             x, y = sim.data.download(f).view(np.uint32), orc.field(f).view(np.uint32)
             assert np.array_equal(x, y), (k, f)
     sim.close()
+
+
+@pytest.mark.parametrize("mode", [_abi.FE_MODE_REFERENCE, _abi.FE_MODE_FIXED])
+@pytest.mark.parametrize("n", [900, 9000, 12000, 20000])
+def test_passes_past_the_neighbour_list(n, mode):
+    """Pass by pass, in the shapes for few particles and above them, where some
+    particles walk the buckets: the fields of the whole frame."""
+    p = scene.dam_break_params((0, 0, 0), (4.0, 4.0, 4.0), mode=mode)
+    p.density_solver_iterations = p.divergence_solver_iterations = 3
+    p.dt = 0.0002
+    pos = _with_clumps(n, 90, 6)
+    sim, data = Simulation(pos, p), GpuPhysicsData(pos, p)
+    steps = ComputePipelines()
+    steps.prepare_all(data)
+    builder = CommandBufferBuilder(data)
+    for k in range(2):
+        sim.step(1, want_stats=False)
+        steps.submit_substeps(builder, 3, 1, k == 0)
+        for f in FIELDS:
+            a, b = sim.data.download(f), data.download(f)
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (k, f)
+    assert sim.data.read_stats().flags & _abi.FE_STATS_NEIGHBOR_OVERFLOW
+    sim.close()
+    data.close()
